@@ -217,7 +217,6 @@ __device__ __forceinline__ void classify_tile_mc_inner(const Plan &p, const uint
         }
         if (lane < WY) {
             p.flags[((int64_t)chunk * p.tiles_x + tx) * p.cy + y0 + lane] = mine != 0u;
-            if (p.cmask) p.cmask[((int64_t)tx * p.cy + y0 + lane) * p.nchunks + chunk] = mine;
         }
     }
     if (lane >= TILE_X) return;
@@ -325,7 +324,6 @@ __device__ __forceinline__ void classify_tile_mc(const Plan &p, const uint32_t *
         }
         if (lane < WY && y0 + lane < p.cy) {
             p.flags[((int64_t)chunk * p.tiles_x + tx) * p.cy + y0 + lane] = mine != 0u;
-            if (p.cmask) p.cmask[((int64_t)tx * p.cy + y0 + lane) * p.nchunks + chunk] = mine;
         }
     }
     if (!cellx) return;
@@ -617,7 +615,7 @@ __global__ void __launch_bounds__(32 * (WARPS + 1)) k_classify_tma(const Plan p,
 // one packed-word lookup per cell row; an activity chunk (ZC = 2 stages)
 // closes at the first plane of every even stage.  Tiles at the volume's edge
 // take the same loop with per-lane and per-row guards.  Outputs as the load
-// walk: piece counts, activity bytes and the active-column masks (cmask).
+// walk: piece counts and activity bytes.
 template <class T, bool INNER>
 __device__ __forceinline__ void tma_mc_consume(const Plan &p, const uint32_t *s_tab, const T *buf, uint64_t *full,
                                                uint64_t *empty, int *s_fail, int lane, int w, int tx, int seg,
@@ -688,7 +686,6 @@ __device__ __forceinline__ void tma_mc_consume(const Plan &p, const uint32_t *s_
         }
         if (lane < WY && (INNER || y0 + lane < p.cy)) {
             p.flags[((int64_t)chunk * p.tiles_x + tx) * p.cy + y0 + lane] = mine != 0u;
-            if (p.cmask) p.cmask[((int64_t)tx * p.cy + y0 + lane) * p.nchunks + chunk] = mine;
         }
     };
     auto release = [&](int slot) {

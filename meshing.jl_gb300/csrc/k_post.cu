@@ -88,5 +88,6 @@ extern "C" int mesh_vertex_normals(mesh_ctx *c, const void *verts, int float_bit
                                              c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "normals launch");
     c->have_plan = 0;  // the error word no longer belongs to an extraction
+    c->bits_on = 0;
     return MESH_OK;
 }

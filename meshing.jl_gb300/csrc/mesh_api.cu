@@ -231,7 +231,117 @@ cudaError_t upload_and_classify(mesh_ctx *c) {
 }
 
 bool one_walk(const mesh_ctx *c);
-bool direct_mc(const mesh_ctx *c);
+bool bits_path(const mesh_ctx *c);
+
+// Buffers and tiling of the sign-bit path (mesh_bits.cuh).  The columns are cut into
+// z segments until there are 512 items per SM, 20 for each warp of the emission, so
+// that its last items end together (1024^3: 1.75 ms a call against 1.81 with 64).
+int prepare_bits(mesh_ctx *c) {
+    Plan &P = c->plan;
+    P.nxb = (P.cx + BCOL - 1) / BCOL;
+    P.nyb = (P.cy + BROW - 1) / BROW;
+    P.nzw = (int32_t)((P.nz + 31) / 32);
+    const int ncw = (P.cz + 31) / 32;
+    const int64_t rows = (int64_t)P.nxb * P.cy, target = (int64_t)c->sms * 512;
+    auto segments = [&](int zws) {
+        P.zws = zws;
+        P.bseg = (ncw + zws - 1) / zws;
+    };
+    const int nseg = (int)std::min<int64_t>(ncw, std::max<int64_t>(1, (target + rows - 1) / rows));
+    segments(std::min(ZWS_MAX, (ncw + nseg - 1) / nseg));
+    const size_t word = (size_t)P.nx * P.ny * sizeof(uint32_t);  // one word of every column
+    // the whole volume's words, or windows of whole segments and the word after them
+    int keep = P.nzw;
+    cudaError_t e = cudaErrorMemoryAllocation;
+    for (;;) {
+        const size_t need = (size_t)(keep == P.nzw ? keep : keep + 1) * word;
+        if (c->bits_max <= 0 || (int64_t)need <= c->bits_max || keep <= 1) e = c->bits.ensure(need);
+        if (e == cudaSuccess) break;
+        cudaGetLastError();
+        if (keep <= 1) return cuda_fail(c, e, "sign words");
+        keep = (keep + 1) / 2;
+        e = cudaErrorMemoryAllocation;
+    }
+    if (keep < P.nzw) segments(std::min(P.zws, keep));
+    c->win_segs = keep < P.nzw ? keep / P.zws : P.bseg;
+    P.npc = (int64_t)P.cx * P.cy * P.bseg;
+    const int64_t ntiles = (P.npc + BITS_TILE - 1) / BITS_TILE;
+    if (ntiles > 0x7fffffff) return fail(c, MESH_ETOOLARGE, "grid too large for this volume shape");
+    P.ntiles = (int32_t)ntiles;
+    if ((e = c->pc.ensure((size_t)P.npc * sizeof(uint2))) != cudaSuccess) return cuda_fail(c, e, "piece counts");
+    if ((e = c->tsum.ensure((size_t)ntiles * sizeof(ulonglong2))) != cudaSuccess) return cuda_fail(c, e, "tile sums");
+    if ((e = c->wmask.ensure((size_t)rows * P.bseg * mask_words(P.zws) * sizeof(uint32_t))) != cudaSuccess)
+        return cuda_fail(c, e, "activity masks");
+    P.bits = (uint32_t *)c->bits.ptr;
+    P.bw0 = 0;
+    P.bw1 = P.nzw;
+    P.pc = (uint2 *)c->pc.ptr;
+    P.tsum = (ulonglong2 *)c->tsum.ptr;
+    P.wmask = (uint32_t *)c->wmask.ptr;
+    int64_t *m = (int64_t *)c->misc.ptr;
+    P.totals = m;
+    P.err = (unsigned int *)(c->h_misc + PIN_ERR);
+    P.done = (unsigned int *)(m + MISC_DONE);
+    P.work = (unsigned int *)(m + MISC_WORK);
+    return MESH_OK;
+}
+
+// Sign words of the window of segments s0 .. s1 - 1 (and the word after them).
+cudaError_t window_bits(mesh_ctx *c, Plan &P, int s0, int s1, bool first) {
+    P.bw0 = s0 * P.zws;
+    P.bw1 = std::min(P.nzw, s1 * P.zws + 1);
+    TabArgs ta = c->targs;
+    ta.on = first;
+    return launch_bits(P, P.bw0, P.bw1 - P.bw0, ta, c->sms, c->stream);
+}
+
+// Sign words, piece counts and offsets.
+cudaError_t count_bits(mesh_ctx *c) {
+    Plan &P = c->plan;
+    cudaError_t e = cudaSuccess;
+    if (c->ngroups > 1) {
+        // host volume: groups of words go up on the copy stream, each classified on
+        // the compute stream as soon as its planes have arrived
+        const size_t plane = (size_t)P.nx * P.ny * dtype_size(P.T);
+        e = cudaEventRecord(c->ev_ready, c->stream);  // earlier work on the volume buffer
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(c->copy, c->ev_ready, 0);
+        for (int g = 0; g < c->ngroups && e == cudaSuccess; g++) {
+            const int w0 = (int)((int64_t)g * P.nzw / c->ngroups), w1 = (int)((int64_t)(g + 1) * P.nzw / c->ngroups);
+            const int64_t p0 = (int64_t)w0 * 32, p1 = std::min<int64_t>((int64_t)w1 * 32, P.nz);
+            e = cudaMemcpyAsync((char *)c->vol.ptr + p0 * plane, (const char *)c->upl_src + p0 * plane,
+                                (size_t)(p1 - p0) * plane, cudaMemcpyHostToDevice, c->copy);
+            if (e == cudaSuccess) e = cudaEventRecord(c->ev_part[g], c->copy);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_part[g], 0);
+            TabArgs ta = c->targs;
+            ta.on = g == 0;
+            if (e == cudaSuccess) e = launch_bits(P, w0, w1 - w0, ta, c->sms, c->stream);
+        }
+        if (e == cudaSuccess) e = launch_count(P, 0, P.bseg, c->stream);
+    } else {
+        for (int s0 = 0; s0 < P.bseg && e == cudaSuccess; s0 += c->win_segs) {
+            const int s1 = std::min(P.bseg, s0 + c->win_segs);
+            e = window_bits(c, P, s0, s1, s0 == 0);
+            if (e == cudaSuccess) e = launch_count(P, s0, s1 - s0, c->stream);
+        }
+    }
+    return e;
+}
+
+// Emission of the column blocks of `q` (slot: its cleared work counter).
+cudaError_t emit_bits(mesh_ctx *c, Plan q, int slot) {
+    if (c->win_segs >= q.bseg && slot < WORK_SLOTS) {
+        q.work += 2 * slot;
+        return launch_emit_bits_mc(q, c->Q64, c->P64, 0, q.bseg, c->stream);
+    }
+    cudaError_t e = cudaSuccess;
+    for (int s0 = 0; s0 < q.bseg && e == cudaSuccess; s0 += c->win_segs) {
+        const int s1 = std::min(q.bseg, s0 + c->win_segs);
+        e = window_bits(c, q, s0, s1, false);
+        if (e == cudaSuccess) e = cudaMemsetAsync(q.work, 0, sizeof(unsigned), c->stream);
+        if (e == cudaSuccess) e = launch_emit_bits_mc(q, c->Q64, c->P64, s0, s1 - s0, c->stream);
+    }
+    return e;
+}
 
 int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t nz, int vol_on_device,
             const mesh_params *p) {
@@ -304,16 +414,36 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
     }
 
     // coordinate tables: xp yp zp dx dy dz (double), the same as float, then the
-    // hi/lo float split of the nodes and spacings, computed on the device
+    // hi/lo float split of the nodes and spacings, computed on the device (on the
+    // sign-bit path by the launch that packs the first words)
     const int64_t ntab = nx + ny + nz;
+    c->bits_on = bits_path(c);
     if ((e = c->tabs.ensure(table_bytes(ntab))) != cudaSuccess) return cuda_fail(c, e, "table buffer");
     if (c->win_nx && c->win_x0 + nx > c->win_nx) return fail(c, MESH_EINVAL, "volume extends past its x window");
-    if ((e = launch_tables((double *)c->tabs.ptr, nx, ny, nz, p->range, L32, c->stream, c->win_x0, c->win_nx)) !=
-        cudaSuccess)
-        return cuda_fail(c, e, "table launch");
-    count_kernels(c, 0, 1);  // the coordinate tables count with the classification
+    if (c->bits_on) {
+        c->targs = TabArgs{(double *)c->tabs.ptr, nx, ny, nz, c->win_x0, c->win_nx, {}, L32, 0};
+        for (int k = 0; k < 6; k++) c->targs.range[k] = p->range[k];
+    } else {
+        if ((e = launch_tables((double *)c->tabs.ptr, nx, ny, nz, p->range, L32, c->stream, c->win_x0, c->win_nx)) !=
+            cudaSuccess)
+            return cuda_fail(c, e, "table launch");
+        count_kernels(c, 0, 1);  // the coordinate tables count with the classification
+    }
     bind_tables(P, (double *)c->tabs.ptr, nx, ny, nz);
     P.force_fp64 = c->force_fp64;
+
+    if (c->bits_on) {
+        const int rc = prepare_bits(c);
+        if (rc == MESH_OK && c->ngroups > 1) {
+            c->ngroups = std::min(PIPE_MAX, P.nzw);
+            if (c->win_segs < P.bseg || c->ngroups < 2) {  // windows: the volume goes up first
+                c->ngroups = 1;
+                if ((e = cudaMemcpyAsync(c->vol.ptr, vol, vbytes, cudaMemcpyHostToDevice, c->stream)) != cudaSuccess)
+                    return cuda_fail(c, e, "volume upload");
+            }
+        }
+        return rc;
+    }
 
     // scratch
     const int64_t np = npieces(P);
@@ -327,12 +457,6 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
     P.cnt = (uint32_t *)c->cnt.ptr;
     P.base = (int64_t *)c->base.ptr;
     P.flags = (uint8_t *)c->flags.ptr;
-    P.cmask = nullptr;
-    if (direct_mc(c)) {
-        const size_t mb = (size_t)P.tiles_x * P.cy * P.nchunks * sizeof(uint32_t);
-        if ((e = c->cmask.ensure(mb)) != cudaSuccess) return cuda_fail(c, e, "mask buffer");
-        P.cmask = (uint32_t *)c->cmask.ptr;
-    }
     P.scan_state = (unsigned long long *)c->scan.ptr;
     P.scan_ticket = (unsigned int *)((char *)c->scan.ptr + sb);
     // misc: totals[NCNT] int64, then the error word, the work counter and the
@@ -419,16 +543,29 @@ bool one_walk(const mesh_ctx *c) {
     return c->plan.alg == MESH_ALG_MC && !c->weld && (c->one_walk || c->host_mapped);
 }
 
-// Marching Cubes emitted straight from the volume (the default): the classify
-// walk leaves per-chunk active-column masks and no list of active cells is
-// built (both classify walks write the masks).
-bool direct_mc(const mesh_ctx *c) {
-    return c->plan.alg == MESH_ALG_MC && !c->list_emit && !one_walk(c);
-}
+// Marching Cubes classified into sign bits and emitted from them (the default).
+bool bits_path(const mesh_ctx *c) { return c->plan.alg == MESH_ALG_MC && !c->list_emit && !one_walk(c); }
 
 int run_count(mesh_ctx *c) {
     Plan &P = c->plan;
     cudaError_t e;
+    if (c->bits_on) {
+        mark(c, 0);
+        if ((e = count_bits(c)) != cudaSuccess) return cuda_fail(c, e, "classify launch");
+        mark(c, 0);
+        const int parts = c->ngroups > 1 ? c->ngroups + 1 : 2 * ((P.bseg + c->win_segs - 1) / c->win_segs);
+        count_kernels(c, 0, parts);
+        if (P.tot_out == c->h_misc + PIN_TOT) {  // the host reads the totals while the offsets are scanned
+            if (!c->ev_cnt && (e = cudaEventCreateWithFlags(&c->ev_cnt, cudaEventDisableTiming)) != cudaSuccess)
+                return cuda_fail(c, e, "count event");
+            if ((e = cudaEventRecord(c->ev_cnt, c->stream)) != cudaSuccess) return cuda_fail(c, e, "count event");
+        }
+        mark(c, 1);
+        if ((e = launch_offsets(P, c->stream)) != cudaSuccess) return cuda_fail(c, e, "scan launch");
+        mark(c, 1);
+        count_kernels(c, 1, 1);
+        return MESH_OK;
+    }
     if ((e = cudaMemsetAsync(c->misc.ptr, 0, MISC_SLOTS * sizeof(int64_t), c->stream)) != cudaSuccess)
         return cuda_fail(c, e, "memset");
     // the pipelined upload classifies each group with the load walk as it arrives
@@ -469,7 +606,29 @@ int fetch_misc(mesh_ctx *c) {
                                     c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "synchronize");
+    if (c->bits_on) c->h_misc[NCNT] = c->h_misc[PIN_ERR];
     c->h_misc[NCNT] &= 0xffffffffll;
+    return MESH_OK;
+}
+
+// Wait for the count's totals (sign-bit path: written by the kernel itself).
+int fetch_totals(mesh_ctx *c) {
+    if (!c->bits_on) return fetch_misc(c);
+    cudaError_t e = cudaEventSynchronize(c->ev_cnt);
+    if (e != cudaSuccess) return cuda_fail(c, e, "synchronize");
+    c->h_misc[0] = c->h_misc[PIN_TOT];
+    c->h_misc[1] = c->h_misc[PIN_TOT + 1];
+    c->h_misc[2] = 0;
+    c->h_misc[NCNT] = 0;
+    return MESH_OK;
+}
+
+// Wait for the stream and take the error word (sign-bit path: in pinned memory).
+int finish(mesh_ctx *c) {
+    if (!c->bits_on) return fetch_misc(c);
+    cudaError_t e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess) return cuda_fail(c, e, "synchronize");
+    c->h_misc[NCNT] = c->h_misc[PIN_ERR] & 0xffffffffll;
     return MESH_OK;
 }
 
@@ -506,9 +665,9 @@ int launch_emit(mesh_ctx *c) {
         count_kernels(c, 3, 1);
         return e != cudaSuccess ? cuda_fail(c, e, "expand launch") : MESH_OK;
     }
-    if (direct_mc(c)) {
+    if (c->bits_on) {
         mark(c, 2);
-        e = launch_direct_mc(c->plan, c->Q64, c->P64, c->stream);
+        e = emit_bits(c, c->plan, 0);
         mark(c, 2);
         count_kernels(c, 2, 1);
         return e != cudaSuccess ? cuda_fail(c, e, "emit launch") : MESH_OK;
@@ -541,16 +700,26 @@ int emit_pipelined(mesh_ctx *c, int K, void *verts, int64_t *faces) {
     const int64_t np = P.pstride;
     const size_t vsz = (size_t)3 * (P.out64 ? 8 : 4);
     int tx[PIPE_MAX + 1];
-    for (int g = 0; g <= K; g++) tx[g] = (int)((int64_t)g * P.tiles_x / K);
+    const int blocks = c->bits_on ? P.nxb : P.tiles_x;
+    for (int g = 0; g <= K; g++) tx[g] = (int)((int64_t)g * blocks / K);
+    const int per = c->bits_on ? 2 : 3;  // values per split point
     GatherIdx gi{};
-    gi.n = 3 * (K - 1);
-    for (int g = 1; g < K; g++) {
-        const int64_t i = piece(P, 0, 0, tx[g] * TILE_X);
-        for (int k = 0; k < 3; k++) gi.idx[3 * (g - 1) + k] = k * np + i;
+    cudaError_t e;
+    if (c->bits_on) {
+        gi.n = K - 1;
+        for (int g = 1; g < K; g++) gi.idx[g - 1] = (int64_t)tx[g] * BCOL * P.cy * P.bseg;
+        e = launch_gather_pieces(P, gi, (int64_t *)c->gat.ptr, c->stream);
+    } else {
+        gi.n = 3 * (K - 1);
+        for (int g = 1; g < K; g++) {
+            const int64_t i = piece(P, 0, 0, tx[g] * TILE_X);
+            for (int k = 0; k < 3; k++) gi.idx[3 * (g - 1) + k] = k * np + i;
+        }
+        e = launch_gather(P.base, gi, (int64_t *)c->gat.ptr, c->stream);
     }
-    cudaError_t e = launch_gather(P.base, gi, (int64_t *)c->gat.ptr, c->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(c->h_gat, c->gat.ptr, (size_t)gi.n * sizeof(int64_t), cudaMemcpyDeviceToHost, c->stream);
+        e = cudaMemcpyAsync(c->h_gat, c->gat.ptr, (size_t)per * (K - 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
+                            c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "split points");
     int64_t V[PIPE_MAX + 1], F[PIPE_MAX + 1], E[PIPE_MAX + 1];
@@ -559,9 +728,9 @@ int emit_pipelined(mesh_ctx *c, int K, void *verts, int64_t *faces) {
     F[K] = c->nfaces;
     E[K] = c->nactive;
     for (int g = 1; g < K; g++) {
-        V[g] = c->h_gat[3 * (g - 1)];
-        F[g] = c->h_gat[3 * (g - 1) + 1];
-        E[g] = c->h_gat[3 * (g - 1) + 2];
+        V[g] = c->h_gat[per * (g - 1)];
+        F[g] = c->h_gat[per * (g - 1) + 1];
+        E[g] = per == 3 ? c->h_gat[per * (g - 1) + 2] : 0;
     }
     for (int g = 0; g < K; g++)
         if (V[g] > V[g + 1] || F[g] > F[g + 1] || E[g] > E[g + 1] || V[g + 1] > c->nverts || F[g + 1] > c->nfaces)
@@ -574,8 +743,8 @@ int emit_pipelined(mesh_ctx *c, int K, void *verts, int64_t *faces) {
         q.ntx = tx[g + 1] - tx[g];
         q.e_lo = E[g];
         q.e_hi = E[g + 1];
-        if (direct_mc(c)) {
-            e = launch_direct_mc(q, c->Q64, c->P64, c->stream);
+        if (c->bits_on) {
+            e = emit_bits(c, q, g);
         } else {
             e = launch_emit_mc(q, c->Q64, c->P64, 0, c->stream);
             if (e == cudaSuccess && E[g + 1] > E[g]) {
@@ -659,13 +828,16 @@ int mesh_ctx_create(int device, mesh_ctx **out) {
     c->device = device;
     cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, device);
     if (cudaStreamCreateWithFlags(&c->own, cudaStreamNonBlocking) != cudaSuccess ||
-        c->misc.ensure(MISC_SLOTS * sizeof(int64_t)) != cudaSuccess ||
-        cudaHostAlloc((void **)&c->h_misc, MISC_SLOTS * sizeof(int64_t), cudaHostAllocDefault) != cudaSuccess) {
+        c->misc.ensure(MISC_WORDS * sizeof(int64_t)) != cudaSuccess ||
+        cudaHostAlloc((void **)&c->h_misc, PIN_WORDS * sizeof(int64_t), cudaHostAllocDefault) != cudaSuccess) {
         cudaGetLastError();
         mesh_ctx_destroy(c);
         return MESH_ENOMEM;
     }
     c->stream = c->own;
+    memset(c->h_misc, 0, PIN_WORDS * sizeof(int64_t));
+    const char *bb = getenv("MESHING_GB300_BITS_BYTES");
+    if (bb && bb[0]) c->bits_max = strtoll(bb, nullptr, 10);
     const char *ff = getenv("MESHING_GB300_FORCE_FP64");
     c->force_fp64 = ff && ff[0] == '1';
     const char *wt = getenv("MESHING_GB300_TMA");
@@ -689,12 +861,13 @@ void mesh_ctx_destroy(mesh_ctx *c) {
     if (c->copy) cudaStreamSynchronize(c->copy);
     DevBuf *bufs[] = {&c->vol,   &c->tabs,  &c->cnt, &c->base, &c->flags,    &c->scan,   &c->misc,
                       &c->out_v, &c->out_f, &c->ent, &c->nrm,  &c->weld_buf, &c->weld_v, &c->gat,
-                      &c->cmask};
+                      &c->bits, &c->pc,   &c->tsum, &c->wmask};
     for (DevBuf *b : bufs) b->release();
     for (cudaEvent_t e : c->ev_part)
         if (e) cudaEventDestroy(e);
     if (c->ev_ready) cudaEventDestroy(c->ev_ready);
     if (c->ev_done) cudaEventDestroy(c->ev_done);
+    if (c->ev_cnt) cudaEventDestroy(c->ev_cnt);
     if (c->copy) cudaStreamDestroy(c->copy);
     if (c->h_gat) cudaFreeHost(c->h_gat);
     for (auto &v : c->ev_pairs)
@@ -754,8 +927,10 @@ int run_weld(mesh_ctx *c) {
     P.faces_cap = nf;
     P.vkey = (long long *)wb;
     int rc;
-    if (!direct_mc(c) && (rc = ensure_entries(c, c->nactive))) return rc;
-    if ((e = cudaMemsetAsync(P.err, 0, sizeof(unsigned), c->stream)) != cudaSuccess) return cuda_fail(c, e, "memset");
+    if (!c->bits_on) {
+        if ((rc = ensure_entries(c, c->nactive))) return rc;
+        if ((e = cudaMemsetAsync(P.err, 0, sizeof(unsigned), c->stream)) != cudaSuccess) return cuda_fail(c, e, "memset");
+    }
     if ((rc = launch_emit(c))) return rc;
     if ((e = launch_weld(P.vkey, nv, P.verts, P.out64, P.faces, nf, (long long *)(wb + o_bsum), c->weld_v.ptr,
                          (unsigned long long *)(wb + o_hkey), (long long *)(wb + o_hval), hcap, P.err, c->sms,
@@ -821,6 +996,7 @@ int mesh_count(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int6
     }
     if (!vol) return fail(c, MESH_EINVAL, "volume is NULL");
     if ((rc = prepare(c, vol, T, nx, ny, nz, vol_on_device, p))) return rc;
+    if (c->bits_on) c->plan.tot_out = c->h_misc + PIN_TOT;
     if (one_walk(c)) {
         // the list of active cells is filled during the count: start from a
         // guess (or the context's earlier list), and if the walk ran out of
@@ -830,7 +1006,7 @@ int mesh_count(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int6
         if ((rc = ensure_entries(c, guess))) return rc;
     }
     if ((rc = run_count(c))) return rc;
-    if ((rc = fetch_misc(c))) return rc;
+    if ((rc = fetch_totals(c))) return rc;
     if (one_walk(c) && ((unsigned)c->h_misc[NCNT] & ERR_STAGE)) {
         if ((rc = ensure_entries(c, c->h_misc[NCNT + 2]))) return rc;
         if ((rc = run_count(c))) return rc;
@@ -879,13 +1055,14 @@ int mesh_fill(mesh_ctx *c, void *verts, int64_t *faces, int out_on_device) {
     P.verts_cap = c->nverts;
     P.faces_cap = c->nfaces;
     int rc;
-    if (P.alg == MESH_ALG_MC && !one_walk(c) && !direct_mc(c) && (rc = ensure_entries(c, c->nactive))) return rc;
-    if ((e = cudaMemsetAsync(P.err, 0, sizeof(unsigned), c->stream)) != cudaSuccess) return cuda_fail(c, e, "memset");
+    if (P.alg == MESH_ALG_MC && !one_walk(c) && !c->bits_on && (rc = ensure_entries(c, c->nactive))) return rc;
+    if (!c->bits_on && (e = cudaMemsetAsync(P.err, 0, sizeof(unsigned), c->stream)) != cudaSuccess)
+        return cuda_fail(c, e, "memset");
     int parts = 1;
     if (!out_on_device && P.alg == MESH_ALG_MC && !one_walk(c) && c->pipe_bytes > 0 &&
-        (int64_t)(vb + fbytes) >= c->pipe_bytes && P.tiles_x >= 2) {
+        (int64_t)(vb + fbytes) >= c->pipe_bytes && (c->bits_on ? P.nxb : P.tiles_x) >= 2) {
         if ((rc = ensure_pipe(c))) return rc;
-        parts = std::min(PIPE_MAX, P.tiles_x);
+        parts = std::min(PIPE_MAX, c->bits_on ? P.nxb : P.tiles_x);
     }
     if (parts > 1) {
         if ((rc = emit_pipelined(c, parts, verts, faces))) return rc;
@@ -899,7 +1076,7 @@ int mesh_fill(mesh_ctx *c, void *verts, int64_t *faces, int out_on_device) {
                 return cuda_fail(c, e, "face download");
         }
     }
-    if ((rc = fetch_misc(c))) return rc;
+    if ((rc = finish(c))) return rc;
     c->have_plan = 0;  // a plan may reference a caller's device volume: one fill per count
     return check_err(c);
 }
@@ -927,14 +1104,16 @@ int mesh_extract_device(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t
     P.faces = faces;
     P.verts_cap = verts ? verts_cap : 0;
     P.faces_cap = faces ? faces_cap : 0;
+    if (c->bits_on) P.tot_out = counts;
     // an active Marching Cubes cell emits at least 3 vertices; the one walk
     // also leaves up to a block of slots per warp unused
-    if (P.alg == MESH_ALG_MC && !direct_mc(c) &&
+    if (P.alg == MESH_ALG_MC && !c->bits_on &&
         (rc = ensure_entries(c, P.verts_cap / 3 + (one_walk(c) ? stage_slack(P) : 0))))
         return rc;
     if ((rc = run_count(c))) return rc;
     if ((rc = launch_emit(c))) return rc;
-    if ((e = cudaMemcpyAsync(counts, P.totals, 2 * sizeof(int64_t), cudaMemcpyDeviceToDevice, c->stream)) !=
+    if (!c->bits_on &&
+        (e = cudaMemcpyAsync(counts, P.totals, 2 * sizeof(int64_t), cudaMemcpyDeviceToDevice, c->stream)) !=
         cudaSuccess)
         return cuda_fail(c, e, "count copy");
     c->have_plan = 0;

@@ -1,0 +1,86 @@
+// Sign bits of a volume and what the kernels built on them share.
+//
+// k_bits.cu reads the volume once and keeps one bit per sample, `v < iso`, in
+// words of 32 consecutive z: bit k of word (zw, y, x) is sample (x, y, 32 zw + k).
+// Words of one zw lie like the samples of one plane (x fastest), so a lane that
+// owns column x reads its own four corner columns with coalesced loads and
+// classifies 32 cells of the column with a few logic instructions.
+#pragma once
+#include "mesh_internal.cuh"
+
+namespace mesh {
+
+constexpr int BITS_TILE = 2048;  // pieces per tile of the offset scan
+constexpr int BCOL = 32;         // cell columns (x) of a warp's item
+constexpr int BROW = 8;          // cell rows (y) of a CTA of k_count
+// Words of z in a segment: the vertices and faces of a tile of pieces stay below
+// 2^32 (at most 12 per cell or node).
+constexpr int ZWS_MAX = 4096;
+constexpr int WORK_SLOTS = 8;    // work counters (8 bytes apart) that k_bits clears, one per emission launch
+
+// One volume as the bit kernels see it: the plan's single volume or one of a batch.
+struct BView {
+    const void *vol;
+    const uint32_t *bits;  // word (zw, y, x) at bits[(zw - bw0) * sxy + y * nx + x]
+    int64_t nx, ny, nz, sxy;
+    int32_t cx, cy, cz;
+    int32_t nxb, nyb, nseg, zws, nzw, bw0;  // column / row blocks, z segments of zws words, words of z
+    int64_t e0;            // first piece
+    int64_t m0;            // first word of the activity masks
+};
+
+inline __host__ __device__ int mask_words(int zws) { return (zws + 31) / 32; }
+// Piece of column (x, y) in z segment seg: emission order (x outermost, z fastest).
+inline __host__ __device__ int64_t bpiece(const BView &v, int seg, int y, int x) {
+    return v.e0 + ((int64_t)x * v.cy + y) * v.nseg + seg;
+}
+// Activity mask words of item (seg, y, xb): bit k of word q set when word
+// seg * zws + 32 q + k of z has an active cell in the item's 32 columns.
+inline __host__ __device__ int64_t bmask(const BView &v, int seg, int y, int xb) {
+    return v.m0 + (((int64_t)seg * v.cy + y) * v.nxb + xb) * mask_words(v.zws);
+}
+
+}  // namespace mesh
+
+#ifdef __CUDACC__
+namespace mesh {
+
+__device__ __forceinline__ BView view_of(const Plan &p) {
+    return BView{p.vol, p.bits, p.nx, p.ny, p.nz, p.nx * p.ny, p.cx, p.cy, p.cz, p.nxb, p.nyb,
+                 p.bseg, p.zws, p.nzw, p.bw0, 0, 0};
+}
+
+// The four corner columns of column (x, y) in one word of z, and the same one
+// sample up (bit k: sample z + 1).
+struct Corners {
+    uint32_t a, b, c, d;      // (x, y) (x+1, y) (x, y+1) (x+1, y+1)
+    uint32_t as, bs, cs, ds;  // shifted
+    // cells of the word with corners on both sides
+    __device__ __forceinline__ uint32_t active() const {
+        return (a | b | c | d | as | bs | cs | ds) & ~(a & b & c & d & as & bs & cs & ds);
+    }
+};
+
+// Cells of word zw that exist.
+__device__ __forceinline__ uint32_t cell_mask(int cz, int zw) {
+    const int n = cz - 32 * zw;
+    return n >= 32 ? 0xffffffffu : (n <= 0 ? 0u : (1u << n) - 1u);
+}
+
+// Index bits 0..7 of a cell: corners (x,y) at z, z+1, then (x+1,y), (x,y+1),
+// (x+1,y+1); the cube case of src/common.jl:10-20 is a permutation of them.
+__device__ __forceinline__ uint32_t cell_index(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t na, uint32_t nb,
+                                               uint32_t nc, uint32_t nd, int z) {
+    return (__funnelshift_r(a, na, z) & 3u) | ((__funnelshift_r(b, nb, z) & 3u) << 2) |
+           ((__funnelshift_r(c, nc, z) & 3u) << 4) | ((__funnelshift_r(d, nd, z) & 3u) << 6);
+}
+
+}  // namespace mesh
+#endif
+
+namespace mesh {
+constexpr unsigned mc_case_of_bits(unsigned u) {
+    return (u & 1u) | (((u >> 2) & 1u) << 1) | (((u >> 6) & 1u) << 2) | (((u >> 4) & 1u) << 3) | (((u >> 1) & 1u) << 4) |
+           (((u >> 3) & 1u) << 5) | (((u >> 7) & 1u) << 6) | (((u >> 5) & 1u) << 7);
+}
+}  // namespace mesh

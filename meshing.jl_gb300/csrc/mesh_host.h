@@ -8,14 +8,21 @@
 #include <string>
 #include <vector>
 
+#include "mesh_bits.cuh"
 #include "mesh_internal.cuh"
 
 namespace mesh {
 
 constexpr int NSTAGE = 4;  // classify (or the one-walk MC pass), scan, emit (second walk), expand
 // device word slots of the misc buffer: totals[NCNT], error word, work counter,
-// staging counter
+// staging counter; then, for the sign-bit path, the CTA counter of the piece
+// counts and the emissions' work counters
 constexpr int MISC_SLOTS = NCNT + 3;
+constexpr int MISC_DONE = MISC_SLOTS, MISC_WORK = MISC_SLOTS + 1;
+constexpr int MISC_WORDS = MISC_WORK + WORK_SLOTS;
+// pinned words: the copy of the misc slots, then what the sign-bit path's kernels
+// write themselves: the two totals and the error word
+constexpr int PIN_TOT = MISC_SLOTS, PIN_ERR = MISC_SLOTS + 2, PIN_WORDS = MISC_SLOTS + 3;
 // parts of the pipelined host path: upload groups of z segments, x ranges of the emission
 constexpr int PIPE_MAX = 8;
 
@@ -53,8 +60,17 @@ struct mesh_ctx {
     cudaStream_t own = nullptr;
     cudaStream_t stream = nullptr;
     mesh::DevBuf vol, tabs, cnt, base, flags, scan, misc, out_v, out_f, ent;
+    // sign-bit path: sign words, piece counts / offsets, tile sums, activity masks;
+    // bits_max caps the sign words (MESHING_GB300_BITS_BYTES; 0: what the device
+    // gives): a volume whose words do not fit is classified, and emitted, in
+    // windows of win_segs z segments
+    mesh::DevBuf bits, pc, tsum, wmask;
+    int64_t bits_max = 0;
+    int win_segs = 0;
+    int bits_on = 0;  // the current plan takes the sign-bit path
+    cudaEvent_t ev_cnt = nullptr;
+    mesh::TabArgs targs{};
     mesh::DevBuf nrm;  // mesh_vertex_normals: double accumulators
-    mesh::DevBuf cmask;  // Marching Cubes: per (x tile, cell row, chunk) active-column masks
     // welded Marching Cubes (MESH_ALG_MC_WELDED): the count runs the whole
     // extraction into out_v / out_f and welds it into weld_v; mesh_fill copies
     int weld = 0;
@@ -100,8 +116,8 @@ struct mesh_ctx {
     // walk 2.24 + expand 1.41 ms vs classify 1.24 + compact 1.18 + expand 0.75 ms).
     int one_walk = 0;
     // MESHING_GB300_LIST_EMIT=1: Marching Cubes emitted through the list of
-    // active cells (compaction, then expansion) instead of straight from the
-    // volume (k_direct_mc.cu); kept for comparison tests.
+    // active cells (compaction, then expansion) instead of from the sign bits
+    // (k_emit_bits.cu); kept for comparison tests.
     int list_emit = 0;
     // MESHING_GB300_ZEROCOPY=1: a Marching Cubes host volume in pinned, mapped
     // memory is read in place over the host link (NVLink-C2C) by the one walk

@@ -75,9 +75,6 @@ struct Plan {
     uint32_t *cnt;        // [NCNT][nseg][cy][cx] per-piece vertex / face / active-cell counts
     int64_t *base;        // [NCNT][nseg][cy][cx] exclusive prefix in traversal order
     uint8_t *flags;       // [nchunks][tiles_x][cy] 1 if the tile row has an active cell
-    // Marching Cubes, single volume (null otherwise): [tiles_x][cy][nchunks] bit l
-    // set when cell column tx * TILE_X + l of that row has an active cell in the chunk
-    uint32_t *cmask;
     unsigned long long *scan_state;  // [NCNT][scan tiles] decoupled look-back words
     unsigned int *scan_ticket;
     int64_t *totals;      // [NCNT] total vertices, faces, active cells
@@ -127,6 +124,22 @@ struct Plan {
     // expand list entries e_lo .. e_hi - 1
     int32_t seg0, seg1, tx0, ntx;
     int64_t e_lo, e_hi;
+    // sign bits (mesh_bits.cuh): words bw0 .. bw1 - 1 of z at `bits`, z segments of
+    // zws words (bseg of them) and column / row blocks; per piece, the vertex and
+    // face counts that the offset scan turns into offsets within their scan tile
+    // (pc), per tile the sums that become the tiles' offsets (tsum), and the masks
+    // of active words (wmask)
+    uint32_t *bits;
+    uint2 *pc;
+    ulonglong2 *tsum;
+    uint32_t *wmask;
+    unsigned int *done;   // CTAs of k_count that have finished
+    int64_t npc;
+    int64_t *tot_out;     // where k_count also leaves the totals (device or pinned; null: nowhere)
+    int32_t nxb, nyb, bseg, zws, nzw, bw0, bw1, ntiles;
+    // batches: the volume of each CTA of the bit and count kernels, and their number
+    const uint32_t *bblk_vol, *cblk_vol;
+    int64_t nbblk, ncblk;
 };
 
 // One volume of a batch.  Its work items, pieces, activity bytes and scan
@@ -144,6 +157,10 @@ struct BatchVol {
     int64_t *faces;
     int64_t vcap, fcap;
     int64_t kbase;  // welded batches: the volume's lattice-edge keys start here
+    // sign bits: tiling, first word, piece, mask word and CTAs, and whether its
+    // planes start on 16-byte boundaries
+    int32_t nxb, nyb, bseg, zws, nzw, vec;
+    int64_t bits0, e0, m0, bblk0, cblk0;
 };
 
 // Bytes per sample of a volume dtype.
@@ -251,10 +268,26 @@ struct GatherIdx {
     int n;
 };
 cudaError_t launch_gather(const int64_t *src, const GatherIdx &g, int64_t *dst, cudaStream_t s);
+// First vertex and face of pieces e[0..n) (after the offset scan): dst[2 i], dst[2 i + 1].
+cudaError_t launch_gather_pieces(const Plan &p, const GatherIdx &g, int64_t *dst, cudaStream_t s);
 cudaError_t launch_scan(const Plan &p, cudaStream_t s);
 cudaError_t launch_emit(const Plan &p, int Q64, int A64, int P64, cudaStream_t s);
-// Marching Cubes emitted straight from the volume (k_direct_mc.cu): needs cmask.
-cudaError_t launch_direct_mc(const Plan &p, int Q64, int P64, cudaStream_t s);
+// Sign bits of words w0 .. w0 + nw - 1 of z (k_bits.cu); with a job, the launch
+// also fills its coordinate tables and clears the counters (Plan::totals, tsum).
+struct TabArgs {
+    double *tabs;
+    int64_t nx, ny, nz, xoff, nxt;
+    double range[6];
+    int32_t L32, on;
+};
+cudaError_t launch_bits(const Plan &p, int w0, int nw, const TabArgs &ta, int sms, cudaStream_t s);
+// Piece counts of segments seg0 .. seg0 + nseg - 1 from the bits; the last CTA of
+// all segments' launches leaves the totals and the tiles' offsets.
+cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s);
+// Piece counts to offsets within their tile.
+cudaError_t launch_offsets(const Plan &p, cudaStream_t s);
+// Marching Cubes emitted from the bits (k_emit_bits.cu).
+cudaError_t launch_emit_bits_mc(const Plan &p, int Q64, int P64, int seg0, int nseg, cudaStream_t s);
 // Marching Cubes in one walk: classify + stage entries, then expand them.
 constexpr int STG_BLK = 128;  // staging slots a walking warp takes at a time
 cudaError_t launch_walk_mc(const Plan &p, cudaStream_t s);

@@ -759,7 +759,7 @@ int launch_wave(mesh_server *s, Slot &sl) {
             if (rc) return rc;
             // the context's error word of this request
             if (sl.ctx->plan.err &&
-                (e = cudaMemcpyAsync(sl.d_counts + 3 * i + 2, sl.ctx->plan.err, 4, cudaMemcpyDeviceToDevice,
+                (e = cudaMemcpyAsync(sl.d_counts + 3 * i + 2, sl.ctx->plan.err, 4, cudaMemcpyDefault,
                                      sl.stream)) != cudaSuccess)
                 return MESH_ECUDA;
         }

@@ -243,7 +243,7 @@ template <int E> __device__ __forceinline__ uint32_t mt_boundary(const uint32_t 
 
 // CTA: 32 columns (x) by BROW rows of one z segment; warp = row, lane = column.
 template <int ALG>
-__global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, unsigned nblocks) {
+__global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, unsigned nblocks, bool vpre_only) {
     __shared__ __align__(4) uint8_t s_loops[256];
     __shared__ uint2 s_c[BCOL][BROW + 1];
     __shared__ unsigned long long s_w[2][BROW];
@@ -274,6 +274,8 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, uns
         b[0] = r0[1];
         c[0] = r1[0];
         d[0] = r1[1];
+        bool before = true;  // the word before has active cells, or is another segment's
+        uint32_t *vp = ALG == MESH_ALG_MC ? nullptr : p.vpre + (int64_t)(zw0 - v.bw0) * v.sxy + v.nx * y + x;
         for (int zb = zw0; zb < zw1; zb += U) {
 #pragma unroll
             for (int k = 1; k <= U; k++) {
@@ -298,7 +300,10 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, uns
                                      ~(lo_and & __funnelshift_r(lo_and, hi_and, 1)) & zm;
                 lo_or = hi_or;
                 lo_and = hi_and;
-                if (!__any_sync(FULL, act != 0u)) continue;
+                const bool any = __any_sync(FULL, act != 0u);
+                if (ALG != MESH_ALG_MC && (any || before) && xin) vp[(int64_t)(zw - zw0) * v.sxy] = nv;
+                before = any;
+                if (!any) continue;
                 mask |= 1u << ((zw - zw0) & 31);
                 const Corners q{a[k], b[k], c[k], d[k], __funnelshift_r(a[k], a[k + 1], 1),
                                 __funnelshift_r(b[k], b[k + 1], 1), __funnelshift_r(c[k], c[k + 1], 1),
@@ -341,11 +346,12 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, uns
             d[0] = d[U];
             // masks of 32 words (segments start at multiples of U words of them)
             if (((zb - zw0) & 31) == 32 - U || zb + U >= zw1) {
-                if (lane == 0) mo[(zb - zw0) >> 5] = mask;
+                if (lane == 0) mo[(zb - zw0) >> 5] = mask;  // (the same again for vpre_only)
                 mask = 0;
             }
         }
     }
+    if (ALG != MESH_ALG_MC && vpre_only) return;
     s_c[lane][w] = make_uint2(nv, nf);
     __syncthreads();
     {
@@ -536,15 +542,15 @@ cudaError_t launch_bits(const Plan &p, int w0, int nw, const TabArgs &ta, int sm
     }
 }
 
-cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s) {
+cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s, bool vpre_only) {
     const int64_t per = (int64_t)p.nxb * p.nyb, grid = per * nseg, all = per * p.bseg;
     if (all > 0x7fffffff) return cudaErrorInvalidConfiguration;
     if (p.alg == MESH_ALG_MC)
-        k_count<MESH_ALG_MC><<<(unsigned)grid, 32 * BROW, 0, s>>>(p, seg0, (unsigned)all);
+        k_count<MESH_ALG_MC><<<(unsigned)grid, 32 * BROW, 0, s>>>(p, seg0, (unsigned)all, vpre_only);
     else if (p.alg == MESH_ALG_MT)
-        k_count<MESH_ALG_MT><<<(unsigned)grid, 32 * BROW, 0, s>>>(p, seg0, (unsigned)all);
+        k_count<MESH_ALG_MT><<<(unsigned)grid, 32 * BROW, 0, s>>>(p, seg0, (unsigned)all, vpre_only);
     else
-        k_count<MESH_ALG_NSN><<<(unsigned)grid, 32 * BROW, 0, s>>>(p, seg0, (unsigned)all);
+        k_count<MESH_ALG_NSN><<<(unsigned)grid, 32 * BROW, 0, s>>>(p, seg0, (unsigned)all, vpre_only);
     return cudaGetLastError();
 }
 

@@ -126,24 +126,6 @@ template <class P, class O> __device__ __noinline__ O still_slow(double c, doubl
     return (O)Ar<P>::add((P)c, Ar<P>::mul((P)mu, P(0)));
 }
 
-// Three consecutive values in two stores, the pair at the address that allows it.
-__device__ __forceinline__ void put3(float *o, float a, float b, float c) {
-    const bool up = ((uintptr_t)o & 4) != 0;
-    *reinterpret_cast<float2 *>(o + (up ? 1 : 0)) = up ? make_float2(b, c) : make_float2(a, b);
-    o[up ? 0 : 2] = up ? a : c;
-}
-__device__ __forceinline__ void put3(double *o, double a, double b, double c) {
-    const bool up = ((uintptr_t)o & 8) != 0;
-    *reinterpret_cast<double2 *>(o + (up ? 1 : 0)) = up ? make_double2(b, c) : make_double2(a, b);
-    o[up ? 0 : 2] = up ? a : c;
-}
-__device__ __forceinline__ void put3(int64_t *o, long long a, long long b, long long c) {
-    const bool up = ((uintptr_t)o & 8) != 0;
-    *reinterpret_cast<longlong2 *>(o + (up ? 1 : 0)) = up ? make_longlong2(b, c) : make_longlong2(a, b);
-    o[up ? 0 : 2] = up ? a : c;
-}
-__device__ __forceinline__ uint32_t lanemask_le(int lane) { return (2u << lane) - 1u; }
-
 // The crossing on edge `ev` of cell j (column ln, plane z of the word) to `out`.
 template <class T, class Q, class P, int PM>
 __device__ __forceinline__ void put_vertex(const Plan &p, const Tabs &tb, const EmitWarp<T, PM> &w, uint32_t ev, int j,
@@ -202,20 +184,6 @@ __device__ __forceinline__ void put_vertex(const Plan &p, const Tabs &tb, const 
     }
 }
 
-// The eight corner samples of queue entry `ent`, sw at column x0 and the word's
-// first plane (entry 0 is in range: the word has active cells).
-template <class T> __device__ __forceinline__ void load_corners(T (&s)[8], const T *sw, uint32_t ent, const BView &v) {
-    const T *s0 = sw + (ent & 31u) + (int64_t)(ent >> 5) * v.sxy, *s1 = s0 + v.sxy;
-    const T *t0 = s0 + v.nx, *t1 = s1 + v.nx;
-    s[0] = ldv(s0);
-    s[1] = ldv(s0 + 1);
-    s[2] = ldv(t0);
-    s[3] = ldv(t0 + 1);
-    s[4] = ldv(s1);
-    s[5] = ldv(s1 + 1);
-    s[6] = ldv(t1);
-    s[7] = ldv(t1 + 1);
-}
 template <class T, class Q, class P, int PM, bool KEY>
 __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const Tabs &tb, EmitWarp<T, PM> &w,
                                           const CaseTabs &ct, int lane, int xb, int y, int seg) {

@@ -1,4 +1,6 @@
-// K3 (Marching Tetrahedra, Naive Surface Nets) -- emit with neighbour lookups.
+// K3 (Marching Tetrahedra, Naive Surface Nets) -- emit with neighbour lookups, for
+// the allocation-free form (mesh_noalloc.cu): it needs no scratch per sample, where
+// the sign-bit form (k_emit_shared.cu, twice as fast) keeps a quarter of a byte.
 //
 // MT shares vertices between cells: the reference keys every lattice edge in
 // a Dict and numbers a vertex when a cell first touches its edge in

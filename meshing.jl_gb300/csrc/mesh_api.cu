@@ -28,7 +28,6 @@
 namespace mesh {
 cudaError_t launch_classify_tma(const Plan &p, const CUtensorMap &map, cudaStream_t s);
 cudaError_t launch_emit_mc(const Plan &p, int Q64, int P64, int stage, cudaStream_t s);
-cudaError_t launch_emit_halo(const Plan &p, int Q64, int A64, int P64, cudaStream_t s);
 size_t scan_scratch_bytes(const Plan &p);
 }  // namespace mesh
 
@@ -250,12 +249,15 @@ int prepare_bits(mesh_ctx *c) {
     const int nseg = (int)std::min<int64_t>(ncw, std::max<int64_t>(1, (target + rows - 1) / rows));
     segments(std::min(ZWS_MAX, (ncw + nseg - 1) / nseg));
     const size_t word = (size_t)P.nx * P.ny * sizeof(uint32_t);  // one word of every column
-    // the whole volume's words, or windows of whole segments and the word after them
+    // the whole volume's words, or windows of whole segments and the words around them
     int keep = P.nzw;
     cudaError_t e = cudaErrorMemoryAllocation;
     for (;;) {
-        const size_t need = (size_t)(keep == P.nzw ? keep : keep + 1) * word;
-        if (c->bits_max <= 0 || (int64_t)need <= c->bits_max || keep <= 1) e = c->bits.ensure(need);
+        const size_t need = (size_t)(keep == P.nzw ? keep : keep + 2) * word;
+        if (c->bits_max <= 0 || (int64_t)need <= c->bits_max || keep <= 1) {
+            e = c->bits.ensure(need);
+            if (e == cudaSuccess && P.alg != MESH_ALG_MC) e = c->vpre.ensure(need);
+        }
         if (e == cudaSuccess) break;
         cudaGetLastError();
         if (keep <= 1) return cuda_fail(c, e, "sign words");
@@ -278,6 +280,7 @@ int prepare_bits(mesh_ctx *c) {
     P.pc = (uint2 *)c->pc.ptr;
     P.tsum = (ulonglong2 *)c->tsum.ptr;
     P.wmask = (uint32_t *)c->wmask.ptr;
+    P.vpre = (uint32_t *)c->vpre.ptr;
     int64_t *m = (int64_t *)c->misc.ptr;
     P.totals = m;
     P.err = (unsigned int *)(c->h_misc + PIN_ERR);
@@ -286,9 +289,9 @@ int prepare_bits(mesh_ctx *c) {
     return MESH_OK;
 }
 
-// Sign words of the window of segments s0 .. s1 - 1 (and the word after them).
+// Sign words of the window of segments s0 .. s1 - 1 (and the words around them).
 cudaError_t window_bits(mesh_ctx *c, Plan &P, int s0, int s1, bool first) {
-    P.bw0 = s0 * P.zws;
+    P.bw0 = std::max(0, s0 * P.zws - 1);
     P.bw1 = std::min(P.nzw, s1 * P.zws + 1);
     TabArgs ta = c->targs;
     ta.on = first;
@@ -329,16 +332,22 @@ cudaError_t count_bits(mesh_ctx *c) {
 
 // Emission of the column blocks of `q` (slot: its cleared work counter).
 cudaError_t emit_bits(mesh_ctx *c, Plan q, int slot) {
+    const bool mc = q.alg == MESH_ALG_MC;
+    auto emit = [&](int s0, int n) {
+        return mc ? launch_emit_bits_mc(q, c->Q64, c->P64, s0, n, c->stream)
+                  : launch_emit_shared(q, c->Q64, c->A64, c->P64, s0, n, c->stream);
+    };
     if (c->win_segs >= q.bseg && slot < WORK_SLOTS) {
         q.work += 2 * slot;
-        return launch_emit_bits_mc(q, c->Q64, c->P64, 0, q.bseg, c->stream);
+        return emit(0, q.bseg);
     }
     cudaError_t e = cudaSuccess;
     for (int s0 = 0; s0 < q.bseg && e == cudaSuccess; s0 += c->win_segs) {
         const int s1 = std::min(q.bseg, s0 + c->win_segs);
         e = window_bits(c, q, s0, s1, false);
         if (e == cudaSuccess) e = cudaMemsetAsync(q.work, 0, sizeof(unsigned), c->stream);
-        if (e == cudaSuccess) e = launch_emit_bits_mc(q, c->Q64, c->P64, s0, s1 - s0, c->stream);
+        if (e == cudaSuccess && !mc) e = launch_count(q, s0, s1 - s0, c->stream, true);
+        if (e == cudaSuccess) e = emit(s0, s1 - s0);
     }
     return e;
 }
@@ -543,8 +552,9 @@ bool one_walk(const mesh_ctx *c) {
     return c->plan.alg == MESH_ALG_MC && !c->weld && (c->one_walk || c->host_mapped);
 }
 
-// Marching Cubes classified into sign bits and emitted from them (the default).
-bool bits_path(const mesh_ctx *c) { return c->plan.alg == MESH_ALG_MC && !c->list_emit && !one_walk(c); }
+// Classified into sign bits and emitted from them: all but the Marching Cubes forms
+// kept for comparison.
+bool bits_path(const mesh_ctx *c) { return c->plan.alg != MESH_ALG_MC || (!c->list_emit && !one_walk(c)); }
 
 int run_count(mesh_ctx *c) {
     Plan &P = c->plan;
@@ -673,19 +683,15 @@ int launch_emit(mesh_ctx *c) {
         return e != cudaSuccess ? cuda_fail(c, e, "emit launch") : MESH_OK;
     }
     mark(c, 2);
-    if (c->plan.alg == MESH_ALG_MC) e = launch_emit_mc(c->plan, c->Q64, c->P64, 0, c->stream);
-    else e = launch_emit_halo(c->plan, c->Q64, c->A64, c->P64, c->stream);
+    e = launch_emit_mc(c->plan, c->Q64, c->P64, 0, c->stream);
     mark(c, 2);
     count_kernels(c, 2, 1);
     if (e != cudaSuccess) return cuda_fail(c, e, "emit launch");
-    if (c->plan.alg == MESH_ALG_MC) {
-        mark(c, 3);
-        e = launch_emit_mc(c->plan, c->Q64, c->P64, 1, c->stream);
-        mark(c, 3);
-        count_kernels(c, 3, 1);
-        if (e != cudaSuccess) return cuda_fail(c, e, "expand launch");
-    }
-    return MESH_OK;
+    mark(c, 3);
+    e = launch_emit_mc(c->plan, c->Q64, c->P64, 1, c->stream);
+    mark(c, 3);
+    count_kernels(c, 3, 1);
+    return e != cudaSuccess ? cuda_fail(c, e, "expand launch") : MESH_OK;
 }
 
 // Marching Cubes emission into host buffers in K x ranges of whole x tiles.  The
@@ -861,7 +867,8 @@ void mesh_ctx_destroy(mesh_ctx *c) {
     if (c->copy) cudaStreamSynchronize(c->copy);
     DevBuf *bufs[] = {&c->vol,   &c->tabs,  &c->cnt, &c->base, &c->flags,    &c->scan,   &c->misc,
                       &c->out_v, &c->out_f, &c->ent, &c->nrm,  &c->weld_buf, &c->weld_v, &c->gat,
-                      &c->bits, &c->pc,   &c->tsum, &c->wmask};
+                      &c->bits, &c->pc,   &c->tsum, &c->wmask,
+                      &c->vpre};
     for (DevBuf *b : bufs) b->release();
     for (cudaEvent_t e : c->ev_part)
         if (e) cudaEventDestroy(e);
@@ -951,17 +958,16 @@ int run_weld(mesh_ctx *c) {
 namespace {
 // An x window with a halo column (MT / NSN slab after the first): the halo
 // column's vertices and faces come first in the scan and are not emitted, so
-// the counts lose its totals (the scanned base of piece (seg 0, y 0, x 1)).
+// the counts lose its totals (the first vertex and face of piece (x 1, y 0, seg 0)).
 int drop_halo_counts(mesh_ctx *c) {
     const Plan &P = c->plan;
     int64_t v0 = c->nverts, f0 = c->nfaces;  // a window of the halo column alone emits nothing
     if (P.cx > 1) {
         GatherIdx gi{};
-        gi.n = 2;
-        gi.idx[0] = piece(P, 0, 0, 1);
-        gi.idx[1] = P.pstride + piece(P, 0, 0, 1);
+        gi.n = 1;
+        gi.idx[0] = (int64_t)P.cy * P.bseg;
         cudaError_t e = c->gat.ensure(GATHER_MAX * sizeof(int64_t));
-        if (e == cudaSuccess) e = launch_gather(P.base, gi, (int64_t *)c->gat.ptr, c->stream);
+        if (e == cudaSuccess) e = launch_gather_pieces(P, gi, (int64_t *)c->gat.ptr, c->stream);
         int64_t h[2] = {0, 0};
         if (e == cudaSuccess) e = cudaMemcpyAsync(h, c->gat.ptr, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
@@ -1055,7 +1061,7 @@ int mesh_fill(mesh_ctx *c, void *verts, int64_t *faces, int out_on_device) {
     P.verts_cap = c->nverts;
     P.faces_cap = c->nfaces;
     int rc;
-    if (P.alg == MESH_ALG_MC && !one_walk(c) && !c->bits_on && (rc = ensure_entries(c, c->nactive))) return rc;
+    if (!one_walk(c) && !c->bits_on && (rc = ensure_entries(c, c->nactive))) return rc;
     if (!c->bits_on && (e = cudaMemsetAsync(P.err, 0, sizeof(unsigned), c->stream)) != cudaSuccess)
         return cuda_fail(c, e, "memset");
     int parts = 1;
@@ -1107,7 +1113,7 @@ int mesh_extract_device(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t
     if (c->bits_on) P.tot_out = counts;
     // an active Marching Cubes cell emits at least 3 vertices; the one walk
     // also leaves up to a block of slots per warp unused
-    if (P.alg == MESH_ALG_MC && !c->bits_on &&
+    if (!c->bits_on &&
         (rc = ensure_entries(c, P.verts_cap / 3 + (one_walk(c) ? stage_slack(P) : 0))))
         return rc;
     if ((rc = run_count(c))) return rc;

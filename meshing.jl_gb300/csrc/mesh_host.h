@@ -60,11 +60,12 @@ struct mesh_ctx {
     cudaStream_t own = nullptr;
     cudaStream_t stream = nullptr;
     mesh::DevBuf vol, tabs, cnt, base, flags, scan, misc, out_v, out_f, ent;
-    // sign-bit path: sign words, piece counts / offsets, tile sums, activity masks;
+    // sign-bit path: sign words, piece counts / offsets, tile sums, activity masks and
+    // (MT / NSN) the words' vertex prefixes;
     // bits_max caps the sign words (MESHING_GB300_BITS_BYTES; 0: what the device
     // gives): a volume whose words do not fit is classified, and emitted, in
     // windows of win_segs z segments
-    mesh::DevBuf bits, pc, tsum, wmask;
+    mesh::DevBuf bits, pc, tsum, wmask, vpre;
     int64_t bits_max = 0;
     int win_segs = 0;
     int bits_on = 0;  // the current plan takes the sign-bit path

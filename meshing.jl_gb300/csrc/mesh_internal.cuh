@@ -133,6 +133,7 @@ struct Plan {
     uint2 *pc;
     ulonglong2 *tsum;
     uint32_t *wmask;
+    uint32_t *vpre;       // MT / NSN: vertices of a column's segment before word zw, at the words' places
     unsigned int *done;   // CTAs of k_count that have finished
     int64_t npc;
     int64_t *tot_out;     // where k_count also leaves the totals (device or pinned; null: nowhere)
@@ -283,11 +284,14 @@ struct TabArgs {
 cudaError_t launch_bits(const Plan &p, int w0, int nw, const TabArgs &ta, int sms, cudaStream_t s);
 // Piece counts of segments seg0 .. seg0 + nseg - 1 from the bits; the last CTA of
 // all segments' launches leaves the totals and the tiles' offsets.
-cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s);
+cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s, bool vpre_only = false);
+// (vpre_only: leave the words' vertex prefixes alone, for a later window's emission)
 // Piece counts to offsets within their tile.
 cudaError_t launch_offsets(const Plan &p, cudaStream_t s);
 // Marching Cubes emitted from the bits (k_emit_bits.cu).
 cudaError_t launch_emit_bits_mc(const Plan &p, int Q64, int P64, int seg0, int nseg, cudaStream_t s);
+// Marching Tetrahedra / Naive Surface Nets from the bits (k_emit_shared.cu).
+cudaError_t launch_emit_shared(const Plan &p, int Q64, int A64, int P64, int seg0, int nseg, cudaStream_t s);
 // Marching Cubes in one walk: classify + stage entries, then expand them.
 constexpr int STG_BLK = 128;  // staging slots a walking warp takes at a time
 cudaError_t launch_walk_mc(const Plan &p, cudaStream_t s);

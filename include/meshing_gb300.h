@@ -233,9 +233,10 @@ MESH_API int mesh_batch_sync(mesh_batch *b);
  * and first face of volume i (row n holds the totals). */
 MESH_API int mesh_batch_outputs(mesh_batch *b, void **verts, int64_t **faces, int64_t **offsets);
 MESH_API int mesh_batch_set_graph(mesh_batch *b, int enable);
-/* knobs[4]: z cells per work item (0 = whole columns; rounded up to 8),
- * classify and compact CTAs per SM (0 = as many as fit), threads per scan CTA
- * (96..1024, a multiple of 32).  A new first knob needs a new count. */
+/* knobs[4]: z cells per segment (0 = chosen from the batch; rounded up to 32), a
+ * number that is kept and has no effect, CTAs per SM of the emission (0 = as many
+ * as fit), another one without effect (96..1024, a multiple of 32).  A new first
+ * knob needs a new count. */
 MESH_API int mesh_batch_set_knobs(mesh_batch *b, const int *knobs);
 MESH_API int mesh_batch_knobs(const mesh_batch *b, int *knobs);
 /* Autotuner: times `reps` runs of every candidate of one knob at a time,

@@ -1,4 +1,4 @@
-// Sign bits, piece counts and piece offsets (single volumes).
+// Sign bits, piece counts and piece offsets (single volumes and batches).
 //
 // Replaces the classification half of the reference's cell loops
 // (src/marching_cubes.jl:40-56, src/marching_tetrahedra.jl:144-157,
@@ -17,11 +17,13 @@
 //   k_offsets  turns the counts of a tile into offsets within it, in place.
 //
 // Measured (Float32 1024^3): bits 0.606 ms = 7.1 TB/s of volume, bound by HBM;
-// counts 0.123 ms, bound by issue (a word of 32 x 32 cells costs about 25
-// instructions when nothing crosses it, 150 when something does); offsets 6 us.
-// They replaced a walk that classified the volume step by step (0.763 ms, bound by
-// issue) and a four-kernel scan of three counters (35 us; 39 us at 256^3, where
-// these take 3.5 us and the counts 15).
+// counts 0.148 ms, bound by issue (a word of 32 x 32 cells costs about 25
+// instructions when nothing crosses it, 150 when something does); tiles and offsets
+// 18 us.  They replaced a walk that classified the volume step by step (0.763 ms,
+// bound by issue) and a four-kernel scan of three counters (35 us; 39 us at 256^3,
+// where the counts take 15 us and tiles and offsets 9).  A batch of 1024 volumes of
+// 16..128 samples an axis: bits 0.243 ms (6.2 TB/s), counts 0.140, tiles and offsets
+// 0.023, against 0.453 + 0.144 for the batched walk and scan.
 #define MESH_TBL static constexpr
 #include "mesh_internal.cuh"
 #include "mesh_tables.h"
@@ -98,6 +100,17 @@ template <int V> __device__ __forceinline__ void put_words(uint32_t *o, const ui
     }
 }
 
+// Thread t of nt: the counters of a new extraction.
+__device__ __forceinline__ void clear_counters(const Plan &p, int64_t t, int64_t nt) {
+    for (int64_t k = t; k < p.ntiles; k += nt) p.tsum[k] = make_ulonglong2(0ull, 0ull);
+    if (t < NCNT) p.totals[t] = 0;
+    if (t < WORK_SLOTS) p.work[2 * t] = 0u;
+    if (t == 0) {
+        *p.err = 0u;
+        *p.done = 0u;
+    }
+}
+
 // CTA b < nib * nw: 256 V consecutive samples of a plane in word w0 + b / nib;
 // the CTAs after those fill the coordinate tables and clear the counters.
 template <class T, int V>
@@ -105,17 +118,11 @@ __global__ void __launch_bounds__(256) k_bits(const Plan p, int64_t nib, int w0,
     const int64_t nb = nib * nw;
     if ((int64_t)blockIdx.x >= nb) {
         const int64_t t = ((int64_t)blockIdx.x - nb) * 256 + threadIdx.x, nt = ((int64_t)gridDim.x - nb) * 256;
+        clear_counters(p, t, nt);
         const int64_t ntab = ta.nx + ta.ny + ta.nz;
         for (int64_t k = t; k < ntab; k += nt)
             table_entry(ta.tabs, k, ta.nx, ta.ny, ta.nz, ta.range[0], ta.range[1], ta.range[2], ta.range[3],
                         ta.range[4], ta.range[5], ta.L32, ta.xoff, ta.nxt);
-        for (int64_t k = t; k < p.ntiles; k += nt) p.tsum[k] = make_ulonglong2(0ull, 0ull);
-        if (t < NCNT) p.totals[t] = 0;
-        if (t < WORK_SLOTS) p.work[2 * t] = 0u;
-        if (t == 0) {
-            *p.err = 0u;
-            *p.done = 0u;
-        }
         return;
     }
     const int zw = w0 + (int)((int64_t)blockIdx.x / nib);
@@ -125,6 +132,33 @@ __global__ void __launch_bounds__(256) k_bits(const Plan p, int64_t nib, int w0,
     uint32_t w[V];
     pack_words<T, V>(p, (const T *)p.vol + (int64_t)zw * 32 * sxy + i, sxy, (int)min((int64_t)32, p.nz - 32 * (int64_t)zw), w);
     put_words<V>(p.bits + (int64_t)(zw - p.bw0) * sxy + i, w);
+}
+
+// Batch: the CTAs of volume v pack its planes as above (Plan::bblk_vol names the
+// volume); the CTAs after all of them clear the counters.
+template <class T> __global__ void __launch_bounds__(256) k_bits_batch(const Plan p) {
+    if ((int64_t)blockIdx.x >= p.nbblk) {
+        clear_counters(p, ((int64_t)blockIdx.x - p.nbblk) * 256 + threadIdx.x, ((int64_t)gridDim.x - p.nbblk) * 256);
+        return;
+    }
+    const BatchVol &b = p.bvols[p.bblk_vol[blockIdx.x]];
+    constexpr int V = 16 / sizeof(T);
+    const int64_t sxy = b.nx * b.ny, step = b.vec ? 256 * V : 256, nib = (sxy + step - 1) / step;
+    const int64_t k = (int64_t)blockIdx.x - b.bblk0;
+    const int zw = (int)(k / nib), n = (int)min((int64_t)32, b.nz - 32 * (int64_t)zw);
+    const int64_t i = (k % nib) * step + (int64_t)threadIdx.x * (b.vec ? V : 1);
+    if (i >= sxy) return;
+    const T *src = (const T *)b.vol + (int64_t)zw * 32 * sxy + i;
+    uint32_t *dst = p.bits + b.bits0 + (int64_t)zw * sxy + i;
+    if (b.vec) {
+        uint32_t w[V];
+        pack_words<T, V>(p, src, sxy, n, w);
+        put_words<V>(dst, w);
+    } else {
+        uint32_t w[1];
+        pack_words<T, 1>(p, src, sxy, n, w);
+        dst[0] = w[0];
+    }
 }
 
 // ---- piece counts ----
@@ -241,9 +275,66 @@ template <int E> __device__ __forceinline__ uint32_t mt_boundary(const uint32_t 
     return r;
 }
 
-// CTA: 32 columns (x) by BROW rows of one z segment; warp = row, lane = column.
-template <int ALG>
-__global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, unsigned nblocks, bool vpre_only) {
+// The tiles' sums (and the totals), scanned by one CTA of W warps.
+template <int W> __device__ __forceinline__ void scan_tiles(const Plan &p, unsigned long long (*s_w)[W]) {
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int per = (p.ntiles + 32 * W - 1) / (32 * W);
+    const int k0 = min(p.ntiles, tid * per), k1 = min(p.ntiles, k0 + per);
+    unsigned long long sv = 0, sf = 0;
+    for (int k = k0; k < k1; k++) {
+        sv += __ldcg(&p.tsum[k].x);
+        sf += __ldcg(&p.tsum[k].y);
+    }
+    unsigned long long iv = sv, jf = sf;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long u = __shfl_up_sync(FULL, iv, o), t = __shfl_up_sync(FULL, jf, o);
+        if (lane >= o) {
+            iv += u;
+            jf += t;
+        }
+    }
+    if (lane == 31) {
+        s_w[0][w] = iv;
+        s_w[1][w] = jf;
+    }
+    __syncthreads();
+    unsigned long long bv = 0, bf = 0, tv = 0, tf = 0;
+#pragma unroll
+    for (int k = 0; k < W; k++) {
+        if (k < w) {
+            bv += s_w[0][k];
+            bf += s_w[1][k];
+        }
+        tv += s_w[0][k];
+        tf += s_w[1][k];
+    }
+    bv += iv - sv;
+    bf += jf - sf;
+    for (int k = k0; k < k1; k++) {
+        const unsigned long long u = __ldcg(&p.tsum[k].x), t = __ldcg(&p.tsum[k].y);
+        p.tsum[k] = make_ulonglong2(bv, bf);
+        bv += u;
+        bf += t;
+    }
+    if (tid == 0) {
+        p.totals[0] = (int64_t)tv;
+        p.totals[1] = (int64_t)tf;
+        if (p.tot_out) {
+            p.tot_out[0] = (int64_t)tv;
+            p.tot_out[1] = (int64_t)tf;
+        }
+    }
+}
+
+// Item: 32 columns (x) by BROW rows of up to gs z segments (of seg0 .. seg1 - 1; the
+// batches' items are one segment each, Plan::cblk_vol names their volume); warp =
+// row, lane = column; a CTA takes one item.  Where one wave of CTAs holds an
+// extraction, each reports when its sums have arrived and the last of the `all`
+// CTAs scans the tiles' sums; else (all 0) that is a launch of its own, since the
+// wait costs every CTA of a large grid more.
+template <int ALG, bool BATCH>
+__global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, int seg1, int gs, unsigned all, bool vpre_only) {
     __shared__ __align__(4) uint8_t s_loops[256];
     __shared__ uint2 s_c[BCOL][BROW + 1];
     __shared__ unsigned long long s_w[2][BROW];
@@ -254,19 +345,27 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, uns
         static_assert(32 * BROW == 256, "one entry per thread");
         __syncthreads();
     }
-    const BView v = view_of(p);
-    const int xb = (int)(blockIdx.x % v.nxb);
-    const int seg = seg0 + (int)((blockIdx.x / v.nxb) / v.nyb);
-    const int yb = (int)((blockIdx.x / v.nxb) % v.nyb);
+    BView v;
+    unsigned blk = blockIdx.x;
+    if constexpr (BATCH) {
+        const BatchVol &b = p.bvols[p.cblk_vol[blk]];
+        v = view_of(p, b);
+        blk -= (unsigned)b.cblk0;
+    } else {
+        v = view_of(p);
+    }
+    const int xb = (int)(blk % v.nxb);
+    const int sa = seg0 + (int)((blk / v.nxb) / v.nyb) * gs, sb = min(sa + gs, BATCH ? v.nseg : seg1);
+    const int yb = (int)((blk / v.nxb) % v.nyb);
     const int x = xb * BCOL + lane, y = yb * BROW + w;
-    uint32_t nv = 0, nf = 0;
+    uint32_t nv = 0, nf = 0, tv = 0, tf = 0;  // of the segment, of the item's column
     if (y < v.cy) {
         const bool xin = x < v.cx;
-        const int zw0 = seg * v.zws, zw1 = min(zw0 + v.zws, (v.cz + 31) / 32);
+        const int ncw = (v.cz + 31) / 32, zw0 = sa * v.zws, zw1 = min(sb * v.zws, ncw);
+        int seg = sa, zs0 = zw0, zs1 = min(zs0 + v.zws, ncw);  // the segment and its words
         const uint32_t *r0 = v.bits + (int64_t)(zw0 - v.bw0) * v.sxy + v.nx * y + min(x, v.cx - 1);
         const uint32_t *r1 = r0 + v.nx;
         uint32_t mask = 0;
-        uint32_t *mo = p.wmask + bmask(v, seg, y, xb);
         // corner columns at word zw (index 0) and the U words after it, in flight together
         constexpr int U = 4;
         uint32_t a[U + 1], b[U + 1], c[U + 1], d[U + 1];
@@ -303,67 +402,75 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, uns
                 const bool any = __any_sync(FULL, act != 0u);
                 if (ALG != MESH_ALG_MC && (any || before) && xin) vp[(int64_t)(zw - zw0) * v.sxy] = nv;
                 before = any;
-                if (!any) continue;
-                mask |= 1u << ((zw - zw0) & 31);
-                const Corners q{a[k], b[k], c[k], d[k], __funnelshift_r(a[k], a[k + 1], 1),
-                                __funnelshift_r(b[k], b[k + 1], 1), __funnelshift_r(c[k], c[k + 1], 1),
-                                __funnelshift_r(d[k], d[k + 1], 1)};
-                if (ALG == MESH_ALG_MC) {
-                    uint32_t loops = __popc(act);
-                    const uint32_t cross = __popc((q.a ^ q.b) & zm) + __popc((q.c ^ q.d) & zm) + __popc((q.a ^ q.c) & zm) +
-                                           __popc((q.b ^ q.d) & zm) + __popc((q.as ^ q.bs) & zm) +
-                                           __popc((q.cs ^ q.ds) & zm) + __popc((q.as ^ q.cs) & zm) +
-                                           __popc((q.bs ^ q.ds) & zm) + __popc((q.a ^ q.as) & zm) +
-                                           __popc((q.b ^ q.bs) & zm) + __popc((q.c ^ q.cs) & zm) + __popc((q.d ^ q.ds) & zm);
-                    for (uint32_t m = many_loops(q) & zm; m; m &= m - 1)
-                        loops += s_loops[cell_index(a[k], b[k], c[k], d[k], a[k + 1], b[k + 1], c[k + 1], d[k + 1],
-                                                    __ffs(m) - 1)];
-                    nv += cross;
-                    nf += cross - 2 * loops;
-                } else if (ALG == MESH_ALG_MT) {
-                    const MtWords m(q);
-                    uint32_t own = 0;
+                if (any) {
+                    mask |= 1u << ((zw - zs0) & 31);
+                    const Corners q{a[k], b[k], c[k], d[k], __funnelshift_r(a[k], a[k + 1], 1),
+                                    __funnelshift_r(b[k], b[k + 1], 1), __funnelshift_r(c[k], c[k + 1], 1),
+                                    __funnelshift_r(d[k], d[k + 1], 1)};
+                    if (ALG == MESH_ALG_MC) {
+                        uint32_t loops = __popc(act);
+                        const uint32_t cross = __popc((q.a ^ q.b) & zm) + __popc((q.c ^ q.d) & zm) + __popc((q.a ^ q.c) & zm) +
+                                               __popc((q.b ^ q.d) & zm) + __popc((q.as ^ q.bs) & zm) +
+                                               __popc((q.cs ^ q.ds) & zm) + __popc((q.as ^ q.cs) & zm) +
+                                               __popc((q.bs ^ q.ds) & zm) + __popc((q.a ^ q.as) & zm) +
+                                               __popc((q.b ^ q.bs) & zm) + __popc((q.c ^ q.cs) & zm) + __popc((q.d ^ q.ds) & zm);
+                        for (uint32_t m = many_loops(q) & zm; m; m &= m - 1)
+                            loops += s_loops[cell_index(a[k], b[k], c[k], d[k], a[k + 1], b[k + 1], c[k + 1], d[k + 1],
+                                                        __ffs(m) - 1)];
+                        nv += cross;
+                        nf += cross - 2 * loops;
+                    } else if (ALG == MESH_ALG_MT) {
+                        const MtWords m(q);
+                        uint32_t own = 0;
 #pragma unroll
-                    for (int i = 0; i < 8; i++) own += i == 6 ? 0u : __popc((m.w[i] ^ m.w[6]) & zm);
-                    const int low = (x + p.xg0 == 0) | ((y == 0) << 1);
-                    if (zw == 0 || __any_sync(FULL, low != 0)) own += mt_boundary<0>(m.w, zm, zw == 0 ? zm & 1u : 0u, low);
-                    nv += own;
-                    nf += mt_triangles<0>(m.w, zm);
-                } else {
-                    nv += __popc(act);
-                    const uint32_t zk = zw == 0 ? zm & ~1u : zm;  // cells with a -z neighbour
-                    const bool xk = x + p.xg0 > 0, yk = y > 0;
-                    uint32_t n = 0;
-                    if (yk) n += __popc((q.a ^ q.b) & zk);
-                    if (xk) n += __popc((q.a ^ q.c) & zk);
-                    if (xk && yk) n += __popc((q.a ^ q.as) & zm);
-                    nf += 2 * n;
+                        for (int i = 0; i < 8; i++) own += i == 6 ? 0u : __popc((m.w[i] ^ m.w[6]) & zm);
+                        const int low = (x + p.xg0 == 0) | ((y == 0) << 1);
+                        if (zw == 0 || __any_sync(FULL, low != 0)) own += mt_boundary<0>(m.w, zm, zw == 0 ? zm & 1u : 0u, low);
+                        nv += own;
+                        nf += mt_triangles<0>(m.w, zm);
+                    } else {
+                        nv += __popc(act);
+                        const uint32_t zk = zw == 0 ? zm & ~1u : zm;  // cells with a -z neighbour
+                        const bool xk = x + p.xg0 > 0, yk = y > 0;
+                        uint32_t n = 0;
+                        if (yk) n += __popc((q.a ^ q.b) & zk);
+                        if (xk) n += __popc((q.a ^ q.c) & zk);
+                        if (xk && yk) n += __popc((q.a ^ q.as) & zm);
+                        nf += 2 * n;
+                    }
+                }
+                const bool ends = zw + 1 == zs1;
+                if (((zw - zs0) & 31) == 31 || ends) {
+                    if (lane == 0) p.wmask[bmask(v, seg, y, xb) + ((zw - zs0) >> 5)] = mask;
+                    mask = 0;
+                }
+                if (ends) {
+                    if (xin && !vpre_only) p.pc[bpiece(v, seg, y, x)] = make_uint2(nv, nf);
+                    tv += nv;
+                    tf += nf;
+                    nv = nf = 0;
+                    before = true;
+                    seg++;
+                    zs0 = zs1;
+                    zs1 = min(zs0 + v.zws, ncw);
                 }
             }
             a[0] = a[U];
             b[0] = b[U];
             c[0] = c[U];
             d[0] = d[U];
-            // masks of 32 words (segments start at multiples of U words of them)
-            if (((zb - zw0) & 31) == 32 - U || zb + U >= zw1) {
-                if (lane == 0) mo[(zb - zw0) >> 5] = mask;  // (the same again for vpre_only)
-                mask = 0;
-            }
         }
     }
     if (ALG != MESH_ALG_MC && vpre_only) return;
-    s_c[lane][w] = make_uint2(nv, nf);
+    s_c[lane][w] = make_uint2(tv, tf);
     __syncthreads();
     {
-        // BROW consecutive rows of one column are consecutive pieces (of one segment)
+        // the tiles' sums: the pieces of a column's BROW rows mostly share one
         const int xl = tid / BROW, yl = tid % BROW;
         const int X = xb * BCOL + xl, Y = yb * BROW + yl;
         const bool in = X < v.cx && Y < v.cy;
-        uint2 n = s_c[xl][yl];
-        const int64_t e = bpiece(v, seg, Y, X);
-        if (in) p.pc[e] = n;
-        else n = make_uint2(0u, 0u);
-        const int64_t e0 = bpiece(v, seg, yb * BROW, X), e1 = bpiece(v, seg, min(yb * BROW + BROW, v.cy) - 1, X);
+        const uint2 n = in ? s_c[xl][yl] : make_uint2(0u, 0u);
+        const int64_t e0 = bpiece(v, sa, yb * BROW, X), e1 = bpiece(v, sb - 1, min(yb * BROW + BROW, v.cy) - 1, X);
         unsigned long long sv = n.x, sf = n.y;
 #pragma unroll
         for (int o = BROW / 2; o; o >>= 1) {
@@ -376,64 +483,28 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, uns
                 atomicAdd(&p.tsum[e0 / BITS_TILE].y, sf);
             }
         } else if (in && (n.x | n.y)) {
-            atomicAdd(&p.tsum[e / BITS_TILE].x, (unsigned long long)n.x);
-            atomicAdd(&p.tsum[e / BITS_TILE].y, (unsigned long long)n.y);
+            for (int q = sa; q < sb; q++) {
+                const int64_t e = bpiece(v, q, Y, X);
+                const uint2 c = __ldcg(&p.pc[e]);
+                atomicAdd(&p.tsum[e / BITS_TILE].x, (unsigned long long)c.x);
+                atomicAdd(&p.tsum[e / BITS_TILE].y, (unsigned long long)c.y);
+            }
         }
     }
-    // the last CTA scans the tiles' sums
+    if (all == 0u) return;
     __threadfence();
     __syncthreads();
-    if (tid == 0) s_last = atomicAdd(p.done, 1u) == nblocks - 1;
+    if (tid == 0) s_last = atomicAdd(p.done, 1u) == all - 1;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    const int per = (p.ntiles + 32 * BROW - 1) / (32 * BROW);
-    const int k0 = min(p.ntiles, tid * per), k1 = min(p.ntiles, k0 + per);
-    unsigned long long sv = 0, sf = 0;
-    for (int k = k0; k < k1; k++) {
-        sv += __ldcg(&p.tsum[k].x);
-        sf += __ldcg(&p.tsum[k].y);
-    }
-    unsigned long long iv = sv, jf = sf;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned long long u = __shfl_up_sync(FULL, iv, o), t = __shfl_up_sync(FULL, jf, o);
-        if (lane >= o) {
-            iv += u;
-            jf += t;
-        }
-    }
-    if (lane == 31) {
-        s_w[0][w] = iv;
-        s_w[1][w] = jf;
-    }
-    __syncthreads();
-    unsigned long long bv = 0, bf = 0, tv = 0, tf = 0;
-#pragma unroll
-    for (int k = 0; k < BROW; k++) {
-        if (k < w) {
-            bv += s_w[0][k];
-            bf += s_w[1][k];
-        }
-        tv += s_w[0][k];
-        tf += s_w[1][k];
-    }
-    bv += iv - sv;
-    bf += jf - sf;
-    for (int k = k0; k < k1; k++) {
-        const unsigned long long u = __ldcg(&p.tsum[k].x), t = __ldcg(&p.tsum[k].y);
-        p.tsum[k] = make_ulonglong2(bv, bf);
-        bv += u;
-        bf += t;
-    }
-    if (tid == 0) {
-        p.totals[0] = (int64_t)tv;
-        p.totals[1] = (int64_t)tf;
-        if (p.tot_out) {
-            p.tot_out[0] = (int64_t)tv;
-            p.tot_out[1] = (int64_t)tf;
-        }
-    }
+    scan_tiles<BROW>(p, s_w);
+}
+
+// The tiles' sums to offsets, for grids that do not scan them themselves.
+__global__ void __launch_bounds__(1024) k_scan_tiles(const Plan p) {
+    __shared__ unsigned long long s_w[2][32];
+    scan_tiles<32>(p, s_w);
 }
 
 // ---- piece offsets ----
@@ -497,6 +568,22 @@ __global__ void __launch_bounds__(OFF_T) k_offsets(const Plan p) {
     }
 }
 
+// Batch: first vertex / face of every volume, then the totals.
+__global__ void __launch_bounds__(256) k_batch_rows(const Plan p) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i > p.nvols) return;
+    const int64_t e = i < p.nvols ? p.bvols[i].e0 : p.npc;
+    int64_t vo = p.totals[0], fo = p.totals[1];
+    if (e < p.npc) {
+        const ulonglong2 t = p.tsum[e / BITS_TILE];
+        const uint2 o = p.pc[e];
+        vo = (int64_t)(t.x + o.x);
+        fo = (int64_t)(t.y + o.y);
+    }
+    p.vol_off[2 * (int64_t)i] = vo;
+    p.vol_off[2 * (int64_t)i + 1] = fo;
+}
+
 __global__ void k_gather_pieces(const Plan p, const GatherIdx g, int64_t *dst) {
     const int i = threadIdx.x;
     if (i >= g.n) return;
@@ -542,19 +629,62 @@ cudaError_t launch_bits(const Plan &p, int w0, int nw, const TabArgs &ta, int sm
     }
 }
 
+// CTAs of k_count that 152 SMs hold at once.
+constexpr int ONE_WAVE = 456;
+
+template <int ALG, bool BATCH>
+static cudaError_t go_count(const Plan &p, int seg0, int nseg, bool vpre_only, cudaStream_t s) {
+    const int64_t per = (int64_t)p.nxb * p.nyb;
+    // segments to an item: as many as leave 2048 items
+    const int gs = BATCH ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(nseg, per * nseg / 2048));
+    const int64_t nitems = BATCH ? p.ncblk : per * ((nseg + gs - 1) / gs);
+    const bool one = nitems <= ONE_WAVE && (BATCH || nseg == p.bseg);
+    if (nitems > 0x7fffffff) return cudaErrorInvalidConfiguration;
+    if (nitems > 0)
+        k_count<ALG, BATCH><<<(unsigned)nitems, 32 * BROW, 0, s>>>(p, seg0, seg0 + nseg, gs, one ? (unsigned)nitems : 0u,
+                                                                 vpre_only);
+    if (!one && !vpre_only && (BATCH || seg0 + nseg == p.bseg)) k_scan_tiles<<<1, 1024, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s, bool vpre_only) {
-    const int64_t per = (int64_t)p.nxb * p.nyb, grid = per * nseg, all = per * p.bseg;
-    if (all > 0x7fffffff) return cudaErrorInvalidConfiguration;
-    if (p.alg == MESH_ALG_MC)
-        k_count<MESH_ALG_MC><<<(unsigned)grid, 32 * BROW, 0, s>>>(p, seg0, (unsigned)all, vpre_only);
-    else if (p.alg == MESH_ALG_MT)
-        k_count<MESH_ALG_MT><<<(unsigned)grid, 32 * BROW, 0, s>>>(p, seg0, (unsigned)all, vpre_only);
-    else
-        k_count<MESH_ALG_NSN><<<(unsigned)grid, 32 * BROW, 0, s>>>(p, seg0, (unsigned)all, vpre_only);
+    if (p.alg == MESH_ALG_MC) return go_count<MESH_ALG_MC, false>(p, seg0, nseg, vpre_only, s);
+    if (p.alg == MESH_ALG_MT) return go_count<MESH_ALG_MT, false>(p, seg0, nseg, vpre_only, s);
+    return go_count<MESH_ALG_NSN, false>(p, seg0, nseg, vpre_only, s);
+}
+
+template <class T> static cudaError_t go_bits_batch(const Plan &p, cudaStream_t s) {
+    const int64_t grid = p.nbblk + std::min<int64_t>((p.ntiles + 255) / 256 + 1, 64);
+    if (grid > 0x7fffffff) return cudaErrorInvalidConfiguration;
+    k_bits_batch<T><<<(unsigned)grid, 256, 0, s>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_bits_batch(const Plan &p, cudaStream_t s) {
+    switch (p.T) {
+    case MESH_DT_U16: return go_bits_batch<uint16_t>(p, s);
+    case MESH_DT_F16: return go_bits_batch<h16>(p, s);
+    case MESH_DT_I16: return go_bits_batch<int16_t>(p, s);
+    case MESH_DT_I8: return go_bits_batch<int8_t>(p, s);
+    case MESH_DT_U8: return go_bits_batch<uint8_t>(p, s);
+    case MESH_DT_F32: return go_bits_batch<float>(p, s);
+    case MESH_DT_I32: return go_bits_batch<int32_t>(p, s);
+    case MESH_DT_I64: return go_bits_batch<int64_t>(p, s);
+    default: return go_bits_batch<double>(p, s);
+    }
+}
+
+cudaError_t launch_count_batch(const Plan &p, cudaStream_t s) {
+    return go_count<MESH_ALG_MC, true>(p, 0, 0, false, s);
+}
+
+cudaError_t launch_batch_rows(const Plan &p, cudaStream_t s) {
+    k_batch_rows<<<p.nvols / 256 + 1, 256, 0, s>>>(p);
     return cudaGetLastError();
 }
 
 cudaError_t launch_offsets(const Plan &p, cudaStream_t s) {
+    if (p.ntiles < 1) return cudaSuccess;
     k_offsets<<<(unsigned)p.ntiles, OFF_T, 0, s>>>(p);
     return cudaGetLastError();
 }

@@ -1,4 +1,4 @@
-// Marching Cubes emission from the sign bits (single volumes).
+// Marching Cubes emission from the sign bits (single volumes and batches).
 //
 // Replaces process_mc_voxel! (src/marching_cubes.jl:67-92), vertex_interp
 // (:100-104) and mc_vert_points (:111-120): vertices and faces are written
@@ -29,7 +29,9 @@
 // 0.126 against 0.163 ms.  Of the 0.89 ms, leaving out the face stores saves 0.20,
 // the vertices 0.27, the task look-ups 0.12 and the batch set-up 0.19; leaving out
 // the corner loads alone 0.06 (512^3: 950 instructions per batch, 63% of issue).
-// Three CTAs per SM: with four (64 registers) it is 4% slower, with five 13%.
+// Three CTAs per SM: with four (64 registers) it is 4% slower, with five 13%.  A
+// batch of 1024 volumes (1.5 GB of samples): 0.383 ms against 0.575 for listing the
+// active cells and expanding the list.
 #define MESH_TBL static constexpr
 #include "mesh_internal.cuh"
 #include "mesh_tables.h"
@@ -184,9 +186,19 @@ __device__ __forceinline__ void put_vertex(const Plan &p, const Tabs &tb, const 
     }
 }
 
-template <class T, class Q, class P, int PM, bool KEY>
-__device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const Tabs &tb, EmitWarp<T, PM> &w,
-                                          const CaseTabs &ct, int lane, int xb, int y, int seg) {
+// Where an item's mesh goes: buffers and their room, what the scanned offsets lose
+// to index them (v0, f0), what vertex ids lose beyond that (id0: batches number the
+// vertices of each volume from 1) and the volume's first edge key.
+struct OutView {
+    char *verts;
+    int64_t *faces;
+    long long vcap, fcap, v0, f0, id0, kbase;
+};
+
+// b: the item's volume of a batch (null: the plan's single volume).
+template <class T, class Q, class P, int PM, bool BATCH>
+__device__ __forceinline__ void emit_item(const Plan &p, const BatchVol *b, const BView &v, const Tabs &tb,
+                                          EmitWarp<T, PM> &w, const CaseTabs &ct, int lane, int xb, int y, int seg) {
     constexpr int VB = 3 * (PM == PM_F64 ? 8 : 4);  // bytes of a vertex
     const int mw = mask_words(min(v.zws, (v.cz + 31) / 32 - seg * v.zws));
     const uint32_t *mp = p.wmask + bmask(v, seg, y, xb);
@@ -196,18 +208,27 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
     bool ready = false;            // the item's offsets and x, y nodes are loaded
     bool zeroxy = false;
     long long gv = 0, gf = 0;      // this column's next vertex / face
+    OutView out{(char *)p.verts, p.faces, p.verts_cap, p.faces_cap, 0, 0, 0, 0};
     const uint32_t *r0 = v.bits + (int64_t)(zws0 - v.bw0) * v.sxy + v.nx * y + min(x, v.cx - 1);
     const T *s0 = (const T *)v.vol + v.nx * y + x0;
     for (int q = 0; q < mw; q++) {
         uint32_t todo = __ldg(mp + q);
         if (todo && !ready) {
             ready = true;
+            if constexpr (BATCH) {
+                const ulonglong2 t = p.tsum[v.e0 / BITS_TILE];
+                const uint2 o = p.pc[v.e0];
+                const long long v0 = (long long)t.x + o.x, f0 = (long long)t.y + o.y;
+                if (p.vol_outputs) out = OutView{(char *)b->verts, b->faces, b->vcap, b->fcap, v0, f0, 0, 0};
+                else out.id0 = v0;
+                if (p.vkey) out.kbase = b->kbase;
+            }
             if (xin) {
                 const int64_t e = bpiece(v, seg, y, x);
                 const ulonglong2 t = p.tsum[e / BITS_TILE];
                 const uint2 o = p.pc[e];
-                gv = (long long)t.x + o.x;
-                gf = (long long)t.y + o.y;
+                gv = (long long)t.x + o.x - out.v0;
+                gf = (long long)t.y + o.y - out.f0;
             }
             __syncwarp();  // the previous item's tasks are done with the node table
             bool z = false;
@@ -273,7 +294,7 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                 const long long g0 = gv - (long long)(tl & 0xffffu), f0 = gf - (long long)(tl >> 16);
                 gv = g0 + (th & 0xffffu);
                 gf = f0 + (th >> 16);
-                const bool fit = __all_sync(FULL, gv <= p.verts_cap && gf <= p.faces_cap);
+                const bool fit = __all_sync(FULL, gv <= out.vcap && gf <= out.fcap);
                 w.iv[lane] = g0;
                 w.jf[lane] = f0;
 #pragma unroll
@@ -297,10 +318,10 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                     if (t < VW) {
                         const int cl = (int)((rec >> 8) & 31u), cz = (int)((rec >> 13) & 31u);
                         const uint32_t ev = ct.ev[(rec & 255u) * MC_MAX_VERTS + (t - (int)(rec >> 18))];
-                        const long long out = w.iv[cl] + t;
-                        if (fit || out < p.verts_cap) {
-                            put_vertex<T, Q, P, PM>(p, tb, w, ev, j, cl, cz, x0, y, z0, zero, (char *)p.verts + VB * out);
-                            if (KEY) {
+                        const long long at = w.iv[cl] + t;
+                        if (fit || at < out.vcap) {
+                            put_vertex<T, Q, P, PM>(p, tb, w, ev, j, cl, cz, x0, y, z0, zero, out.verts + VB * at);
+                            if (p.vkey) {
                                 // the edge's lower node; the cell owns the edge when, across
                                 // each other axis, the edge lies on the cell's upper side or
                                 // the cell is first
@@ -310,8 +331,9 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                                 const bool own = (ax == 0 || ox || cx == 0) && (ax == 1 || oy || y == 0) &&
                                                  (ax == 2 || oz || cw == 0);
                                 const long long key =
-                                    ax + 3 * ((long long)(cx + ox) + v.nx * ((long long)(y + oy) + v.ny * (long long)(cw + oz)));
-                                p.vkey[out] = key | (own ? (long long)(1ull << 63) : 0ll);
+                                    out.kbase + ax +
+                                    3 * ((long long)(cx + ox) + v.nx * ((long long)(y + oy) + v.ny * (long long)(cw + oz)));
+                                p.vkey[at] = key | (own ? (long long)(1ull << 63) : 0ll);
                             }
                         } else {
                             *p.err = ERR_CAPACITY;
@@ -327,9 +349,10 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                     if (t < FW) {
                         const int cl = (int)((rec >> 8) & 31u);
                         const uint32_t sf = ct.ef[(rec & 255u) * MC_MAX_FACES + (t - (int)(rec >> 22))];
-                        const long long out = w.jf[cl] + t, vb = w.iv[cl] + 1 + (long long)((rec >> 13) & 511u);  // 1-based
-                        if (fit || out < p.faces_cap)
-                            put3(p.faces + 3 * out, vb + (sf & 15u), vb + ((sf >> 4) & 15u), vb + ((sf >> 8) & 15u));
+                        const long long at = w.jf[cl] + t;
+                        const long long vb = w.iv[cl] + 1 - out.id0 + (long long)((rec >> 13) & 511u);  // 1-based
+                        if (fit || at < out.fcap)
+                            put3(out.faces + 3 * at, vb + (sf & 15u), vb + ((sf >> 4) & 15u), vb + ((sf >> 8) & 15u));
                         else
                             *p.err = ERR_CAPACITY;
                     }
@@ -340,7 +363,7 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
     }
 }
 
-template <class T, class Q, class P, int PM, bool KEY>
+template <class T, class Q, class P, int PM>
 __global__ void __launch_bounds__(32 * EW, 3) k_emit_bits_mc(const Plan p, int seg0, int nseg, int nitems) {
     extern __shared__ __align__(16) unsigned char esm[];
     CaseTabs &ct = *reinterpret_cast<CaseTabs *>(esm);
@@ -360,75 +383,139 @@ __global__ void __launch_bounds__(32 * EW, 3) k_emit_bits_mc(const Plan p, int s
         const int xb = p.tx0 + item % nxb;
         const int seg = seg0 + (item / nxb) % nseg;
         const int y = item / (nxb * nseg);
-        emit_item<T, Q, P, PM, KEY>(p, v, tb, sw[wi], ct, lane, xb, y, seg);
+        emit_item<T, Q, P, PM, false>(p, nullptr, v, tb, sw[wi], ct, lane, xb, y, seg);
     }
 }
 
-// Resident CTAs of a kernel on the current device, with its dynamic shared memory
-// allowed (one-time per device and instantiation).
-template <class T, class Q, class P, int PM, bool KEY> int emit_grid() {
+// Batch: an item is `rows` rows (1, 2, 4 or 8) of an item of k_count (Plan::cblk_vol
+// names its volume).  Four rows fetch the descriptor and their masks once; batches
+// too small for eight such items per warp take single rows.
+constexpr int BITEM = 4;
+static_assert(BROW % BITEM == 0, "whole items per item of k_count");
+template <class T, class Q, class P, int PM>
+__global__ void __launch_bounds__(32 * EW, 3) k_emit_bits_batch(const Plan p, int64_t nitems, int rows) {
+    extern __shared__ __align__(16) unsigned char esm[];
+    CaseTabs &ct = *reinterpret_cast<CaseTabs *>(esm);
+    EmitWarp<T, PM> *sw = reinterpret_cast<EmitWarp<T, PM> *>(esm + sizeof(CaseTabs));
+    for (int i = threadIdx.x; i < (int)(sizeof(CaseTabs) / 16); i += blockDim.x)
+        reinterpret_cast<uint4 *>(&ct)[i] = reinterpret_cast<const uint4 *>(&d_cases)[i];
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    for (;;) {
+        unsigned item = 0;
+        if (lane == 0) item = atomicAdd(p.work, 1u);
+        item = __shfl_sync(FULL, item, 0);
+        if ((int64_t)item >= nitems) break;
+        const unsigned per = BROW / rows, blk = item / per;
+        const BatchVol *b = p.bvols + p.cblk_vol[blk];
+        const BView v = view_of(p, *b);
+        const unsigned k = blk - (unsigned)b->cblk0;
+        const int xb = (int)(k % v.nxb), seg = (int)((k / v.nxb) / v.nyb);
+        const int y0 = (int)((k / v.nxb) % v.nyb) * BROW + (int)(item % per) * rows;
+        uint32_t any = 0;
+        if (lane < rows && y0 + lane < v.cy) {
+            const uint32_t *mp = p.wmask + bmask(v, seg, y0 + lane, xb);
+            const int mw = mask_words(min(v.zws, (v.cz + 31) / 32 - seg * v.zws));
+            for (int q = 0; q < mw; q++) any |= __ldg(mp + q);
+        }
+        const Tabs tb = tabs_at(b->tabs, v.nx, v.ny, v.nz);
+        for (uint32_t todo = __ballot_sync(FULL, any != 0u); todo; todo &= todo - 1)
+            emit_item<T, Q, P, PM, true>(p, b, v, tb, sw[wi], ct, lane, xb, y0 + __ffs(todo) - 1, seg);
+    }
+}
+
+// Resident CTAs per SM of a kernel on the current device, with its dynamic shared
+// memory allowed (one-time per device and instantiation), and the device's SMs.
+template <class T, class Q, class P, int PM, bool BATCH> int emit_ctas(int *sms) {
     static std::mutex mu;
-    static int grid[64] = {0};
+    static int ctas[64] = {0}, nsm[64] = {0};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return 0;
     std::lock_guard<std::mutex> lk(mu);
-    if (!grid[dev]) {
-        const void *fn = (const void *)k_emit_bits_mc<T, Q, P, PM, KEY>;
+    if (!ctas[dev]) {
+        const void *fn = BATCH ? (const void *)k_emit_bits_batch<T, Q, P, PM> : (const void *)k_emit_bits_mc<T, Q, P, PM>;
         const int smem = (int)emit_smem<T, PM>();
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        int sms = 0, per_sm = 0;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        int per_sm = 0;
+        cudaDeviceGetAttribute(&nsm[dev], cudaDevAttrMultiProcessorCount, dev);
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * EW, smem) != cudaSuccess || per_sm < 1)
             per_sm = 1;
         cudaGetLastError();
-        grid[dev] = per_sm * sms;
+        ctas[dev] = per_sm;
     }
-    return grid[dev];
+    *sms = nsm[dev];
+    return ctas[dev];
 }
 
-template <class T, class Q, class P, int PM, bool KEY>
-cudaError_t go_k(const Plan &p, int seg0, int nseg, cudaStream_t s) {
-    const int grid = emit_grid<T, Q, P, PM, KEY>();
+// What a launch covers: segments of a single volume, or a batch (ctas per SM).
+struct Range {
+    int seg0, nseg, batch, ctas;
+};
+
+template <class T, class Q, class P, int PM> cudaError_t go_batch(const Plan &p, int ctas, cudaStream_t s) {
+    int sms = 0;
+    const int fit = emit_ctas<T, Q, P, PM, true>(&sms);
+    const int64_t grid = (int64_t)sms * (ctas > 0 ? std::min(ctas, fit) : fit);
+    const int rows = p.ncblk * (BROW / BITEM) >= 8 * EW * grid ? BITEM : 1;
+    const int64_t nitems = p.ncblk * (BROW / rows);
+    if (grid < 1) return cudaErrorInvalidDevice;
+    if (nitems > 0x7fffffff) return cudaErrorInvalidConfiguration;
+    if (nitems < 1) return cudaSuccess;
+    k_emit_bits_batch<T, Q, P, PM>
+        <<<(int)std::min<int64_t>(grid, (nitems + EW - 1) / EW), 32 * EW, emit_smem<T, PM>(), s>>>(p, nitems, rows);
+    return cudaGetLastError();
+}
+
+template <class T, class Q, class P, int PM> cudaError_t go(const Plan &p, const Range &r, cudaStream_t s) {
+    if (r.batch) return go_batch<T, Q, P, PM>(p, r.ctas, s);
+    const int seg0 = r.seg0, nseg = r.nseg;
+    int sms = 0;
+    const int grid = emit_ctas<T, Q, P, PM, false>(&sms) * sms;
     const int64_t nitems = (int64_t)(p.ntx > 0 ? p.ntx : p.nxb) * nseg * p.cy;
     if (grid < 1) return cudaErrorInvalidDevice;
     if (nitems > 0x7fffffff - 65536) return cudaErrorInvalidConfiguration;
     if (nitems < 1) return cudaSuccess;
-    k_emit_bits_mc<T, Q, P, PM, KEY><<<(int)std::min<int64_t>(grid, (nitems + EW - 1) / EW), 32 * EW, emit_smem<T, PM>(), s>>>(
+    k_emit_bits_mc<T, Q, P, PM><<<(int)std::min<int64_t>(grid, (nitems + EW - 1) / EW), 32 * EW, emit_smem<T, PM>(), s>>>(
         p, seg0, nseg, (int)nitems);
     return cudaGetLastError();
 }
-template <class T, class Q, class P, int PM> cudaError_t go(const Plan &p, int seg0, int nseg, cudaStream_t s) {
-    return p.vkey ? go_k<T, Q, P, PM, true>(p, seg0, nseg, s) : go_k<T, Q, P, PM, false>(p, seg0, nseg, s);
-}
-
-template <class T> cudaError_t go_t(const Plan &p, int Q64, int P64, int seg0, int nseg, cudaStream_t s) {
+template <class T> cudaError_t go_t(const Plan &p, int Q64, int P64, const Range &r, cudaStream_t s) {
     if (p.out64) {
-        if (Q64) return go<T, double, double, PM_F64>(p, seg0, nseg, s);
-        return go<T, float, double, PM_F64>(p, seg0, nseg, s);
+        if (Q64) return go<T, double, double, PM_F64>(p, r, s);
+        return go<T, float, double, PM_F64>(p, r, s);
     }
-    if (Q64) return go<T, double, double, PM_MIX>(p, seg0, nseg, s);  // integer data, Int iso, Float32 ranges
-    if (P64) return go<T, float, double, PM_MIX>(p, seg0, nseg, s);
-    return go<T, float, float, PM_F32>(p, seg0, nseg, s);
+    if (Q64) return go<T, double, double, PM_MIX>(p, r, s);  // integer data, Int iso, Float32 ranges
+    if (P64) return go<T, float, double, PM_MIX>(p, r, s);
+    return go<T, float, float, PM_F32>(p, r, s);
 }
 
 }  // namespace
+
+static cudaError_t launch(const Plan &p, int Q64, int P64, const Range &r, cudaStream_t s) {
+    switch (p.T) {
+    case MESH_DT_U16: return go_t<uint16_t>(p, Q64, P64, r, s);
+    case MESH_DT_F16: return go_t<h16>(p, Q64, P64, r, s);
+    case MESH_DT_I16: return go_t<int16_t>(p, Q64, P64, r, s);
+    case MESH_DT_I8: return go_t<int8_t>(p, Q64, P64, r, s);
+    case MESH_DT_U8: return go_t<uint8_t>(p, Q64, P64, r, s);
+    case MESH_DT_F32: return go_t<float>(p, Q64, P64, r, s);
+    case MESH_DT_I32: return go_t<int32_t>(p, Q64, P64, r, s);
+    case MESH_DT_I64: return go_t<int64_t>(p, Q64, P64, r, s);
+    default: return go<double, double, double, PM_F64>(p, r, s);
+    }
+}
 
 // Marching Cubes emission of segments seg0 .. seg0 + nseg - 1 of a single volume
 // (bits, masks and offsets from k_bits.cu); column blocks tx0 .. tx0 + ntx - 1 when
 // ntx > 0.  Plan::work is a cleared counter.
 cudaError_t launch_emit_bits_mc(const Plan &p, int Q64, int P64, int seg0, int nseg, cudaStream_t s) {
-    switch (p.T) {
-    case MESH_DT_U16: return go_t<uint16_t>(p, Q64, P64, seg0, nseg, s);
-    case MESH_DT_F16: return go_t<h16>(p, Q64, P64, seg0, nseg, s);
-    case MESH_DT_I16: return go_t<int16_t>(p, Q64, P64, seg0, nseg, s);
-    case MESH_DT_I8: return go_t<int8_t>(p, Q64, P64, seg0, nseg, s);
-    case MESH_DT_U8: return go_t<uint8_t>(p, Q64, P64, seg0, nseg, s);
-    case MESH_DT_F32: return go_t<float>(p, Q64, P64, seg0, nseg, s);
-    case MESH_DT_I32: return go_t<int32_t>(p, Q64, P64, seg0, nseg, s);
-    case MESH_DT_I64: return go_t<int64_t>(p, Q64, P64, seg0, nseg, s);
-    default: return go<double, double, double, PM_F64>(p, seg0, nseg, s);
-    }
+    return launch(p, Q64, P64, Range{seg0, nseg, 0, 0}, s);
+}
+
+// Emission of a batch.
+cudaError_t launch_emit_batch(const Plan &p, int Q64, int P64, int ctas, cudaStream_t s) {
+    return launch(p, Q64, P64, Range{0, 0, 1, ctas}, s);
 }
 
 }  // namespace mesh

@@ -45,15 +45,13 @@ struct CompactSmem {
     long long bv[WARPS][WY][32], bf[WARPS][WY][32];
 };
 
-// Entries of warp tile (tx, ty) of z segment seg; with a batch, each entry
-// also records its volume `vol`.  The activity bytes of 32 chunks are read at
+// Entries of warp tile (tx, ty) of z segment seg.  The activity bytes of 32 chunks are read at
 // once and the walk visits only the active chunks.  Inside a chunk a step whose corners are not all on one side costs,
 // per cell row, one lookup of the case's packed word (mesh_case.cuh); the
 // lanes whose cell is active write its entry at the piece's entry offset plus
 // the entries before it in the chunk (bits 23.. of the running word).
 template <class T, int NR>
-__device__ __forceinline__ void compact_tile(const Plan &p, CompactSmem &sm, int w, int lane, int tx, int ty, int seg,
-                                             uint32_t vol) {
+__device__ __forceinline__ void compact_tile(const Plan &p, CompactSmem &sm, int w, int lane, int tx, int ty, int seg) {
     const T *volp = (const T *)p.vol;
     const int64_t sxy = p.nx * p.ny;
     const int64_t np = p.pstride;
@@ -168,7 +166,6 @@ __device__ __forceinline__ void compact_tile(const Plan &p, CompactSmem &sm, int
                                     p.ent_cs[e] = sm.cs[idx];
                                     const T cv[8] = {l0, l1, L1, L0, h0, h1, H1, H0};
                                     store8<T>((T *)p.ent_val + 8 * e, cv);
-                                    if (p.ent_vol) p.ent_vol[e] = vol;
                                     if ((e & (ENT_BLOCK - 1)) == 0) {
                                         p.ent_side[2 * (e / ENT_BLOCK)] =
                                             sm.bv[w][r][lane] + (pk[r] & ((1u << PK_F) - 1u));
@@ -223,7 +220,6 @@ __global__ void __launch_bounds__(256, COMPACT_MIN_CTAS) k_compact_mc(const Plan
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int tiles_y = (p.cy + CR - 1) / CR;
-    const int ntx = p.ntx > 0 ? p.ntx : p.tiles_x;  // x tiles tx0 .. tx0 + ntx - 1
     // persistent warps: take (y tile, x tile, segment) items in order from a counter
     for (;;) {
         int item = 0;
@@ -231,34 +227,9 @@ __global__ void __launch_bounds__(256, COMPACT_MIN_CTAS) k_compact_mc(const Plan
         item = __shfl_sync(FULL, item, 0);
         if (item >= nitems) break;
         const int ty = item % tiles_y;
-        const int tx = p.tx0 + (item / tiles_y) % ntx;
-        const int seg = item / (tiles_y * ntx);
-        compact_tile<T, CR>(p, sm, w, lane, tx, ty, seg, 0);
-    }
-}
-
-// Batch: the work items of k_classify_batch, in the same order, each split
-// into its WY / CR tiles of CR cell rows.
-template <class T>
-__global__ void __launch_bounds__(256, COMPACT_MIN_CTAS) k_compact_batch(const Plan p) {
-    static_assert(WY % CR == 0, "compaction tiles split the classify tile");
-    constexpr int SUB = WY / CR;
-    __shared__ CompactSmem sm;
-    load_tables_mc_packed(sm.pk, sm.cs);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (;;) {
-        unsigned item = 0;  // p.nitems * SUB < 2^31 (checked when the batch is planned)
-        if (lane == 0) item = atomicAdd(p.work, 1u);
-        item = __shfl_sync(FULL, item, 0);
-        if ((int64_t)(item / SUB) >= p.nitems) break;
-        const uint32_t v = p.item_vol[item / SUB];
-        const BatchVol b = p.bvols[v];
-        const int64_t local = (int64_t)(item / SUB) - b.item0;
-        const int ty = (int)(local % b.tiles_y);
-        const int tx = (int)((local / b.tiles_y) % b.tiles_x);
-        const int seg = (int)(local / ((int64_t)b.tiles_y * b.tiles_x));
-        compact_tile<T, CR>(vol_view(p, b), sm, w, lane, tx, ty * SUB + (int)(item % SUB), seg, v);
+        const int tx = (item / tiles_y) % p.tiles_x;
+        const int seg = item / (tiles_y * p.tiles_x);
+        compact_tile<T, CR>(p, sm, w, lane, tx, ty, seg);
     }
 }
 
@@ -284,7 +255,7 @@ template <class T, class Q, class P> cudaError_t go(const Plan &p, int stage, cu
     int grid_a = 0, grid_b = 0;
     list_grids<T, Q, P>(&grid_a, &grid_b);
     if (stage == 0) {
-        const int nitems = (p.ntx > 0 ? p.ntx : p.tiles_x) * ((p.cy + CR - 1) / CR) * p.nseg;
+        const int nitems = p.tiles_x * ((p.cy + CR - 1) / CR) * p.nseg;
         cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(unsigned), s);
         if (e != cudaSuccess) return e;
         k_compact_mc<T><<<std::min(grid_a, (nitems + WARPS - 1) / WARPS), 32 * WARPS, 0, s>>>(p, nitems);
@@ -300,70 +271,9 @@ template <class T> cudaError_t go_t(const Plan &p, int Q64, int P64, int stage, 
     return go<T, float, float>(p, stage, s);
 }
 
-int persistent_ctas(const void *fn, int threads, int ctas_per_sm) {
-    int dev = 0, sms = 0, fit = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, fn, threads, 0) != cudaSuccess || fit < 1) {
-        cudaGetLastError();
-        fit = 1;
-    }
-    return sms * (ctas_per_sm > 0 ? std::min(ctas_per_sm, fit) : fit);
-}
-
-template <class T> cudaError_t compact_batch_t(const Plan &p, int ctas, cudaStream_t s) {
-    const int grid = (int)std::min<int64_t>(persistent_ctas((const void *)k_compact_batch<T>, 32 * WARPS, ctas),
-                                            (p.nitems * (WY / CR) + WARPS - 1) / WARPS);
-    cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(unsigned), s);
-    if (e != cudaSuccess || grid < 1) return e;
-    k_compact_batch<T><<<grid, 32 * WARPS, 0, s>>>(p);
-    return cudaGetLastError();
-}
-
-template <class T, class Q, class P> cudaError_t expand_batch_t(const Plan &p, cudaStream_t s) {
-    // per instantiation: resident CTAs on this device (thread-safe one-time initialisation)
-    static const int grid = expand_ctas((const void *)k_expand_mc<T, Q, P, EXP_BATCH>);
-    k_expand_mc<T, Q, P, EXP_BATCH><<<grid, XW, 0, s>>>(p);
-    return cudaGetLastError();
-}
-
-template <class T> cudaError_t expand_batch_tt(const Plan &p, int Q64, int P64, cudaStream_t s) {
-    if (Q64) return expand_batch_t<T, double, double>(p, s);
-    if (P64) return expand_batch_t<T, float, double>(p, s);
-    return expand_batch_t<T, float, float>(p, s);
-}
-
 }  // namespace
 
-cudaError_t launch_compact_batch(const Plan &p, int ctas, cudaStream_t s) {
-    switch (p.T) {
-    case MESH_DT_U16: return compact_batch_t<uint16_t>(p, ctas, s);
-    case MESH_DT_F16: return compact_batch_t<h16>(p, ctas, s);
-    case MESH_DT_I16: return compact_batch_t<int16_t>(p, ctas, s);
-    case MESH_DT_I8: return compact_batch_t<int8_t>(p, ctas, s);
-    case MESH_DT_U8: return compact_batch_t<uint8_t>(p, ctas, s);
-    case MESH_DT_F32: return compact_batch_t<float>(p, ctas, s);
-    case MESH_DT_I32: return compact_batch_t<int32_t>(p, ctas, s);
-    case MESH_DT_I64: return compact_batch_t<int64_t>(p, ctas, s);
-    default: return compact_batch_t<double>(p, ctas, s);
-    }
-}
-
-cudaError_t launch_expand_batch(const Plan &p, int Q64, int P64, cudaStream_t s) {
-    switch (p.T) {
-    case MESH_DT_U16: return expand_batch_tt<uint16_t>(p, Q64, P64, s);
-    case MESH_DT_F16: return expand_batch_tt<h16>(p, Q64, P64, s);
-    case MESH_DT_I16: return expand_batch_tt<int16_t>(p, Q64, P64, s);
-    case MESH_DT_I8: return expand_batch_tt<int8_t>(p, Q64, P64, s);
-    case MESH_DT_U8: return expand_batch_tt<uint8_t>(p, Q64, P64, s);
-    case MESH_DT_F32: return expand_batch_tt<float>(p, Q64, P64, s);
-    case MESH_DT_I32: return expand_batch_tt<int32_t>(p, Q64, P64, s);
-    case MESH_DT_I64: return expand_batch_tt<int64_t>(p, Q64, P64, s);
-    default: return expand_batch_t<double, double, double>(p, s);
-    }
-}
-
-// stage 0: K3a compact (active-cell list); stage 1: K3b expand (vertices and faces)
+// stage 0: the list of active cells; stage 1: their vertices and faces.
 cudaError_t launch_emit_mc(const Plan &p, int Q64, int P64, int stage, cudaStream_t s) {
     switch (p.T) {
     case MESH_DT_U16: return go_t<uint16_t>(p, Q64, P64, stage, s);

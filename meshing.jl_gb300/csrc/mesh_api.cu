@@ -7,8 +7,6 @@
 // Base.lerpi arithmetic (k_tables.cu), and the kernels run on the context's
 // stream: classify -> scan -> emit.  Nothing waits on the host between
 // launches.  Device scratch grows monotonically and is reused across calls.
-#include <cuda.h>
-#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -23,10 +21,8 @@
 #include "mesh_host.h"
 #include "mesh_internal.cuh"
 #include "mesh_tables.h"
-#include "mesh_tma.cuh"
 
 namespace mesh {
-cudaError_t launch_classify_tma(const Plan &p, const CUtensorMap &map, cudaStream_t s);
 cudaError_t launch_emit_mc(const Plan &p, int Q64, int P64, int stage, cudaStream_t s);
 size_t scan_scratch_bytes(const Plan &p);
 }  // namespace mesh
@@ -202,33 +198,6 @@ int ensure_pipe(mesh_ctx *c) {
     return MESH_OK;
 }
 
-// Host volume upload in c->ngroups groups of z segments on the copy stream, each
-// group classified on the compute stream as soon as it has arrived: group g holds
-// the sample planes its segments read (segment s reads planes s*zs ..
-// min((s+1)*zs, cz)).  Copies and launches are enqueued alternately, so that a
-// pageable source (whose copies return only once staged) overlaps too.
-cudaError_t upload_and_classify(mesh_ctx *c) {
-    const Plan &P = c->plan;
-    const size_t plane = (size_t)P.nx * P.ny * dtype_size(P.T);
-    cudaError_t e = cudaEventRecord(c->ev_ready, c->stream);  // earlier work on the volume buffer
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(c->copy, c->ev_ready, 0);
-    int64_t p0 = 0;
-    int s0 = 0;
-    for (int g = 0; g < c->ngroups && e == cudaSuccess; g++) {
-        const int s1 = (int)((int64_t)(g + 1) * P.nseg / c->ngroups);
-        const int64_t p1 = g + 1 == c->ngroups ? P.nz : std::min<int64_t>((int64_t)s1 * P.zs, P.nz - 1) + 1;
-        if (p1 > p0)
-            e = cudaMemcpyAsync((char *)c->vol.ptr + p0 * plane, (const char *)c->upl_src + p0 * plane,
-                                (size_t)(p1 - p0) * plane, cudaMemcpyHostToDevice, c->copy);
-        if (e == cudaSuccess) e = cudaEventRecord(c->ev_part[g], c->copy);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(c->stream, c->ev_part[g], 0);
-        if (e == cudaSuccess && s1 > s0) e = launch_classify(P, c->stream, s0, s1 - s0);
-        p0 = std::max(p0, p1);
-        s0 = s1;
-    }
-    return e;
-}
-
 bool one_walk(const mesh_ctx *c);
 bool bits_path(const mesh_ctx *c);
 
@@ -379,14 +348,7 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
     const int64_t per_seg = (int64_t)P.tiles_x * P.tiles_y;
     const int64_t target = (int64_t)c->sms * 64;
     const int maxseg = (P.cz + ZC - 1) / ZC;
-    int nseg = (int)std::min<int64_t>(maxseg, std::max<int64_t>(1, (target + per_seg - 1) / per_seg));
-    // a host volume uploaded in groups of z segments (upload_and_classify) gets at
-    // least PIPE_MAX segments, so that all but the last group's classification
-    // runs under the upload (a mapped host volume read in place is not uploaded)
-    const size_t vbytes0 = (size_t)nx * ny * nz * dtype_size(T);
-    if (!vol_on_device && !c->zerocopy && c->pipe_bytes > 0 && (int64_t)vbytes0 >= c->pipe_bytes && c->tma_env != 1 &&
-        !c->one_walk)
-        nseg = std::min(maxseg, std::max(nseg, PIPE_MAX));
+    const int nseg = (int)std::min<int64_t>(maxseg, std::max<int64_t>(1, (target + per_seg - 1) / per_seg));
     int zs = (P.cz + nseg - 1) / nseg;
     zs = (zs + ZC - 1) / ZC * ZC;
     P.zs = zs;
@@ -412,10 +374,10 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
         cudaGetLastError();
         if ((e = c->vol.ensure(vbytes)) != cudaSuccess) return cuda_fail(c, e, "volume buffer");
         P.vol = c->vol.ptr;
-        if (c->pipe_bytes > 0 && (int64_t)vbytes >= c->pipe_bytes && P.nseg >= 2 && c->tma_env != 1 && !c->one_walk) {
+        if (c->pipe_bytes > 0 && (int64_t)vbytes >= c->pipe_bytes && bits_path(c) && nz > 32) {
             int rc = ensure_pipe(c);
             if (rc) return rc;
-            c->ngroups = std::min(PIPE_MAX, P.nseg);  // the count uploads and classifies
+            c->ngroups = (int)std::min<int64_t>(PIPE_MAX, (nz + 31) / 32);  // the count uploads and classifies
             c->upl_src = vol;
         } else if ((e = cudaMemcpyAsync(c->vol.ptr, vol, vbytes, cudaMemcpyHostToDevice, c->stream)) != cudaSuccess) {
             return cuda_fail(c, e, "volume upload");
@@ -444,8 +406,7 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
     if (c->bits_on) {
         const int rc = prepare_bits(c);
         if (rc == MESH_OK && c->ngroups > 1) {
-            c->ngroups = std::min(PIPE_MAX, P.nzw);
-            if (c->win_segs < P.bseg || c->ngroups < 2) {  // windows: the volume goes up first
+            if (c->win_segs < P.bseg) {  // windows: the volume goes up first
                 c->ngroups = 1;
                 if ((e = cudaMemcpyAsync(c->vol.ptr, vol, vbytes, cudaMemcpyHostToDevice, c->stream)) != cudaSuccess)
                     return cuda_fail(c, e, "volume upload");
@@ -505,46 +466,6 @@ void mark(mesh_ctx *c, int stage) {
     c->ev_pairs[stage].push_back(e);
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-    // thread-safe one-time lookup
-    static const PFN_cuTensorMapEncodeTiled_v12000 fn = []() -> PFN_cuTensorMapEncodeTiled_v12000 {
-        cudaDriverEntryPointQueryResult q;
-        void *f = nullptr;
-        const bool ok = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault,
-                                                         &q) == cudaSuccess &&
-                        q == cudaDriverEntryPointSuccess;
-        cudaGetLastError();
-        return ok ? (PFN_cuTensorMapEncodeTiled_v12000)f : nullptr;
-    }();
-    return fn;
-}
-
-// Tensor map of the volume for the TMA walk: rows must start on 16-byte
-// boundaries and the volume must be at least one box large.
-bool make_tensor_map(mesh_ctx *c) {
-    const Plan &P = c->plan;
-    if (!(c->tma_env == 1 || (c->tma_env < 0 && P.alg == MESH_ALG_MC))) return false;
-    int bx;
-    size_t es;
-    CUtensorMapDataType dt;
-    switch (P.T) {
-    case MESH_DT_U16: bx = TmaBox<uint16_t>::BX; es = 2; dt = CU_TENSOR_MAP_DATA_TYPE_UINT16; break;
-    case MESH_DT_F32: bx = TmaBox<float>::BX; es = 4; dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT32; break;
-    case MESH_DT_F64: bx = TmaBox<double>::BX; es = 8; dt = CU_TENSOR_MAP_DATA_TYPE_FLOAT64; break;
-    default: return false;  // integer and Float16 volumes take the load walk
-    }
-    if (((uintptr_t)P.vol & 15) || ((size_t)P.nx * es) % 16 || P.nx < bx || P.ny < TMA_BY || P.nz < TMA_BZ) return false;
-    PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
-    if (!enc) return false;
-    const cuuint64_t dims[3] = {(cuuint64_t)P.nx, (cuuint64_t)P.ny, (cuuint64_t)P.nz};
-    const cuuint64_t strides[2] = {(cuuint64_t)P.nx * es, (cuuint64_t)P.nx * P.ny * es};
-    const cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)TMA_BY, (cuuint32_t)TMA_BZ};
-    const cuuint32_t elem[3] = {1, 1, 1};
-    return enc(&c->tmap, dt, 3, const_cast<void *>(P.vol), dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) ==
-           CUDA_SUCCESS;
-}
-
 // Marching Cubes walked once, classification staging the active cells (opt-in;
 // also the form that reads a mapped host volume in place).
 // (welded meshes need the expansion in emission order, which writes the edge keys)
@@ -578,23 +499,11 @@ int run_count(mesh_ctx *c) {
     }
     if ((e = cudaMemsetAsync(c->misc.ptr, 0, MISC_SLOTS * sizeof(int64_t), c->stream)) != cudaSuccess)
         return cuda_fail(c, e, "memset");
-    // the pipelined upload classifies each group with the load walk as it arrives
-    c->use_tma = !one_walk(c) && c->ngroups == 1 && make_tensor_map(c);
     mark(c, 0);
-    int nlaunch = 1;
-    if (one_walk(c)) {
-        e = launch_walk_mc(P, c->stream);
-    } else if (c->use_tma) {
-        e = launch_classify_tma(P, c->tmap, c->stream);
-    } else if (c->ngroups > 1) {
-        e = upload_and_classify(c);
-        nlaunch = c->ngroups;
-    } else {
-        e = launch_classify(P, c->stream);
-    }
+    e = one_walk(c) ? launch_walk_mc(P, c->stream) : launch_classify(P, c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "classify launch");
     mark(c, 0);
-    count_kernels(c, 0, nlaunch);
+    count_kernels(c, 0, 1);
     mark(c, 1);
     if ((e = launch_scan(P, c->stream)) != cudaSuccess) return cuda_fail(c, e, "scan launch");
     mark(c, 1);
@@ -604,8 +513,6 @@ int run_count(mesh_ctx *c) {
 
 int check_err(mesh_ctx *c) {
     const unsigned err = (unsigned)c->h_misc[NCNT];
-    if (err & ERR_SCAN_TIMEOUT) return fail(c, MESH_EDEVICE, "scan look-back wait expired");
-    if (err & ERR_TMA_TIMEOUT) return fail(c, MESH_EDEVICE, "TMA stage wait expired");
     if (err & ERR_BOUNDS) return fail(c, MESH_EDEVICE, "device bounds check failed");
     if (err & (ERR_CAPACITY | ERR_STAGE)) return fail(c, MESH_ECAPACITY, "output capacity too small");
     return MESH_OK;
@@ -703,66 +610,39 @@ int launch_emit(mesh_ctx *c) {
 // destination still overlaps the copies with the emission.
 int emit_pipelined(mesh_ctx *c, int K, void *verts, int64_t *faces) {
     const Plan &P = c->plan;
-    const int64_t np = P.pstride;
     const size_t vsz = (size_t)3 * (P.out64 ? 8 : 4);
     int tx[PIPE_MAX + 1];
-    const int blocks = c->bits_on ? P.nxb : P.tiles_x;
-    for (int g = 0; g <= K; g++) tx[g] = (int)((int64_t)g * blocks / K);
-    const int per = c->bits_on ? 2 : 3;  // values per split point
+    for (int g = 0; g <= K; g++) tx[g] = (int)((int64_t)g * P.nxb / K);
     GatherIdx gi{};
-    cudaError_t e;
-    if (c->bits_on) {
-        gi.n = K - 1;
-        for (int g = 1; g < K; g++) gi.idx[g - 1] = (int64_t)tx[g] * BCOL * P.cy * P.bseg;
-        e = launch_gather_pieces(P, gi, (int64_t *)c->gat.ptr, c->stream);
-    } else {
-        gi.n = 3 * (K - 1);
-        for (int g = 1; g < K; g++) {
-            const int64_t i = piece(P, 0, 0, tx[g] * TILE_X);
-            for (int k = 0; k < 3; k++) gi.idx[3 * (g - 1) + k] = k * np + i;
-        }
-        e = launch_gather(P.base, gi, (int64_t *)c->gat.ptr, c->stream);
-    }
+    gi.n = K - 1;
+    for (int g = 1; g < K; g++) gi.idx[g - 1] = (int64_t)tx[g] * BCOL * P.cy * P.bseg;
+    cudaError_t e = launch_gather_pieces(P, gi, (int64_t *)c->gat.ptr, c->stream);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(c->h_gat, c->gat.ptr, (size_t)per * (K - 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
+        e = cudaMemcpyAsync(c->h_gat, c->gat.ptr, (size_t)2 * (K - 1) * sizeof(int64_t), cudaMemcpyDeviceToHost,
                             c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "split points");
-    int64_t V[PIPE_MAX + 1], F[PIPE_MAX + 1], E[PIPE_MAX + 1];
-    V[0] = F[0] = E[0] = 0;
+    int64_t V[PIPE_MAX + 1], F[PIPE_MAX + 1];
+    V[0] = F[0] = 0;
     V[K] = c->nverts;
     F[K] = c->nfaces;
-    E[K] = c->nactive;
     for (int g = 1; g < K; g++) {
-        V[g] = c->h_gat[per * (g - 1)];
-        F[g] = c->h_gat[per * (g - 1) + 1];
-        E[g] = per == 3 ? c->h_gat[per * (g - 1) + 2] : 0;
+        V[g] = c->h_gat[2 * (g - 1)];
+        F[g] = c->h_gat[2 * (g - 1) + 1];
     }
     for (int g = 0; g < K; g++)
-        if (V[g] > V[g + 1] || F[g] > F[g + 1] || E[g] > E[g + 1] || V[g + 1] > c->nverts || F[g + 1] > c->nfaces)
+        if (V[g] > V[g + 1] || F[g] > F[g + 1] || V[g + 1] > c->nverts || F[g + 1] > c->nfaces)
             return fail(c, MESH_EDEVICE, "inconsistent split points");
-    int nexp = 0;
     mark(c, 2);
     for (int g = 0; g < K && e == cudaSuccess; g++) {
         Plan q = P;
         q.tx0 = tx[g];
         q.ntx = tx[g + 1] - tx[g];
-        q.e_lo = E[g];
-        q.e_hi = E[g + 1];
-        if (c->bits_on) {
-            e = emit_bits(c, q, g);
-        } else {
-            e = launch_emit_mc(q, c->Q64, c->P64, 0, c->stream);
-            if (e == cudaSuccess && E[g + 1] > E[g]) {
-                e = launch_emit_mc(q, c->Q64, c->P64, 1, c->stream);
-                nexp++;
-            }
-        }
+        e = emit_bits(c, q, g);
         if (e == cudaSuccess) e = cudaEventRecord(c->ev_part[g], c->stream);
     }
     mark(c, 2);
     count_kernels(c, 2, K);
-    count_kernels(c, 3, nexp);
     if (e != cudaSuccess) return cuda_fail(c, e, "emit launch");
     for (int g = 0; g < K && e == cudaSuccess; g++) {
         e = cudaStreamWaitEvent(c->copy, c->ev_part[g], 0);
@@ -846,8 +726,6 @@ int mesh_ctx_create(int device, mesh_ctx **out) {
     if (bb && bb[0]) c->bits_max = strtoll(bb, nullptr, 10);
     const char *ff = getenv("MESHING_GB300_FORCE_FP64");
     c->force_fp64 = ff && ff[0] == '1';
-    const char *wt = getenv("MESHING_GB300_TMA");
-    c->tma_env = (wt && wt[0] == '1') ? 1 : (wt && wt[0] == '0') ? 0 : -1;
     const char *ow = getenv("MESHING_GB300_ONE_WALK");
     c->one_walk = ow && ow[0] == '1';
     const char *le = getenv("MESHING_GB300_LIST_EMIT");
@@ -1065,10 +943,10 @@ int mesh_fill(mesh_ctx *c, void *verts, int64_t *faces, int out_on_device) {
     if (!c->bits_on && (e = cudaMemsetAsync(P.err, 0, sizeof(unsigned), c->stream)) != cudaSuccess)
         return cuda_fail(c, e, "memset");
     int parts = 1;
-    if (!out_on_device && P.alg == MESH_ALG_MC && !one_walk(c) && c->pipe_bytes > 0 &&
-        (int64_t)(vb + fbytes) >= c->pipe_bytes && (c->bits_on ? P.nxb : P.tiles_x) >= 2) {
+    if (!out_on_device && P.alg == MESH_ALG_MC && c->bits_on && c->pipe_bytes > 0 &&
+        (int64_t)(vb + fbytes) >= c->pipe_bytes && P.nxb >= 2) {
         if ((rc = ensure_pipe(c))) return rc;
-        parts = std::min(PIPE_MAX, c->bits_on ? P.nxb : P.tiles_x);
+        parts = std::min(PIPE_MAX, P.nxb);
     }
     if (parts > 1) {
         if ((rc = emit_pipelined(c, parts, verts, faces))) return rc;

@@ -1,21 +1,20 @@
 // Batched Marching Cubes behind the C ABI (mesh_batch_* in include/meshing_gb300.h).
 //
-// Many volumes of uneven shape are extracted by one pass of each stage over a
-// flattened worklist instead of one launch sequence per volume:
-//   classify  persistent warps over all volumes' warp tiles (k_classify_batch)
-//   scan      one decoupled look-back chain over all volumes' scan tiles, so
-//             the volumes' meshes are concatenated in volume order, plus the
-//             first vertex / face of every volume (k_scan_batch)
-//   compact   persistent warps list the active cells (k_compact_batch)
-//   expand    vertices and faces, faces 1-based within their volume
+// Many volumes of uneven shape are extracted by one pass of each stage over all of
+// them instead of one launch sequence per volume (k_bits.cu, k_emit_bits.cu):
+//   bits      every volume's sign words; a CTA packs 32 planes of one volume
+//   counts    pieces of all volumes in one array, so that one offset scan
+//             concatenates the volumes' meshes in volume order
+//   emission  persistent warps over all volumes' rows, faces 1-based within
+//             their volume
 // Each volume gives the same vertices and faces, in the same order, as a call
 // of isosurface(A_i, MarchingCubes(iso), X_i, Y_i, Z_i) on it alone
 // (src/marching_cubes.jl:27-64).
 //
 // The run after a count can be captured once into a CUDA graph and replayed.
-// The autotuner times the whole sequence over a small set of brick depths
-// (z cells per work item), persistent CTAs per SM and scan CTA widths, one
-// knob at a time, and keeps the fastest.
+// The autotuner times the whole sequence over a small set of segment depths (z
+// cells) and CTAs per SM of the persistent emission, one knob at a time, and keeps
+// the fastest.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -37,16 +36,17 @@ struct mesh_batch {
     std::vector<const void *> vols;
     std::vector<int64_t> dims;    // [n][3]
     std::vector<double> ranges;   // [n][6]
-    // tunables
-    int zs = 0;                   // z cells per work item, a multiple of ZC; 0 = whole columns
-    int cls_ctas = 0, cmp_ctas = 0;  // CTAs per SM of the persistent kernels; 0 = as many as fit
+    // tunables: z cells per segment (0 = whole columns) and CTAs per SM of the
+    // emission (0 = as many as fit).  cls_ctas and scan_threads are taken and given
+    // back: the kernels that they sized are gone.
+    int zs = 0;
+    int cls_ctas = 0, cmp_ctas = 0;
     int scan_threads = 1024;
-    bool scan_vol = false;        // every volume at most 4 column groups wide: the per-volume scan
     Plan P{};
     std::vector<BatchVol> hv;
-    DevBuf dvols, ivol, svol, tabs, jobs, cnt, base, flags, scan, misc, ent, out_v, out_f, offs;
+    DevBuf dvols, bvol, cvol, tabs, jobs, bits, pc, tsum, wmask, misc, out_v, out_f, offs;
     int64_t *h_misc = nullptr;    // pinned copy of the misc words
-    int64_t nverts = 0, nfaces = 0, nactive = 0;
+    int64_t nverts = 0, nfaces = 0;
     int counted = 0;
     int use_graph = 0;
     // welded batches: the per-cell mesh goes to out_v / out_f, its edge keys to
@@ -61,34 +61,43 @@ struct mesh_batch {
 
 namespace mesh {
 
-BatchSizes tile_batch(const int64_t *dims, int n, int zs, std::vector<BatchVol> &hv, std::vector<int64_t> &tab_off) {
+BatchSizes tile_batch(const void *const *vols, size_t es, const int64_t *dims, int n, int zs, std::vector<BatchVol> &hv,
+                      std::vector<int64_t> &tab_off) {
     BatchSizes z;
+    // zs 0: whole columns, or in batches of few columns the segments that give a
+    // device of 152 SMs some 400 rows of 32 columns per SM to emit
+    int64_t rows = 0;
+    for (int v = 0; v < n; v++)
+        if (dims[3 * v] > 1 && dims[3 * v + 1] > 1 && dims[3 * v + 2] > 1)
+            rows += (dims[3 * v] - 2 + BCOL) / BCOL * (dims[3 * v + 1] - 1);
+    const int64_t cuts = std::max<int64_t>(1, ((int64_t)1 << 16) / std::max<int64_t>(rows, 1));
     hv.assign(n, BatchVol{});
     tab_off.assign(n, 0);
     for (int v = 0; v < n; v++) {
         BatchVol &bv = hv[v];
-        const int64_t nx = dims[3 * v], ny = dims[3 * v + 1], nz = dims[3 * v + 2];
+        const int64_t nx = dims[3 * v], ny = dims[3 * v + 1], nz = dims[3 * v + 2], sxy = nx * ny;
+        bv.vol = vols[v];
         bv.nx = nx; bv.ny = ny; bv.nz = nz;
-        bv.item0 = z.items; bv.piece0 = z.pieces; bv.flag0 = z.nflags; bv.stile0 = (int32_t)z.stiles;
+        bv.bits0 = z.words; bv.e0 = z.pieces; bv.m0 = z.masks; bv.bblk0 = z.bblks; bv.cblk0 = z.cblks;
         bv.kbase = z.keys;
         z.keys += 3 * nx * ny * nz;
         tab_off[v] = z.tdoubles;
-        if (nx < 2 || ny < 2 || nz < 2) {  // no cells: an empty mesh
-            bv.zs = ZC; bv.chunks_per_seg = 1;
-            continue;
-        }
+        if (nx < 2 || ny < 2 || nz < 2) continue;  // no cells: an empty mesh
         bv.cx = (int32_t)(nx - 1); bv.cy = (int32_t)(ny - 1); bv.cz = (int32_t)(nz - 1);
-        bv.tiles_x = (bv.cx + TILE_X - 1) / TILE_X;
-        bv.tiles_y = (bv.cy + WY - 1) / WY;
-        const int whole = (bv.cz + ZC - 1) / ZC * ZC;
-        bv.zs = zs > 0 ? std::min(whole, (zs + ZC - 1) / ZC * ZC) : whole;
-        bv.nseg = (bv.cz + bv.zs - 1) / bv.zs;
-        bv.chunks_per_seg = bv.zs / ZC;
-        bv.nchunks = bv.nseg * bv.chunks_per_seg;
-        z.items += (int64_t)bv.tiles_x * bv.tiles_y * bv.nseg;
-        z.pieces += (int64_t)bv.nseg * bv.cy * bv.cx;
-        z.nflags += (int64_t)bv.nchunks * bv.tiles_x * bv.cy;
-        z.stiles += (bv.cx + 31) / 32;
+        bv.nxb = (bv.cx + BCOL - 1) / BCOL;
+        bv.nyb = (bv.cy + BROW - 1) / BROW;
+        bv.nzw = (int32_t)((nz + 31) / 32);
+        const int ncw = (bv.cz + 31) / 32, whole = std::min(ncw, ZWS_MAX);
+        bv.zws = zs > 0 ? std::min(whole, (zs + 31) / 32) : std::min<int>(whole, (int)((ncw + cuts - 1) / cuts));
+        bv.bseg = (ncw + bv.zws - 1) / bv.zws;
+        // 16-byte loads where the planes allow them and fill a CTA
+        const int64_t per = (int64_t)(256 * 16 / es);
+        bv.vec = ((uintptr_t)vols[v] & 15) == 0 && (sxy * es) % 16 == 0 && sxy >= per;
+        z.bblks += (bv.vec ? (sxy + per - 1) / per : (sxy + 255) / 256) * bv.nzw;
+        z.cblks += (int64_t)bv.nxb * bv.nyb * bv.bseg;
+        z.words += (sxy * bv.nzw + 3) / 4 * 4;  // every volume's words on a 16-byte boundary
+        z.pieces += (int64_t)bv.cx * bv.cy * bv.bseg;
+        z.masks += (int64_t)bv.bseg * bv.cy * bv.nxb * mask_words(bv.zws);
         const int64_t ntab = nx + ny + nz;
         z.max_ntab = std::max(z.max_ntab, ntab);
         z.tdoubles += (int64_t)((table_bytes(ntab) + 255) / 256 * 32);  // 256-byte aligned blocks
@@ -96,18 +105,44 @@ BatchSizes tile_batch(const int64_t *dims, int n, int zs, std::vector<BatchVol> 
     return z;
 }
 
-void batch_owners(const std::vector<BatchVol> &hv, const BatchSizes &z, std::vector<uint32_t> &ivol,
-                  std::vector<uint32_t> &svol) {
-    ivol.resize((size_t)z.items);
-    svol.resize((size_t)z.stiles);
+void batch_owners(const std::vector<BatchVol> &hv, const BatchSizes &z, std::vector<uint32_t> &bvol,
+                  std::vector<uint32_t> &cvol) {
+    bvol.resize((size_t)z.bblks);
+    cvol.resize((size_t)z.cblks);
     for (size_t v = 0; v < hv.size(); v++) {
-        const BatchVol &bv = hv[v];
-        if (!bv.cx) continue;
-        const int64_t ni = (int64_t)bv.tiles_x * bv.tiles_y * bv.nseg;
-        std::fill(ivol.begin() + bv.item0, ivol.begin() + bv.item0 + ni, (uint32_t)v);
-        const int ns = (bv.cx + 31) / 32;
-        std::fill(svol.begin() + bv.stile0, svol.begin() + bv.stile0 + ns, (uint32_t)v);
+        const bool last = v + 1 == hv.size();
+        std::fill(bvol.begin() + hv[v].bblk0, last ? bvol.end() : bvol.begin() + hv[v + 1].bblk0, (uint32_t)v);
+        std::fill(cvol.begin() + hv[v].cblk0, last ? cvol.end() : cvol.begin() + hv[v + 1].cblk0, (uint32_t)v);
     }
+}
+
+void bind_batch(Plan &P, const BatchSizes &z, int n, const BatchBufs &b) {
+    P.bvols = (const BatchVol *)b.vols;
+    P.bblk_vol = (const uint32_t *)b.bvol;
+    P.cblk_vol = (const uint32_t *)b.cvol;
+    P.nbblk = z.bblks;
+    P.ncblk = z.cblks;
+    P.nvols = n;
+    P.bits = (uint32_t *)b.bits;
+    P.pc = (uint2 *)b.pc;
+    P.tsum = (ulonglong2 *)b.tsum;
+    P.wmask = (uint32_t *)b.wmask;
+    P.npc = z.pieces;
+    P.ntiles = (int32_t)z.tiles();
+    P.vol_off = (int64_t *)b.offs;
+    int64_t *m = (int64_t *)b.misc;
+    P.totals = m;
+    P.err = (unsigned int *)(m + NCNT);
+    P.done = (unsigned int *)(m + MISC_DONE);
+    P.work = (unsigned int *)(m + MISC_WORK);
+}
+
+cudaError_t launch_batch_counts(const Plan &P, cudaStream_t s) {
+    cudaError_t e = launch_bits_batch(P, s);
+    if (e == cudaSuccess) e = launch_count_batch(P, s);
+    if (e == cudaSuccess) e = launch_offsets(P, s);
+    if (e == cudaSuccess) e = launch_batch_rows(P, s);
+    return e;
 }
 
 }  // namespace mesh
@@ -130,32 +165,28 @@ int build_plan(mesh_batch *b) {
     const int L32 = b->prm.range_type == MESH_DT_F32;
     const int n = b->n;
     std::vector<int64_t> tab_off;
-    const BatchSizes z = tile_batch(b->dims.data(), n, b->zs, b->hv, tab_off);
-    for (int v = 0; v < n; v++) b->hv[v].vol = b->vols[v];
-    const int64_t items = z.items, pieces = z.pieces, nflags = z.nflags, tdoubles = z.tdoubles, stiles = z.stiles;
-    const int64_t max_ntab = z.max_ntab;
-    // the compaction splits each item into up to WY row tiles counted in 32 bits
-    if (items >= ((int64_t)1 << 31) / WY || stiles >= ((int64_t)1 << 31))
+    const BatchSizes z = tile_batch(b->vols.data(), dtype_size(b->T), b->dims.data(), n, b->zs, b->hv, tab_off);
+    if (z.bblks > 0x7fff0000 || z.cblks > 0x3fffffff || z.tiles() > 0x7fffffff)
         return fail(c, MESH_ETOOLARGE, "batch has too many work items");
 
     cudaError_t e;
     const size_t bvb = sizeof(BatchVol) * (size_t)std::max(n, 1);
-    if ((e = b->dvols.ensure(bvb)) != cudaSuccess || (e = b->ivol.ensure(4 * (size_t)items + 4)) != cudaSuccess ||
-        (e = b->svol.ensure(4 * (size_t)stiles + 4)) != cudaSuccess ||
-        (e = b->tabs.ensure(8 * (size_t)tdoubles + 8)) != cudaSuccess ||
+    if ((e = b->dvols.ensure(bvb)) != cudaSuccess || (e = b->bvol.ensure(4 * (size_t)z.bblks + 4)) != cudaSuccess ||
+        (e = b->cvol.ensure(4 * (size_t)z.cblks + 4)) != cudaSuccess ||
+        (e = b->tabs.ensure(8 * (size_t)z.tdoubles + 8)) != cudaSuccess ||
         (e = b->jobs.ensure(sizeof(TabJob) * (size_t)std::max(n, 1))) != cudaSuccess ||
-        (e = b->cnt.ensure((size_t)pieces * NCNT * 4 + 4)) != cudaSuccess ||
-        (e = b->base.ensure((size_t)pieces * NCNT * 8 + 8)) != cudaSuccess ||
-        (e = b->flags.ensure((size_t)nflags + 1)) != cudaSuccess ||
-        (e = b->scan.ensure((size_t)std::max<int64_t>(stiles, n) * NCNT * 8 + 64)) != cudaSuccess ||
-        (e = b->misc.ensure(MISC_SLOTS * sizeof(int64_t))) != cudaSuccess ||
+        (e = b->bits.ensure((size_t)z.words * 4 + 16)) != cudaSuccess ||
+        (e = b->pc.ensure((size_t)z.pieces * sizeof(uint2) + 16)) != cudaSuccess ||
+        (e = b->tsum.ensure((size_t)z.tiles() * sizeof(ulonglong2) + 16)) != cudaSuccess ||
+        (e = b->wmask.ensure((size_t)z.masks * 4 + 4)) != cudaSuccess ||
+        (e = b->misc.ensure(MISC_WORDS * sizeof(int64_t))) != cudaSuccess ||
         (e = b->offs.ensure((size_t)(n + 1) * 2 * 8)) != cudaSuccess)
         return cuda_fail(c, e, "batch buffers");
 
-    // per-volume tables, item and scan-tile owners
+    // per-volume tables and the CTAs' volumes
     std::vector<TabJob> jobs;
-    std::vector<uint32_t> ivol, svol;
-    batch_owners(b->hv, z, ivol, svol);
+    std::vector<uint32_t> bvol, cvol;
+    batch_owners(b->hv, z, bvol, cvol);
     for (int v = 0; v < n; v++) {
         BatchVol &bv = b->hv[v];
         bv.tabs = (const double *)b->tabs.ptr + tab_off[v];
@@ -168,35 +199,19 @@ int build_plan(mesh_batch *b) {
     }
     // plan building is off the hot path: plain synchronous uploads
     if ((e = cudaMemcpy(b->dvols.ptr, b->hv.data(), sizeof(BatchVol) * n, cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (items && (e = cudaMemcpy(b->ivol.ptr, ivol.data(), 4 * (size_t)items, cudaMemcpyHostToDevice)) != cudaSuccess) ||
-        (stiles && (e = cudaMemcpy(b->svol.ptr, svol.data(), 4 * (size_t)stiles, cudaMemcpyHostToDevice)) != cudaSuccess) ||
+        (z.bblks && (e = cudaMemcpy(b->bvol.ptr, bvol.data(), 4 * bvol.size(), cudaMemcpyHostToDevice)) != cudaSuccess) ||
+        (z.cblks && (e = cudaMemcpy(b->cvol.ptr, cvol.data(), 4 * cvol.size(), cudaMemcpyHostToDevice)) != cudaSuccess) ||
         (!jobs.empty() &&
          (e = cudaMemcpy(b->jobs.ptr, jobs.data(), sizeof(TabJob) * jobs.size(), cudaMemcpyHostToDevice)) != cudaSuccess))
         return cuda_fail(c, e, "batch plan upload");
-    if (!jobs.empty() && (e = launch_tables_batch((const TabJob *)b->jobs.ptr, (int)jobs.size(), max_ntab, L32,
-                                                  c->stream)) != cudaSuccess)
+    if (!jobs.empty() && (e = launch_tables_batch((const TabJob *)b->jobs.ptr, (int)jobs.size(), z.max_ntab,
+                                                  L32, c->stream)) != cudaSuccess)
         return cuda_fail(c, e, "batch tables");
 
     P.force_fp64 = c->force_fp64;
-    P.pstride = pieces;
-    P.cnt = (uint32_t *)b->cnt.ptr;
-    P.base = (int64_t *)b->base.ptr;
-    P.flags = (uint8_t *)b->flags.ptr;
-    P.scan_state = (unsigned long long *)b->scan.ptr;
-    P.scan_ticket = (unsigned int *)((char *)b->scan.ptr + (size_t)std::max<int64_t>(stiles, n) * NCNT * 8);
-    b->scan_vol = true;
-    for (const BatchVol &bv : b->hv) b->scan_vol = b->scan_vol && bv.cx <= 4 * 32;
-    P.totals = (int64_t *)b->misc.ptr;
-    P.err = (unsigned int *)((int64_t *)b->misc.ptr + NCNT);
-    P.work = (unsigned int *)((int64_t *)b->misc.ptr + NCNT + 1);
-    P.scan_spin_limit = 1 << 24;
-    P.bvols = (const BatchVol *)b->dvols.ptr;
-    P.item_vol = (const uint32_t *)b->ivol.ptr;
-    P.stile_vol = (const uint32_t *)b->svol.ptr;
-    P.vol_off = (int64_t *)b->offs.ptr;
-    P.nitems = items;
-    P.nvols = n;
-    P.nstiles = (int32_t)stiles;
+    bind_batch(P, z, n,
+               BatchBufs{b->dvols.ptr, b->bvol.ptr, b->cvol.ptr, b->bits.ptr, b->pc.ptr, b->tsum.ptr, b->wmask.ptr,
+                         b->misc.ptr, b->offs.ptr});
     return MESH_OK;
 }
 
@@ -207,31 +222,17 @@ int fetch(mesh_batch *b) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "batch synchronize");
     const unsigned err = (unsigned)(b->h_misc[NCNT] & 0xffffffffll);
-    if (err & ERR_SCAN_TIMEOUT) return fail(c, MESH_EDEVICE, "scan look-back wait expired");
     if (err & ERR_BOUNDS) return fail(c, MESH_EDEVICE, "device bounds check failed");
     if (err & ERR_CAPACITY) return fail(c, MESH_ECAPACITY, "batch outputs larger than at the last count");
     return MESH_OK;
 }
 
-// classify + scan (with the per-volume offsets), on stream s
-int enqueue_count(mesh_batch *b, cudaStream_t s) {
-    mesh_ctx *c = b->ctx;
-    cudaError_t e;
-    if ((e = cudaMemsetAsync(b->misc.ptr, 0, MISC_SLOTS * sizeof(int64_t), s)) != cudaSuccess)
-        return cuda_fail(c, e, "memset");
-    if ((e = launch_classify_batch(b->P, b->cls_ctas, s)) != cudaSuccess) return cuda_fail(c, e, "batch classify");
-    if ((e = launch_scan_batch(b->P, b->scan_threads, s, b->scan_vol)) != cudaSuccess)
-        return cuda_fail(c, e, "batch scan");
-    return MESH_OK;
-}
-
 int enqueue_run(mesh_batch *b, cudaStream_t s) {
-    int rc = enqueue_count(b, s);
-    if (rc) return rc;
     mesh_ctx *c = b->ctx;
     cudaError_t e;
-    if ((e = launch_compact_batch(b->P, b->cmp_ctas, s)) != cudaSuccess) return cuda_fail(c, e, "batch compact");
-    if ((e = launch_expand_batch(b->P, b->Q64, b->P64, s)) != cudaSuccess) return cuda_fail(c, e, "batch expand");
+    if ((e = launch_batch_counts(b->P, s)) != cudaSuccess) return cuda_fail(c, e, "batch counts");
+    if ((e = launch_emit_batch(b->P, b->Q64, b->P64, b->cmp_ctas, s)) != cudaSuccess)
+        return cuda_fail(c, e, "batch emission");
     if (b->weld) {
         const Plan &P = b->P;
         const int64_t nb = weld_blocks(b->nv_cell), hcap = weld_hash_slots(b->nv_cell);
@@ -249,32 +250,18 @@ int enqueue_run(mesh_batch *b, cudaStream_t s) {
 int count(mesh_batch *b) {
     mesh_ctx *c = b->ctx;
     drop_graph(b);
-    int rc = enqueue_count(b, c->stream);
-    if (rc || (rc = fetch(b))) return rc;
+    int rc;
+    cudaError_t e = launch_batch_counts(b->P, c->stream);
+    if (e != cudaSuccess) return cuda_fail(c, e, "batch counts");
+    if ((rc = fetch(b))) return rc;
     b->nverts = b->h_misc[0];
     b->nfaces = b->h_misc[1];
-    b->nactive = b->h_misc[2];
     Plan &P = b->P;
-    // active-cell list (emission order over the batch) and the outputs, sized exactly
-    const size_t es = dtype_size(b->T);
-    const int64_t cap = b->nactive;
+    // the outputs, sized exactly
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-    const size_t o_val = up((size_t)cap * 8);
-    const size_t o_side = o_val + up((size_t)cap * 8 * es);
-    const size_t o_vol = o_side + up((size_t)(cap / ENT_BLOCK + 1) * 16);
-    const size_t o_cs = o_vol + up((size_t)cap * 4);
     const size_t vb = (size_t)b->nverts * 3 * (P.out64 ? 8 : 4), fb = (size_t)b->nfaces * 3 * 8;
-    cudaError_t e;
-    if ((e = b->ent.ensure(o_cs + up((size_t)cap + 1))) != cudaSuccess || (e = b->out_v.ensure(vb + 16)) != cudaSuccess ||
-        (e = b->out_f.ensure(fb + 16)) != cudaSuccess)
+    if ((e = b->out_v.ensure(vb + 16)) != cudaSuccess || (e = b->out_f.ensure(fb + 16)) != cudaSuccess)
         return cuda_fail(c, e, "batch outputs");
-    char *eb = (char *)b->ent.ptr;
-    P.ent_pos = (unsigned long long *)eb;
-    P.ent_val = eb + o_val;
-    P.ent_side = (long long *)(eb + o_side);
-    P.ent_vol = (uint32_t *)(eb + o_vol);
-    P.ent_cs = (uint8_t *)(eb + o_cs);
-    P.ent_cap = cap;
     P.verts = b->out_v.ptr;
     P.faces = (int64_t *)b->out_f.ptr;
     P.verts_cap = b->nverts;
@@ -408,8 +395,8 @@ void mesh_batch_destroy(mesh_batch *b) {
     cudaSetDevice(b->ctx->device);
     cudaStreamSynchronize(b->ctx->stream);
     drop_graph(b);
-    DevBuf *bufs[] = {&b->dvols, &b->ivol, &b->svol,  &b->tabs, &b->jobs, &b->cnt,  &b->base, &b->flags, &b->scan,
-                      &b->misc,  &b->ent,  &b->out_v, &b->out_f, &b->offs, &b->wkey, &b->wbuf, &b->wv,   &b->woffs};
+    DevBuf *bufs[] = {&b->dvols, &b->bvol,  &b->cvol,  &b->tabs, &b->jobs, &b->bits, &b->pc, &b->tsum, &b->wmask,
+                      &b->misc,  &b->out_v, &b->out_f, &b->offs, &b->wkey, &b->wbuf, &b->wv, &b->woffs};
     for (DevBuf *x : bufs) x->release();
     if (b->h_misc) cudaFreeHost(b->h_misc);
     if (b->cap) cudaStreamDestroy(b->cap);
@@ -486,7 +473,7 @@ int mesh_batch_tune(mesh_batch *b, int reps, char *report, int report_len) {
     if (cudaSetDevice(c->device) != cudaSuccess) return fail(c, MESH_ECUDA, "cudaSetDevice");
     std::string rep;
     int cur[4] = {b->zs, b->cls_ctas, b->cmp_ctas, b->scan_threads};
-    const std::vector<int> cand[4] = {{0, 64, 32, 16}, {0, 2, 1}, {0, 2, 1}, {1024, 512, 256}};
+    const std::vector<int> cand[4] = {{0, 64, 32}, {}, {0, 2, 1}, {}};
     const char *names[4] = {"zs", "classify_ctas", "compact_ctas", "scan_threads"};
     double best_ms = -1;
     int rc;

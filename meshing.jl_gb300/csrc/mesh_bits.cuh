@@ -50,6 +50,11 @@ __device__ __forceinline__ BView view_of(const Plan &p) {
                  p.bseg, p.zws, p.nzw, p.bw0, 0, 0};
 }
 
+__device__ __forceinline__ BView view_of(const Plan &p, const BatchVol &b) {
+    return BView{b.vol, p.bits + b.bits0, b.nx, b.ny, b.nz, b.nx * b.ny, b.cx, b.cy, b.cz, b.nxb, b.nyb,
+                 b.bseg, b.zws, b.nzw, 0, b.e0, b.m0};
+}
+
 // The four corner columns of column (x, y) in one word of z, and the same one
 // sample up (bit k: sample z + 1).
 struct Corners {

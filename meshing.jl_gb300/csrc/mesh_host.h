@@ -1,7 +1,6 @@
 // Host-side state shared by the single-volume runtime (mesh_api.cu) and the
 // batched runtime (mesh_batch.cu).  Not part of the public ABI.
 #pragma once
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -105,11 +104,6 @@ struct mesh_ctx {
     // stage timing (diagnostics)
     int timing = 0;
     int force_fp64 = 0;  // MESHING_GB300_FORCE_FP64=1: evaluate every Float64 position in FP64
-    // Classification from TMA-staged bricks: by default for Marching Cubes volumes a
-    // tensor map can describe (Float32 / UInt16 / Float64, 16-byte row strides) and
-    // not uploaded in pipelined groups; MESHING_GB300_TMA=0 (-1 unset) keeps the
-    // global-load walk, MESHING_GB300_TMA=1 also streams MT / NSN volumes.
-    int tma_env = -1;
     // MESHING_GB300_ONE_WALK=1: Marching Cubes in one walk that also lists the
     // active cells (k_walk_mc.cu).  Off by default: on GB300 the walk is issue
     // bound, so dropping the second read of the volume saves little, and
@@ -127,8 +121,6 @@ struct mesh_ctx {
     // one-walk expansion costs more (end to end 42.1 vs 33.6 ms at 1024^3).
     int zerocopy = 0;
     int host_mapped = 0; // the current plan reads a mapped host volume
-    int use_tma = 0;     // the current plan streams the volume through TMA
-    CUtensorMap tmap;
     std::vector<cudaEvent_t> ev_free;
     std::vector<cudaEvent_t> ev_pairs[mesh::NSTAGE];  // start, stop, start, stop, ...
     int64_t nkern[mesh::NSTAGE] = {};                 // kernels launched per stage (with timing on)
@@ -145,16 +137,27 @@ int validate(mesh_ctx *c, int T, int64_t nx, int64_t ny, int64_t nz, const mesh_
 // Float64, P64: positions in Float64), output eltype and the exact thresholds.
 void set_types(Plan &P, int T, const mesh_params *p, int *Q64, int *A64, int *P64);
 
-// Tiling of a batch of volumes of sizes dims[3i..3i+2] with `zs` z cells per
-// work item (0 = whole columns): the descriptors (without device pointers),
-// each volume's table block offset in doubles, and the totals.
+// Tiling of a batch of volumes at vols[i] (es bytes per sample), of sizes
+// dims[3i..3i+2], with `zs` z cells per segment (0 = whole columns; rounded up to
+// words of 32): the descriptors (without the other device pointers), each volume's
+// table block offset in doubles, and the totals.
 struct BatchSizes {
-    int64_t items = 0, pieces = 0, nflags = 0, tdoubles = 0, stiles = 0, max_ntab = 1;
+    int64_t words = 0, pieces = 0, masks = 0, bblks = 0, cblks = 0, tdoubles = 0, max_ntab = 1;
     int64_t keys = 0;  // lattice-edge keys of all volumes (3 per node)
+    int64_t tiles() const { return (pieces + BITS_TILE - 1) / BITS_TILE; }
 };
-BatchSizes tile_batch(const int64_t *dims, int n, int zs, std::vector<BatchVol> &hv, std::vector<int64_t> &tab_off);
-// The volume of every work item and scan tile.
-void batch_owners(const std::vector<BatchVol> &hv, const BatchSizes &z, std::vector<uint32_t> &ivol,
-                  std::vector<uint32_t> &svol);
+BatchSizes tile_batch(const void *const *vols, size_t es, const int64_t *dims, int n, int zs, std::vector<BatchVol> &hv,
+                      std::vector<int64_t> &tab_off);
+// The volume of every CTA of the bit and count kernels.
+void batch_owners(const std::vector<BatchVol> &hv, const BatchSizes &z, std::vector<uint32_t> &bvol,
+                  std::vector<uint32_t> &cvol);
+// Device buffers of a batch.
+struct BatchBufs {
+    void *vols, *bvol, *cvol, *bits, *pc, *tsum, *wmask, *misc, *offs;
+};
+// The plan's sign-bit fields over those buffers (misc: MISC_WORDS words).
+void bind_batch(Plan &P, const BatchSizes &z, int n, const BatchBufs &b);
+// Sign words, piece counts and offsets, and every volume's first vertex / face.
+cudaError_t launch_batch_counts(const Plan &P, cudaStream_t s);
 
 }  // namespace mesh

@@ -25,10 +25,9 @@ constexpr int ENT_BLOCK = 256;   // active-cell entries per expansion block
 constexpr int POS_BITS = 21;     // bits per coordinate in a packed cell position
 
 // Error bits of the device error word.
-constexpr unsigned ERR_SCAN_TIMEOUT = 1u;
 constexpr unsigned ERR_CAPACITY = 2u;
 constexpr unsigned ERR_BOUNDS = 4u;
-constexpr unsigned ERR_STAGE = 16u;  // the staged entry list was too short (8 is the TMA wait)
+constexpr unsigned ERR_STAGE = 16u;  // the staged entry list was too short
 
 struct BatchVol;
 
@@ -102,15 +101,11 @@ struct Plan {
     int64_t verts_cap, faces_cap;
     int32_t scan_spin_limit;
     // batches (Marching Cubes over many volumes in one pass): per-volume
-    // descriptors, the volume of each work item and of each scan tile, the
-    // volume of each active-cell entry, and the first vertex / face of every
-    // volume ([nvols + 1][2], the last row the totals)
+    // descriptors, and the first vertex / face of every volume ([nvols + 1][2],
+    // the last row the totals)
     const BatchVol *bvols;
-    const uint32_t *item_vol, *stile_vol;
-    uint32_t *ent_vol;
     int64_t *vol_off;
-    int64_t nitems;
-    int32_t nvols, nstiles;
+    int32_t nvols;
     int32_t vol_outputs;  // 1: every volume writes to its own BatchVol::verts / faces
     // x window (mesh_set_x_window): global x of the volume's sample 0, for the
     // grid-boundary rules of MT / NSN; with xhalo, the volume's first cell column
@@ -119,11 +114,8 @@ struct Plan {
     // shifted down by that column's totals (base of piece (seg 0, y 0, x 1))
     int64_t xg0;
     int32_t xhalo;
-    // sub-range launches of the pipelined host path (zero: the whole volume):
-    // classify z segments seg0 .. seg1 - 1; compact the x tiles tx0 .. tx0 + ntx - 1;
-    // expand list entries e_lo .. e_hi - 1
-    int32_t seg0, seg1, tx0, ntx;
-    int64_t e_lo, e_hi;
+    // emission of a range of column blocks (the pipelined host path; ntx 0: all)
+    int32_t tx0, ntx;
     // sign bits (mesh_bits.cuh): words bw0 .. bw1 - 1 of z at `bits`, z segments of
     // zws words (bseg of them) and column / row blocks; per piece, the vertex and
     // face counts that the offset scan turns into offsets within their scan tile
@@ -143,25 +135,22 @@ struct Plan {
     int64_t nbblk, ncblk;
 };
 
-// One volume of a batch.  Its work items, pieces, activity bytes and scan
-// tiles are ranges of the batch's arrays starting at item0, piece0, flag0 and
-// stile0; its coordinate tables are a block at `tabs` (k_tables.cu layout).
+// One volume of a batch.  Its sign words, pieces, activity masks and CTAs of the
+// bit and count kernels are ranges of the batch's arrays starting at bits0, e0, m0,
+// bblk0 and cblk0 (tiling as in Plan; vec: its planes take 16-byte loads); its
+// coordinate tables are a block at `tabs` (k_tables.cu layout).
 // With Plan::vol_outputs its mesh goes to its own verts / faces (room for
 // vcap / fcap) instead of the batch's concatenated outputs.
 struct BatchVol {
     const void *vol;
     const double *tabs;
     int64_t nx, ny, nz;
-    int32_t cx, cy, cz, tiles_x, tiles_y, nseg, zs, chunks_per_seg, nchunks, stile0;
-    int64_t item0, piece0, flag0;
+    int32_t cx, cy, cz, nxb, nyb, bseg, zws, nzw, vec;
+    int64_t bits0, e0, m0, bblk0, cblk0;
     void *verts;
     int64_t *faces;
     int64_t vcap, fcap;
     int64_t kbase;  // welded batches: the volume's lattice-edge keys start here
-    // sign bits: tiling, first word, piece, mask word and CTAs, and whether its
-    // planes start on 16-byte boundaries
-    int32_t nxb, nyb, bseg, zws, nzw, vec;
-    int64_t bits0, e0, m0, bblk0, cblk0;
 };
 
 // Bytes per sample of a volume dtype.
@@ -196,20 +185,6 @@ inline __host__ __device__ void set_tabs(Plan &P, const Tabs &t) {
     P.xpf = t.xpf; P.ypf = t.ypf; P.zpf = t.zpf; P.dxf = t.dxf; P.dyf = t.dyf; P.dzf = t.dzf;
     P.split = t.split;
     P.ntab = t.ntab;
-}
-// The batch plan p seen as a plan of its volume b alone (shared arrays offset).
-inline __host__ __device__ Plan vol_view(const Plan &p, const BatchVol &b) {
-    Plan v = p;
-    v.vol = b.vol;
-    v.nx = b.nx; v.ny = b.ny; v.nz = b.nz;
-    v.cx = b.cx; v.cy = b.cy; v.cz = b.cz;
-    v.tiles_x = b.tiles_x; v.tiles_y = b.tiles_y;
-    v.nseg = b.nseg; v.zs = b.zs; v.chunks_per_seg = b.chunks_per_seg; v.nchunks = b.nchunks;
-    v.cnt = p.cnt + b.piece0;
-    v.base = p.base + b.piece0;
-    v.flags = p.flags + b.flag0;
-    set_tabs(v, tabs_at(b.tabs, b.nx, b.ny, b.nz));
-    return v;
 }
 inline __host__ __device__ int64_t piece(const Plan &p, int seg, int y, int x) {
     return ((int64_t)seg * p.cy + y) * p.cx + x;
@@ -252,23 +227,20 @@ struct TabJob {
     double range[6];
 };
 cudaError_t launch_tables_batch(const TabJob *jobs, int njobs, int64_t max_ntab, int L32, cudaStream_t s);
-// Batched Marching Cubes stages (k_classify.cu, k_scan.cu, k_emit_mc.cu);
-// ctas: CTAs per SM of the persistent kernels (0 = as many as fit), threads:
-// threads per scan CTA.
-cudaError_t launch_classify_batch(const Plan &p, int ctas, cudaStream_t s);
-// per_volume: every volume is at most a few 32-column groups wide -- chain the
-// volumes, one CTA each (scan state for NCNT x nvols entries)
-cudaError_t launch_scan_batch(const Plan &p, int threads, cudaStream_t s, bool per_volume = false);
-cudaError_t launch_compact_batch(const Plan &p, int ctas, cudaStream_t s);
-cudaError_t launch_expand_batch(const Plan &p, int Q64, int P64, cudaStream_t s);
-cudaError_t launch_classify(const Plan &p, cudaStream_t s, int seg0 = 0, int nsegs = 0);  // nsegs 0: all
-// A few values of a device int64 array for the host: dst[i] = src[idx[i]], i < n.
+// Batched Marching Cubes stages (k_bits.cu, k_emit_bits.cu); ctas: CTAs per SM of
+// the persistent emission (0 = as many as fit).  launch_batch_rows leaves the first
+// vertex and face of every volume in Plan::vol_off.
+cudaError_t launch_bits_batch(const Plan &p, cudaStream_t s);
+cudaError_t launch_count_batch(const Plan &p, cudaStream_t s);
+cudaError_t launch_batch_rows(const Plan &p, cudaStream_t s);
+cudaError_t launch_emit_batch(const Plan &p, int Q64, int P64, int ctas, cudaStream_t s);
+cudaError_t launch_classify(const Plan &p, cudaStream_t s);
+// Indices of a few pieces whose offsets the host wants.
 constexpr int GATHER_MAX = 32;
 struct GatherIdx {
     int64_t idx[GATHER_MAX];
     int n;
 };
-cudaError_t launch_gather(const int64_t *src, const GatherIdx &g, int64_t *dst, cudaStream_t s);
 // First vertex and face of pieces e[0..n) (after the offset scan): dst[2 i], dst[2 i + 1].
 cudaError_t launch_gather_pieces(const Plan &p, const GatherIdx &g, int64_t *dst, cudaStream_t s);
 cudaError_t launch_scan(const Plan &p, cudaStream_t s);

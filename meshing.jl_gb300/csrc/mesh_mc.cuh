@@ -274,17 +274,12 @@ template <> __device__ __forceinline__ void load8<uint16_t>(const uint16_t *src,
 // carries its vertex / face rank inside its piece (ent_rank), and the scanned
 // piece offsets give the global ones.  Entries: *stage_next slots, of which
 // unused ones have case 0 and emit nothing.
-// EXP_BATCH: as EXP_ORDERED over the volumes of a batch in order
-// (k_compact_batch); each entry also names its volume (ent_vol), whose
-// coordinate tables place its vertices and whose first vertex makes its faces
-// 1-based within the volume.
 
-constexpr int EXP_ORDERED = 0, EXP_STAGED = 1, EXP_BATCH = 2;
+constexpr int EXP_ORDERED = 0, EXP_STAGED = 1;
 
 template <class T> struct ExpandSmem {
     T val[8][XW];
     unsigned long long pos[XW];
-    uint32_t vol[XW];  // EXP_BATCH: the entry's volume
     long long vb[XW], fb[XW];  // global offsets of each entry's first vertex / face
     int32_t vs[XW], fs[XW];    // block-local offsets
     uint8_t cs[XW];
@@ -292,12 +287,6 @@ template <class T> struct ExpandSmem {
     uint8_t fmap[XW * MC_MAX_FACES];
     int32_t wsum[2][XW / 32];
 };
-
-// Coordinate tables of batch volume v.
-__device__ __forceinline__ Tabs batch_tabs(const Plan &p, uint32_t v) {
-    const BatchVol &b = p.bvols[v];
-    return tabs_at(b.tabs, b.nx, b.ny, b.nz);
-}
 
 template <class T, class Q, class P, int MODE>
 __global__ void __launch_bounds__(XW) k_expand_mc(const Plan p) {
@@ -309,23 +298,15 @@ __global__ void __launch_bounds__(XW) k_expand_mc(const Plan p) {
         s_f[i] = MC_CASE_FACES[i];
     }
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    int64_t na = STAGED ? (int64_t)min(*p.stage_next, (unsigned long long)p.ent_cap) : min(p.totals[2], p.ent_cap);
-    // ordered sub-range e_lo .. e_hi - 1: the blocks that hold it, with the
-    // entries of those blocks before e_lo counted (offsets) but not emitted
-    int64_t e_lo = 0;
-    if (MODE == EXP_ORDERED) {
-        if (p.e_hi > 0) na = min(na, p.e_hi);
-        e_lo = p.e_lo;
-    }
+    const int64_t na = STAGED ? (int64_t)min(*p.stage_next, (unsigned long long)p.ent_cap) : min(p.totals[2], p.ent_cap);
     const int64_t nblocks = (na + XW - 1) / XW;
     const int64_t np = p.pstride;
     const uint64_t pmask = (1ull << POS_BITS) - 1;
     const Tabs tb = tabs_of(p);
     __syncthreads();
 
-    for (int64_t blk = e_lo / XW + blockIdx.x; blk < nblocks; blk += gridDim.x) {
+    for (int64_t blk = blockIdx.x; blk < nblocks; blk += gridDim.x) {
         const int64_t e = blk * XW + tid;
-        const int skip = (int)max((int64_t)0, e_lo - blk * XW);  // entries of this block before e_lo
         int nv = 0, nf = 0;
         if (e < na) {
             const int cs = p.ent_cs[e];
@@ -340,7 +321,6 @@ __global__ void __launch_bounds__(XW) k_expand_mc(const Plan p) {
                 load8<T>((const T *)p.ent_val + 8 * e, cv);
 #pragma unroll
                 for (int k = 0; k < 8; k++) sm.val[k][tid] = cv[k];
-                if (MODE == EXP_BATCH) sm.vol[tid] = p.ent_vol[e];
                 if (STAGED) {
                     const uint2 rk = p.ent_rank[e];
                     const int z = (int)(pos >> (2 * POS_BITS));
@@ -398,64 +378,34 @@ __global__ void __launch_bounds__(XW) k_expand_mc(const Plan p) {
             sm.fb[tid] = fb0 + fs;
         }
         __syncthreads();
-        // the entries before e_lo come first in the block's numbering: start after them
-        const int v0 = skip ? sm.vs[skip] : 0, f0 = skip ? sm.fs[skip] : 0;
-        for (int t = v0 + tid; t < V; t += XW) {
+        for (int t = tid; t < V; t += XW) {
             const int j = sm.vmap[t];
             const int k = t - sm.vs[j];
             const uint64_t pos = sm.pos[j];
             const int ed = (int)((s_v[sm.cs[j]] >> (4 * k)) & 15u);
             const int g = edge_info(ed);
-            void *vout = p.verts;
-            int64_t out = sm.vb[j] + k;
-            if (MODE == EXP_BATCH && p.vol_outputs) {  // the volume's own outputs
-                const BatchVol &b = p.bvols[sm.vol[j]];
-                out -= p.vol_off[2 * sm.vol[j]];
-                vout = b.verts;
-                if (out < 0 || out >= b.vcap) {
-                    atomicOr(p.err, ERR_CAPACITY);
-                    continue;
-                }
-            }
-            vertex_task<T, Q, P>(p, MODE == EXP_BATCH ? batch_tabs(p, sm.vol[j]) : tb, ed, (int)(pos & pmask),
+            const int64_t out = sm.vb[j] + k;
+            vertex_task<T, Q, P>(p, tb, ed, (int)(pos & pmask),
                                  (int)((pos >> POS_BITS) & pmask), (int)(pos >> (2 * POS_BITS)), sm.val[g & 7][j],
-                                 sm.val[(g >> 3) & 7][j], vout, out);
-            if ((MODE == EXP_ORDERED || (MODE == EXP_BATCH && !p.vol_outputs)) && p.vkey) {
+                                 sm.val[(g >> 3) & 7][j], p.verts, out);
+            if (MODE == EXP_ORDERED && p.vkey) {
                 // the edge's lower node; the cell owns the edge when, across each
                 // other axis, the edge lies on the cell's upper side or the cell is first
-                // (in a batch, each volume's keys start at its own base)
                 const int x = (int)(pos & pmask), y = (int)((pos >> POS_BITS) & pmask), z = (int)(pos >> (2 * POS_BITS));
                 const int a = g & 7, ax = (g >> 6) & 3;
                 const int ox = ax == 0 ? 0 : cdx(a), oy = ax == 1 ? 0 : cdy(a), oz = ax == 2 ? 0 : cdz(a);
                 const bool own = (ax == 0 || ox || x == 0) && (ax == 1 || oy || y == 0) && (ax == 2 || oz || z == 0);
-                int64_t kx = p.nx, ky = p.ny, kb = 0;
-                if (MODE == EXP_BATCH) {
-                    const BatchVol &b = p.bvols[sm.vol[j]];
-                    kx = b.nx;
-                    ky = b.ny;
-                    kb = b.kbase;
-                }
                 const long long key =
-                    kb + ax + 3 * ((long long)(x + ox) + kx * ((long long)(y + oy) + ky * (long long)(z + oz)));
+                    ax + 3 * ((long long)(x + ox) + p.nx * ((long long)(y + oy) + p.ny * (long long)(z + oz)));
                 p.vkey[out] = key | (own ? (long long)(1ull << 63) : 0ll);
             }
         }
-        for (int t = f0 + tid; t < F; t += XW) {
+        for (int t = tid; t < F; t += XW) {
             const int j = sm.fmap[t];
             const int k = t - sm.fs[j];
             const unsigned s = (unsigned)(s_f[sm.cs[j]] >> (12 * k));
-            // 1-based within the volume
-            const int64_t vb = sm.vb[j] + 1 - (MODE == EXP_BATCH ? p.vol_off[2 * sm.vol[j]] : 0);
+            const int64_t vb = sm.vb[j] + 1;  // 1-based
             int64_t *o = p.faces + 3 * (sm.fb[j] + k);
-            if (MODE == EXP_BATCH && p.vol_outputs) {
-                const BatchVol &b = p.bvols[sm.vol[j]];
-                const int64_t lf = sm.fb[j] + k - p.vol_off[2 * sm.vol[j] + 1];
-                if (lf < 0 || lf >= b.fcap) {
-                    atomicOr(p.err, ERR_CAPACITY);
-                    continue;
-                }
-                o = b.faces + 3 * lf;
-            }
             o[0] = vb + (s & 15u);
             o[1] = vb + ((s >> 4) & 15u);
             o[2] = vb + ((s >> 8) & 15u);

@@ -207,47 +207,33 @@ struct GroupLayout {
     BatchSizes z;
     std::vector<BatchVol> hv;
     std::vector<int64_t> tab_off;
-    size_t o_ivol = 0, o_svol = 0, o_jobs = 0, head = 0;  // head: copied from pinned staging
-    size_t o_tabs = 0, o_cnt = 0, o_base = 0, o_flags = 0, o_scan = 0, o_misc = 0, o_offs = 0;
-    size_t o_pos = 0, o_val = 0, o_side = 0, o_vol = 0, o_cs = 0, total = 0;
-    int64_t cells = 0;
-    bool scan_vol = false;  // the per-volume scan (every volume at most 128 columns wide)
+    size_t o_bvol = 0, o_cvol = 0, o_jobs = 0, head = 0;  // head: copied from pinned staging
+    size_t o_tabs = 0, o_bits = 0, o_pc = 0, o_tsum = 0, o_mask = 0, o_misc = 0, o_offs = 0, total = 0;
 };
 
 
 void layout_group(const std::vector<const Req *> &rs, GroupLayout *L) {
     const int n = (int)rs.size();
     std::vector<int64_t> dims(3 * (size_t)n);
-    L->cells = 0;
+    std::vector<const void *> vols((size_t)n);
     for (int i = 0; i < n; i++) {
+        vols[i] = rs[i]->vol;
         for (int k = 0; k < 3; k++) dims[3 * i + k] = rs[i]->dims[k];
-        if (dims[3 * i] > 1 && dims[3 * i + 1] > 1 && dims[3 * i + 2] > 1)
-            L->cells += (dims[3 * i] - 1) * (dims[3 * i + 1] - 1) * (dims[3 * i + 2] - 1);
     }
-    L->z = tile_batch(dims.data(), n, 0, L->hv, L->tab_off);
-    // every volume at most 4 column groups wide: one scan CTA per volume, chained
-    L->scan_vol = n > 0;
-    for (const BatchVol &bv : L->hv) L->scan_vol = L->scan_vol && bv.cx <= 4 * 32;
+    L->z = tile_batch(vols.data(), n ? dtype_size(rs[0]->T) : 4, dims.data(), n, 0, L->hv, L->tab_off);
     const BatchSizes &z = L->z;
-    const size_t es = n ? dtype_size(rs[0]->T) : 4;
     size_t o = up(sizeof(BatchVol) * (size_t)std::max(n, 1));
-    L->o_ivol = o; o += up(4 * (size_t)z.items + 4);
-    L->o_svol = o; o += up(4 * (size_t)z.stiles + 4);
+    L->o_bvol = o; o += up(4 * (size_t)z.bblks + 4);
+    L->o_cvol = o; o += up(4 * (size_t)z.cblks + 4);
     L->o_jobs = o; o += up(sizeof(TabJob) * (size_t)std::max(n, 1));
     L->head = o;
     L->o_tabs = o; o += up(8 * (size_t)z.tdoubles + 8);
-    L->o_cnt = o; o += up((size_t)z.pieces * NCNT * 4 + 4);
-    L->o_base = o; o += up((size_t)z.pieces * NCNT * 8 + 8);
-    L->o_flags = o; o += up((size_t)z.nflags + 1);
-    L->o_scan = o; o += up((size_t)std::max<int64_t>(z.stiles, n) * NCNT * 8 + 64);
-    L->o_misc = o; o += up(MISC_SLOTS * 8);
+    L->o_bits = o; o += up(4 * (size_t)z.words + 16);
+    L->o_pc = o; o += up((size_t)z.pieces * sizeof(uint2) + 16);
+    L->o_tsum = o; o += up((size_t)z.tiles() * sizeof(ulonglong2) + 16);
+    L->o_mask = o; o += up(4 * (size_t)z.masks + 4);
+    L->o_misc = o; o += up(MISC_WORDS * 8);
     L->o_offs = o; o += up((size_t)(n + 1) * 16);
-    const size_t cap = (size_t)L->cells;  // worst case: every cell active
-    L->o_pos = o; o += up(cap * 8 + 8);
-    L->o_val = o; o += up(cap * 8 * es + 16);
-    L->o_side = o; o += up((cap / ENT_BLOCK + 1) * 16);
-    L->o_vol = o; o += up(cap * 4 + 4);
-    L->o_cs = o; o += up(cap + 1);
     L->total = o;
 }
 
@@ -255,14 +241,14 @@ void layout_group(const std::vector<const Req *> &rs, GroupLayout *L) {
 // layout_group grows by at most this much when r joins (before rounding).
 size_t vol_scratch_bytes(const Req &r) {
     const int64_t nx = r.dims[0], ny = r.dims[1], nz = r.dims[2];
-    size_t b = sizeof(BatchVol) + sizeof(TabJob) + 16 + 4 + 4 + 8 + NCNT * 8;
+    size_t b = sizeof(BatchVol) + sizeof(TabJob) + 16;
     if (nx > 1 && ny > 1 && nz > 1) {
-        const int64_t cx = nx - 1, cy = ny - 1, cz = nz - 1, cells = cx * cy * cz;
-        const int64_t zs = (cz + ZC - 1) / ZC * ZC;
-        const int64_t tx = (cx + TILE_X - 1) / TILE_X, ty = (cy + WY - 1) / WY, st = (cx + 31) / 32;
-        b += 4 * (size_t)(tx * ty) + 4 * (size_t)st + table_bytes(nx + ny + nz) + 256;
-        b += (size_t)cy * cx * NCNT * (4 + 8) + (size_t)(zs / ZC) * tx * cy + (size_t)st * NCNT * 8;
-        b += (size_t)cells * (8 + 8 * dtype_size(r.T) + 4 + 1) + (size_t)(cells / ENT_BLOCK + 1) * 16;
+        const int64_t cx = nx - 1, cy = ny - 1, nzw = (nz + 31) / 32, sxy = nx * ny;
+        const int64_t nxb = (cx + BCOL - 1) / BCOL, nyb = (cy + BROW - 1) / BROW;
+        const int64_t segs = nzw, pieces = cx * cy * segs;  // at most one segment per word
+        b += 4 * (size_t)((sxy + 255) / 256 * nzw) + 4 * (size_t)(nxb * nyb * segs) + table_bytes(nx + ny + nz) + 256;
+        b += 4 * (size_t)(sxy * nzw + 3) + (size_t)pieces * sizeof(uint2);
+        b += (size_t)(pieces / BITS_TILE + 1) * sizeof(ulonglong2) + 4 * (size_t)(segs * cy * nxb);
     }
     return b;
 }
@@ -637,7 +623,7 @@ int launch_wave(mesh_server *s, Slot &sl) {
         std::vector<const Req *> rs;
         for (int64_t id : sl.groups[gi].reqs) rs.push_back(&sl.wave.at(id));
         layout_group(rs, &lays[gi]);
-        if (lays[gi].z.items >= ((int64_t)1 << 31) / WY) return MESH_ETOOLARGE;  // 32-bit compaction counter
+        if (lays[gi].z.bblks > 0x7fff0000 || lays[gi].z.cblks > 0x3fffffff) return MESH_ETOOLARGE;  // launch grids
         if (lays[gi].total > sl.groups[gi].scratch.size) return MESH_EDEVICE;  // bound violated: never launch
         sl.groups[gi].stage_off = stage;
         stage += up(lays[gi].head);
@@ -659,13 +645,12 @@ int launch_wave(mesh_server *s, Slot &sl) {
         int Q64 = 0, A64 = 0, P64 = 0;
         set_types(P, g.T, &prm, &Q64, &A64, &P64);
         const int L32 = prm.range_type == MESH_DT_F32;
-        std::vector<uint32_t> ivol, svol;
-        batch_owners(L.hv, L.z, ivol, svol);
+        std::vector<uint32_t> bvol, cvol;
+        batch_owners(L.hv, L.z, bvol, cvol);
         std::vector<TabJob> jobs;
         for (int v = 0; v < n; v++) {
             BatchVol &bv = L.hv[v];
             const Req &r = *rs[v];
-            bv.vol = r.vol;
             bv.tabs = (const double *)(blk + L.o_tabs) + L.tab_off[v];
             bv.verts = s->arena + r.out.off;
             bv.faces = (int64_t *)(s->arena + r.out.off + r.vbytes);
@@ -681,8 +666,8 @@ int launch_wave(mesh_server *s, Slot &sl) {
         // head: descriptors, owners, table jobs -- one copy from pinned staging
         char *hs = sl.stage + g.stage_off;
         memcpy(hs, L.hv.data(), sizeof(BatchVol) * n);
-        if (!ivol.empty()) memcpy(hs + L.o_ivol, ivol.data(), 4 * ivol.size());
-        if (!svol.empty()) memcpy(hs + L.o_svol, svol.data(), 4 * svol.size());
+        if (!bvol.empty()) memcpy(hs + L.o_bvol, bvol.data(), 4 * bvol.size());
+        if (!cvol.empty()) memcpy(hs + L.o_cvol, cvol.data(), 4 * cvol.size());
         if (!jobs.empty()) memcpy(hs + L.o_jobs, jobs.data(), sizeof(TabJob) * jobs.size());
         if ((e = cudaMemcpyAsync(blk, hs, L.head, cudaMemcpyHostToDevice, sl.stream)) != cudaSuccess)
             return MESH_ECUDA;
@@ -690,36 +675,12 @@ int launch_wave(mesh_server *s, Slot &sl) {
             (e = launch_tables_batch((const TabJob *)(blk + L.o_jobs), (int)jobs.size(), L.z.max_ntab, L32,
                                      sl.stream)) != cudaSuccess)
             return MESH_ECUDA;
-        P.pstride = L.z.pieces;
-        P.cnt = (uint32_t *)(blk + L.o_cnt);
-        P.base = (int64_t *)(blk + L.o_base);
-        P.flags = (uint8_t *)(blk + L.o_flags);
-        P.scan_state = (unsigned long long *)(blk + L.o_scan);
-        P.scan_ticket = (unsigned int *)(blk + L.o_scan + (size_t)std::max<int64_t>(L.z.stiles, n) * NCNT * 8);
-        P.totals = (int64_t *)(blk + L.o_misc);
-        P.err = (unsigned int *)((int64_t *)(blk + L.o_misc) + NCNT);
-        P.work = (unsigned int *)((int64_t *)(blk + L.o_misc) + NCNT + 1);
-        P.scan_spin_limit = 1 << 24;
-        P.bvols = (const BatchVol *)blk;
-        P.item_vol = (const uint32_t *)(blk + L.o_ivol);
-        P.stile_vol = (const uint32_t *)(blk + L.o_svol);
-        P.vol_off = (int64_t *)(blk + L.o_offs);
-        P.nitems = L.z.items;
-        P.nvols = n;
-        P.nstiles = (int32_t)L.z.stiles;
-        P.vol_outputs = 1;
-        P.ent_pos = (unsigned long long *)(blk + L.o_pos);
-        P.ent_val = blk + L.o_val;
-        P.ent_side = (long long *)(blk + L.o_side);
-        P.ent_vol = (uint32_t *)(blk + L.o_vol);
-        P.ent_cs = (uint8_t *)(blk + L.o_cs);
-        P.ent_cap = L.cells;
-        P.verts_cap = P.faces_cap = (int64_t)1 << 62;  // each volume checks its own block
-        if ((e = cudaMemsetAsync(blk + L.o_misc, 0, MISC_SLOTS * 8, sl.stream)) != cudaSuccess ||
-            (e = launch_classify_batch(P, 0, sl.stream)) != cudaSuccess ||
-            (e = launch_scan_batch(P, L.scan_vol ? 1024 : 256, sl.stream, L.scan_vol)) != cudaSuccess ||
-            (e = launch_compact_batch(P, 0, sl.stream)) != cudaSuccess ||
-            (e = launch_expand_batch(P, Q64, P64, sl.stream)) != cudaSuccess ||
+        bind_batch(P, L.z, n,
+                   BatchBufs{blk, blk + L.o_bvol, blk + L.o_cvol, blk + L.o_bits, blk + L.o_pc, blk + L.o_tsum,
+                             blk + L.o_mask, blk + L.o_misc, blk + L.o_offs});
+        P.vol_outputs = 1;  // each volume checks its own block
+        if ((e = launch_batch_counts(P, sl.stream)) != cudaSuccess ||
+            (e = launch_emit_batch(P, Q64, P64, 0, sl.stream)) != cudaSuccess ||
             (e = cudaMemcpyAsync(sl.res + g.res_off, P.vol_off, 16 * (size_t)(n + 1), cudaMemcpyDeviceToHost,
                                  sl.stream)) != cudaSuccess ||
             (e = cudaMemcpyAsync(sl.res + g.res_off + 2 * (n + 1), P.err, 4, cudaMemcpyDeviceToHost, sl.stream)) !=

@@ -238,11 +238,14 @@ __device__ __forceinline__ void mt_point(const Plan &p, int c1, int c2, T sv, T 
     const A hi = sizeof(A) == 4 ? (A)p.hi_f : (A)p.hi_d;
     const A a = jl_min<A>(jl_max<A>((A)q, eps), hi);
     const A b = Ar<A>::sub(A(1), a);
-    const bool nan = bits_nan(a);  // then b and every weight are NaN
     const A ab = Ar<A>::add(b, a);
+    const bool pos = bits_positive(a) && bits_positive(b);  // the products by 0 are +0
+    const bool nan = bits_nan(a);                           // then b and every weight are NaN
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const A w = nan ? a : corner_mix<A>((c1 >> k) & 1, (c2 >> k) & 1, b, a, ab);
+        const int k1 = (c1 >> k) & 1, k2 = (c2 >> k) & 1;
+        A w = k1 ? (k2 ? ab : b) : (k2 ? a : A(0));
+        if (!pos) w = nan ? a : corner_mix<A>(k1, k2, b, a, ab);
         r[k] = Ar<P>::add(b3[k], Ar<P>::mul((P)w, d3[k]));
     }
 }

@@ -158,6 +158,7 @@ void set_types(Plan &P, int T, const mesh_params *p, int *Q64, int *A64, int *P6
         P.iso_l = I == MESH_DT_I64 ? (int64_t)iso : 0;
     }
     P.isoq_d = iso;
+    P.iso_zero = iso == 0;
     P.iso_small = std::floor(iso) == iso && std::fabs(iso) <= 1073741824.0 && !(iso == 0 && std::signbit(iso));
     P.iso_s = P.iso_small ? (int32_t)iso : 0;
     P.isoq_f = (float)iso;

@@ -49,6 +49,7 @@ struct Plan {
     int64_t iso_l;
     int32_t iso_int;
     int32_t iso_small, iso_s;  // iso is the integer iso_s, at most 2^30 in magnitude
+    int32_t iso_zero;          // iso == 0 (tested here: a Float64 comparison is a Float64 operation)
     // iso as it enters (iso - v1)/(v2 - v1)
     float isoq_f;
     double isoq_d;
@@ -368,7 +369,7 @@ static __device__ __noinline__ double div_slow(double a, double b) { return __dd
 __device__ __forceinline__ double quotient_f64(float v1, float diff, const Plan &p) {
     uint64_t q;
     const uint32_t d = __float_as_uint(diff);
-    if (p.isoq_d == 0.0) {  // 0 - v1 (a zero v1 is left to the division)
+    if (p.iso_zero) {  // 0 - v1 (a zero v1 is left to the division)
         if (quot_f32_f32(__float_as_uint(v1) ^ 0x80000000u, d, q)) return __longlong_as_double((long long)q);
         return div_slow(__dsub_rn(p.isoq_d, widen<double>(v1)), (double)diff);
     }
@@ -423,16 +424,29 @@ __device__ __forceinline__ bool bits_finite(double v) {
 __device__ __forceinline__ bool bits_zero(float v) { return (__float_as_uint(v) << 1) == 0u; }
 __device__ __forceinline__ bool bits_zero(double v) { return ((unsigned long long)__double_as_longlong(v) << 1) == 0ull; }
 
+// signbit(x - y) for x, y that are not NaN: x before y in the order of the reals with
+// -0.0 < +0.0, compared as integers.
+__device__ __forceinline__ bool before(float x, float y) {
+    const int32_t a = __float_as_int(x), b = __float_as_int(y);
+    return (a ^ ((a >> 31) & 0x7fffffff)) < (b ^ ((b >> 31) & 0x7fffffff));
+}
+__device__ __forceinline__ bool before(double x, double y) {
+    const long long a = __double_as_longlong(x), b = __double_as_longlong(y);
+    return (a ^ ((a >> 63) & 0x7fffffffffffffffll)) < (b ^ ((b >> 63) & 0x7fffffffffffffffll));
+}
 // Base.max / Base.min on IEEE floats: NaN propagates, -0.0 < +0.0.
 template <class A> __device__ __forceinline__ A jl_max(A x, A y) {
-    A d = Ar<A>::sub(x, y);
-    if (bits_nan(x) || bits_nan(y)) return d;
-    return signbit(d) ? y : x;
+    if (bits_nan(x) || bits_nan(y)) return Ar<A>::sub(x, y);
+    return before(x, y) ? y : x;
 }
 template <class A> __device__ __forceinline__ A jl_min(A x, A y) {
-    A d = Ar<A>::sub(x, y);
-    if (bits_nan(x) || bits_nan(y)) return d;
-    return signbit(d) ? x : y;
+    if (bits_nan(x) || bits_nan(y)) return Ar<A>::sub(x, y);
+    return before(x, y) ? x : y;
+}
+// x > 0 and not NaN, by its bits.
+__device__ __forceinline__ bool bits_positive(float x) { return __float_as_uint(x) - 1u < 0x7f800000u; }
+__device__ __forceinline__ bool bits_positive(double x) {
+    return (unsigned long long)__double_as_longlong(x) - 1ull < 0x7ff0000000000000ull;
 }
 
 // fl32(fl64(p1 + fl64(mu * d))) for a Float32 mu and Float64 p1, d given as

@@ -345,6 +345,7 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, int
         static_assert(32 * BROW == 256, "one entry per thread");
         __syncthreads();
     }
+    after_previous();
     BView v;
     unsigned blk = blockIdx.x;
     if constexpr (BATCH) {
@@ -504,6 +505,7 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, int
 // The tiles' sums to offsets, for grids that do not scan them themselves.
 __global__ void __launch_bounds__(1024) k_scan_tiles(const Plan p) {
     __shared__ unsigned long long s_w[2][32];
+    after_previous();
     scan_tiles<32>(p, s_w);
 }
 
@@ -518,6 +520,7 @@ __global__ void __launch_bounds__(OFF_T) k_offsets(const Plan p) {
     __shared__ uint2 s_w[OFF_T / 32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int64_t e0 = (int64_t)blockIdx.x * BITS_TILE + (int64_t)tid * OFF_N;
+    after_previous();
     uint4 *q = reinterpret_cast<uint4 *>(p.pc + e0);
     uint2 n[OFF_N];
     if (e0 + OFF_N <= p.npc) {
@@ -571,6 +574,7 @@ __global__ void __launch_bounds__(OFF_T) k_offsets(const Plan p) {
 // Batch: first vertex / face of every volume, then the totals.
 __global__ void __launch_bounds__(256) k_batch_rows(const Plan p) {
     const int i = blockIdx.x * 256 + threadIdx.x;
+    after_previous();
     if (i > p.nvols) return;
     const int64_t e = i < p.nvols ? p.bvols[i].e0 : p.npc;
     int64_t vo = p.totals[0], fo = p.totals[1];
@@ -640,11 +644,13 @@ static cudaError_t go_count(const Plan &p, int seg0, int nseg, bool vpre_only, c
     const int64_t nitems = BATCH ? p.ncblk : per * ((nseg + gs - 1) / gs);
     const bool one = nitems <= ONE_WAVE && (BATCH || nseg == p.bseg);
     if (nitems > 0x7fffffff) return cudaErrorInvalidConfiguration;
+    cudaError_t e = cudaSuccess;
     if (nitems > 0)
-        k_count<ALG, BATCH><<<(unsigned)nitems, 32 * BROW, 0, s>>>(p, seg0, seg0 + nseg, gs, one ? (unsigned)nitems : 0u,
-                                                                 vpre_only);
-    if (!one && !vpre_only && (BATCH || seg0 + nseg == p.bseg)) k_scan_tiles<<<1, 1024, 0, s>>>(p);
-    return cudaGetLastError();
+        e = launch_after(k_count<ALG, BATCH>, (unsigned)nitems, 32 * BROW, 0, s, p, seg0, seg0 + nseg, gs,
+                         one ? (unsigned)nitems : 0u, vpre_only);
+    if (e == cudaSuccess && !one && !vpre_only && (BATCH || seg0 + nseg == p.bseg))
+        e = launch_after(k_scan_tiles, 1, 1024, 0, s, p);
+    return e;
 }
 
 cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s, bool vpre_only) {
@@ -679,14 +685,12 @@ cudaError_t launch_count_batch(const Plan &p, cudaStream_t s) {
 }
 
 cudaError_t launch_batch_rows(const Plan &p, cudaStream_t s) {
-    k_batch_rows<<<p.nvols / 256 + 1, 256, 0, s>>>(p);
-    return cudaGetLastError();
+    return launch_after(k_batch_rows, (unsigned)(p.nvols / 256 + 1), 256, 0, s, p);
 }
 
 cudaError_t launch_offsets(const Plan &p, cudaStream_t s) {
     if (p.ntiles < 1) return cudaSuccess;
-    k_offsets<<<(unsigned)p.ntiles, OFF_T, 0, s>>>(p);
-    return cudaGetLastError();
+    return launch_after(k_offsets, (unsigned)p.ntiles, OFF_T, 0, s, p);
 }
 
 cudaError_t launch_gather_pieces(const Plan &p, const GatherIdx &g, int64_t *dst, cudaStream_t s) {

@@ -195,16 +195,18 @@ struct OutView {
     long long vcap, fcap, v0, f0, id0, kbase;
 };
 
-// b: the item's volume of a batch (null: the plan's single volume).
+// b: the item's volume of a batch (null: the plan's single volume); cols: the item's
+// columns of the 32.
 template <class T, class Q, class P, int PM, bool BATCH>
 __device__ __forceinline__ void emit_item(const Plan &p, const BatchVol *b, const BView &v, const Tabs &tb,
-                                          EmitWarp<T, PM> &w, const CaseTabs &ct, int lane, int xb, int y, int seg) {
+                                          EmitWarp<T, PM> &w, const CaseTabs &ct, int lane, int xb, int y, int seg,
+                                          uint32_t cols) {
     constexpr int VB = 3 * (PM == PM_F64 ? 8 : 4);  // bytes of a vertex
     const int mw = mask_words(min(v.zws, (v.cz + 31) / 32 - seg * v.zws));
     const uint32_t *mp = p.wmask + bmask(v, seg, y, xb);
     const int x0 = xb * BCOL, x = x0 + lane;
     const int zws0 = seg * v.zws;
-    const bool xin = x < v.cx;
+    const bool xin = x < v.cx && (BATCH || ((cols >> lane) & 1u));
     bool ready = false;            // the item's offsets and x, y nodes are loaded
     bool zeroxy = false;
     long long gv = 0, gf = 0;      // this column's next vertex / face
@@ -364,7 +366,7 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BatchVol *b, cons
 }
 
 template <class T, class Q, class P, int PM>
-__global__ void __launch_bounds__(32 * EW, 3) k_emit_bits_mc(const Plan p, int seg0, int nseg, int nitems) {
+__global__ void __launch_bounds__(32 * EW, 3) k_emit_bits_mc(const Plan p, int seg0, int nseg, int nitems, int lg) {
     extern __shared__ __align__(16) unsigned char esm[];
     CaseTabs &ct = *reinterpret_cast<CaseTabs *>(esm);
     EmitWarp<T, PM> *sw = reinterpret_cast<EmitWarp<T, PM> *>(esm + sizeof(CaseTabs));
@@ -375,15 +377,15 @@ __global__ void __launch_bounds__(32 * EW, 3) k_emit_bits_mc(const Plan p, int s
     const BView v = view_of(p);
     const Tabs tb = tabs_of(p);
     const int nxb = p.ntx > 0 ? p.ntx : v.nxb;  // column blocks tx0 .. tx0 + ntx - 1
-    for (;;) {
-        int item = 0;
-        if (lane == 0) item = (int)atomicAdd(p.work, 1u);
-        item = __shfl_sync(FULL, item, 0);
-        if (item >= nitems) break;
-        const int xb = p.tx0 + item % nxb;
-        const int seg = seg0 + (item / nxb) % nseg;
-        const int y = item / (nxb * nseg);
-        emit_item<T, Q, P, PM, false>(p, nullptr, v, tb, sw[wi], ct, lane, xb, y, seg);
+    after_previous();
+    // the first item of a warp is its own number, spread over the CTAs
+    for (int item = wi * gridDim.x + blockIdx.x; item < nitems; item = next_item(p, lane)) {
+        const int q = item >> lg, width = 32 >> lg, part = item & ((1 << lg) - 1);  // 1 << lg parts of 32 columns
+        const int xb = p.tx0 + q % nxb;
+        const int seg = seg0 + (q / nxb) % nseg;
+        const int y = q / (nxb * nseg);
+        emit_item<T, Q, P, PM, false>(p, nullptr, v, tb, sw[wi], ct, lane, xb, y, seg,
+                                      (FULL >> (32 - width)) << (width * part));
     }
 }
 
@@ -401,6 +403,7 @@ __global__ void __launch_bounds__(32 * EW, 3) k_emit_bits_batch(const Plan p, in
         reinterpret_cast<uint4 *>(&ct)[i] = reinterpret_cast<const uint4 *>(&d_cases)[i];
     __syncthreads();
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
+    after_previous();
     for (;;) {
         unsigned item = 0;
         if (lane == 0) item = atomicAdd(p.work, 1u);
@@ -420,7 +423,7 @@ __global__ void __launch_bounds__(32 * EW, 3) k_emit_bits_batch(const Plan p, in
         }
         const Tabs tb = tabs_at(b->tabs, v.nx, v.ny, v.nz);
         for (uint32_t todo = __ballot_sync(FULL, any != 0u); todo; todo &= todo - 1)
-            emit_item<T, Q, P, PM, true>(p, b, v, tb, sw[wi], ct, lane, xb, y0 + __ffs(todo) - 1, seg);
+            emit_item<T, Q, P, PM, true>(p, b, v, tb, sw[wi], ct, lane, xb, y0 + __ffs(todo) - 1, seg, FULL);
     }
 }
 
@@ -462,9 +465,8 @@ template <class T, class Q, class P, int PM> cudaError_t go_batch(const Plan &p,
     if (grid < 1) return cudaErrorInvalidDevice;
     if (nitems > 0x7fffffff) return cudaErrorInvalidConfiguration;
     if (nitems < 1) return cudaSuccess;
-    k_emit_bits_batch<T, Q, P, PM>
-        <<<(int)std::min<int64_t>(grid, (nitems + EW - 1) / EW), 32 * EW, emit_smem<T, PM>(), s>>>(p, nitems, rows);
-    return cudaGetLastError();
+    return launch_after(k_emit_bits_batch<T, Q, P, PM>, (unsigned)std::min<int64_t>(grid, nitems), 32 * EW,
+                        emit_smem<T, PM>(), s, p, nitems, rows);
 }
 
 template <class T, class Q, class P, int PM> cudaError_t go(const Plan &p, const Range &r, cudaStream_t s) {
@@ -472,14 +474,19 @@ template <class T, class Q, class P, int PM> cudaError_t go(const Plan &p, const
     const int seg0 = r.seg0, nseg = r.nseg;
     int sms = 0;
     const int grid = emit_ctas<T, Q, P, PM, false>(&sms) * sms;
-    const int64_t nitems = (int64_t)(p.ntx > 0 ? p.ntx : p.nxb) * nseg * p.cy;
+    // volumes of few rows: items of 8 columns, so that every SM has some and dense ones
+    // (a row's word of 32 x 32 active cells is 32 batches) end together (128^3 sines
+    // 56 -> 44 us a call)
+    const int64_t rows = (int64_t)(p.ntx > 0 ? p.ntx : p.nxb) * nseg * p.cy;
+    const int lg = rows < 2 * EW * (int64_t)grid ? 2 : 0;
+    const int64_t nitems = rows << lg;
     if (grid < 1) return cudaErrorInvalidDevice;
     if (nitems > 0x7fffffff - 65536) return cudaErrorInvalidConfiguration;
     if (nitems < 1) return cudaSuccess;
-    k_emit_bits_mc<T, Q, P, PM><<<(int)std::min<int64_t>(grid, (nitems + EW - 1) / EW), 32 * EW, emit_smem<T, PM>(), s>>>(
-        p, seg0, nseg, (int)nitems);
-    return cudaGetLastError();
+    return launch_after(k_emit_bits_mc<T, Q, P, PM>, (unsigned)std::min<int64_t>(grid, nitems), 32 * EW, emit_smem<T, PM>(),
+                        s, p, seg0, nseg, (int)nitems, lg);
 }
+
 template <class T> cudaError_t go_t(const Plan &p, int Q64, int P64, const Range &r, cudaStream_t s) {
     if (p.out64) {
         if (Q64) return go<T, double, double, PM_F64>(p, r, s);

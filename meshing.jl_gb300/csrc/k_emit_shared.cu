@@ -296,7 +296,7 @@ template <int E> __device__ __forceinline__ uint32_t mt_extra(const uint32_t (&w
 template <class T, class Q, class A, class P, int ALG>
 __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const Tabs &tb, SharedWarp<T, P, ALG> &w,
                                           const typename TabsOf<ALG>::type &ct, const P *rcp, int lane, int xb, int y,
-                                          int seg) {
+                                          int seg, uint32_t cols) {
     const int mw = mask_words(min(v.zws, (v.cz + 31) / 32 - seg * v.zws));
     const uint32_t *mp = p.wmask + bmask(v, seg, y, xb);
     const int x0 = xb * BCOL, x = x0 + lane;
@@ -305,7 +305,7 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
     bool zeroxy = false;
     long long V0 = 0;           // with an x halo, its cell column's totals: every output is shifted by them
     long long gf = 0;           // this column's next face
-    const bool mine = x < v.cx && !(p.xhalo && x == 0);
+    const bool mine = x < v.cx && !(p.xhalo && x == 0) && ((cols >> lane) & 1u);
     const T *s0 = (const T *)v.vol + v.nx * y + x0;
     auto first = [&](int yy, int xx, long long &vo, long long &fo) {
         const int64_t e = bpiece(v, seg, yy, xx);
@@ -638,7 +638,7 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
 }
 
 template <class T, class Q, class A, class P, int ALG>
-__global__ void __launch_bounds__(32 * SW, 2) k_emit_shared(const Plan p, int seg0, int nseg, int nitems) {
+__global__ void __launch_bounds__(32 * SW, 2) k_emit_shared(const Plan p, int seg0, int nseg, int nitems, int lg) {
     using Tab = typename TabsOf<ALG>::type;
     extern __shared__ __align__(16) unsigned char ssm[];
     __shared__ P s_rcp[13];  // NSN: RN(1/n) for the crossing counts n
@@ -652,15 +652,18 @@ __global__ void __launch_bounds__(32 * SW, 2) k_emit_shared(const Plan p, int se
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
     const BView v = view_of(p);
     const Tabs tb = tabs_of(p);
+    after_previous();
     for (;;) {
         int item = 0;
         if (lane == 0) item = (int)atomicAdd(p.work, 1u);
         item = __shfl_sync(FULL, item, 0);
         if (item >= nitems) break;
-        const int xb = item % v.nxb;
-        const int seg = seg0 + (item / v.nxb) % nseg;
-        const int y = item / (v.nxb * nseg);
-        emit_item<T, Q, A, P, ALG>(p, v, tb, sw[wi], ct, s_rcp, lane, xb, y, seg);
+        const int q = item >> lg, width = 32 >> lg, part = item & ((1 << lg) - 1);  // 1 << lg parts of 32 columns
+        const int xb = q % v.nxb;
+        const int seg = seg0 + (q / v.nxb) % nseg;
+        const int y = q / (v.nxb * nseg);
+        emit_item<T, Q, A, P, ALG>(p, v, tb, sw[wi], ct, s_rcp, lane, xb, y, seg,
+                                   (FULL >> (32 - width)) << (width * part));
     }
 }
 
@@ -689,13 +692,14 @@ template <class T, class Q, class A, class P, int ALG> int shared_grid() {
 
 template <class T, class Q, class A, class P, int ALG> cudaError_t go(const Plan &p, int seg0, int nseg, cudaStream_t s) {
     const int grid = shared_grid<T, Q, A, P, ALG>();
-    const int64_t nitems = (int64_t)p.nxb * nseg * p.cy;
+    const int64_t rows = (int64_t)p.nxb * nseg * p.cy;
+    const int lg = rows < 2 * SW * (int64_t)grid ? 2 : 0;  // as in k_emit_bits.cu
+    const int64_t nitems = rows << lg;
     if (grid < 1) return cudaErrorInvalidDevice;
     if (nitems > 0x7fffffff - 65536) return cudaErrorInvalidConfiguration;
     if (nitems < 1) return cudaSuccess;
-    k_emit_shared<T, Q, A, P, ALG><<<(int)std::min<int64_t>(grid, (nitems + SW - 1) / SW), 32 * SW,
-                                     shared_smem<T, P, ALG>(), s>>>(p, seg0, nseg, (int)nitems);
-    return cudaGetLastError();
+    return launch_after(k_emit_shared<T, Q, A, P, ALG>, (unsigned)std::min<int64_t>(grid, nitems), 32 * SW,
+                        shared_smem<T, P, ALG>(), s, p, seg0, nseg, (int)nitems, lg);
 }
 
 template <class T> cudaError_t go_t(const Plan &p, int Q64, int A64, int P64, int seg0, int nseg, cudaStream_t s) {

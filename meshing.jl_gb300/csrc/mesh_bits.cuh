@@ -45,6 +45,25 @@ inline __host__ __device__ int64_t bmask(const BView &v, int seg, int y, int xb)
 #ifdef __CUDACC__
 namespace mesh {
 
+// Launch of a kernel that begins with after_previous(): its CTAs may start, and set
+// up what depends on no earlier kernel, while the previous kernel of the stream
+// drains (programmatic dependent launch; 256^3 gyroid 183 -> 171 us a call).
+template <class... A, class... B>
+inline cudaError_t launch_after(void (*k)(A...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s, B... args) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute a = {};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k, static_cast<A>(args)...);
+}
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ BView view_of(const Plan &p) {
     return BView{p.vol, p.bits, p.nx, p.ny, p.nz, p.nx * p.ny, p.cx, p.cy, p.cz, p.nxb, p.nyb,
                  p.bseg, p.zws, p.nzw, p.bw0, 0, 0};
@@ -53,6 +72,13 @@ __device__ __forceinline__ BView view_of(const Plan &p) {
 __device__ __forceinline__ BView view_of(const Plan &p, const BatchVol &b) {
     return BView{b.vol, p.bits + b.bits0, b.nx, b.ny, b.nz, b.nx * b.ny, b.cx, b.cy, b.cz, b.nxb, b.nyb,
                  b.bseg, b.zws, b.nzw, 0, b.e0, b.m0};
+}
+
+// The next item of a persistent warp whose first was its number in the grid.
+__device__ __forceinline__ int next_item(const Plan &p, int lane) {
+    int item = 0;
+    if (lane == 0) item = (int)(gridDim.x * (blockDim.x >> 5) + atomicAdd(p.work, 1u));
+    return __shfl_sync(0xffffffffu, item, 0);
 }
 
 // The four corner columns of column (x, y) in one word of z, and the same one

@@ -262,6 +262,33 @@ template <int T> __device__ __forceinline__ uint32_t mt_triangles(const uint32_t
     return n;
 }
 
+// Welded Marching Cubes: the nine edges that only cells on the lower faces own, as
+// pairs of corner words in MT corner order (the other three end at corner 6).
+struct McLow {
+    uint8_t a[9], b[9], low[9];
+};
+constexpr McLow make_mc_low() {
+    McLow t{};
+    constexpr int EA[12] = {0, 1, 3, 2, 4, 5, 7, 6, 0, 1, 3, 2}, EB[12] = {1, 3, 2, 0, 5, 7, 6, 4, 4, 5, 7, 6};
+    constexpr int WORD[8] = {0, 3, 1, 2, 4, 7, 5, 6};  // corner x | y << 1 | z << 2
+    int n = 0;
+    for (int e = 0; e < 12; e++) {
+        const int low = 7 & ~(EA[e] | EB[e]);
+        if (!low) continue;
+        t.a[n] = (uint8_t)WORD[EA[e]];
+        t.b[n] = (uint8_t)WORD[EB[e]];
+        t.low[n++] = (uint8_t)low;
+    }
+    return t;
+}
+constexpr McLow MC_LOW = make_mc_low();
+template <int K> __device__ __forceinline__ uint32_t mc_boundary(const uint32_t (&w)[8], uint32_t zm, uint32_t z0, int low) {
+    constexpr int la = MC_LOW.low[K], ea = MC_LOW.a[K], eb = MC_LOW.b[K];
+    const uint32_t r = (la & ~low & 3) ? 0u : __popc((w[ea] ^ w[eb]) & ((la & 4) ? z0 : zm));
+    if constexpr (K + 1 < 9) return r + mc_boundary<K + 1>(w, zm, z0, low);
+    return r;
+}
+
 template <int E> __device__ __forceinline__ uint32_t mt_owned(const uint32_t (&w)[8], uint32_t zm, uint32_t z0, int low) {
     // edge E of the cells zm, owned when its low axes are grid boundaries
     constexpr int la = MT_E.low[E], ea = MT_E.a[E], eb = MT_E.b[E];
@@ -340,7 +367,7 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, int
     __shared__ unsigned long long s_w[2][BROW];
     __shared__ int s_last;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    if (ALG == MESH_ALG_MC) {
+    if (ALG == MESH_ALG_MC || ALG == MESH_ALG_MC_WELDED) {
         s_loops[tid] = d_loops.extra[tid];
         static_assert(32 * BROW == 256, "one entry per thread");
         __syncthreads();
@@ -408,7 +435,7 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, int
                     const Corners q{a[k], b[k], c[k], d[k], __funnelshift_r(a[k], a[k + 1], 1),
                                     __funnelshift_r(b[k], b[k + 1], 1), __funnelshift_r(c[k], c[k + 1], 1),
                                     __funnelshift_r(d[k], d[k + 1], 1)};
-                    if (ALG == MESH_ALG_MC) {
+                    if (ALG == MESH_ALG_MC || ALG == MESH_ALG_MC_WELDED) {
                         uint32_t loops = __popc(act);
                         const uint32_t cross = __popc((q.a ^ q.b) & zm) + __popc((q.c ^ q.d) & zm) + __popc((q.a ^ q.c) & zm) +
                                                __popc((q.b ^ q.d) & zm) + __popc((q.as ^ q.bs) & zm) +
@@ -418,8 +445,16 @@ __global__ void __launch_bounds__(32 * BROW) k_count(const Plan p, int seg0, int
                         for (uint32_t m = many_loops(q) & zm; m; m &= m - 1)
                             loops += s_loops[cell_index(a[k], b[k], c[k], d[k], a[k + 1], b[k + 1], c[k + 1], d[k + 1],
                                                         __ffs(m) - 1)];
-                        nv += cross;
                         nf += cross - 2 * loops;
+                        if (ALG == MESH_ALG_MC) {
+                            nv += cross;
+                        } else {
+                            const MtWords m(q);
+                            const int low = (x == 0) | ((y == 0) << 1);
+                            nv += __popc((q.ds ^ q.cs) & zm) + __popc((q.ds ^ q.bs) & zm) + __popc((q.ds ^ q.d) & zm);
+                            if (zw == 0 || __any_sync(FULL, low != 0))
+                                nv += mc_boundary<0>(m.w, zm, zw == 0 ? zm & 1u : 0u, low);
+                        }
                     } else if (ALG == MESH_ALG_MT) {
                         const MtWords m(q);
                         uint32_t own = 0;
@@ -656,6 +691,7 @@ static cudaError_t go_count(const Plan &p, int seg0, int nseg, bool vpre_only, c
 cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s, bool vpre_only) {
     if (p.alg == MESH_ALG_MC) return go_count<MESH_ALG_MC, false>(p, seg0, nseg, vpre_only, s);
     if (p.alg == MESH_ALG_MT) return go_count<MESH_ALG_MT, false>(p, seg0, nseg, vpre_only, s);
+    if (p.alg == MESH_ALG_MC_WELDED) return go_count<MESH_ALG_MC_WELDED, false>(p, seg0, nseg, vpre_only, s);
     return go_count<MESH_ALG_NSN, false>(p, seg0, nseg, vpre_only, s);
 }
 

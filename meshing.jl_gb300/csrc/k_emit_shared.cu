@@ -1,4 +1,5 @@
-// Marching Tetrahedra and Naive Surface Nets emission from the sign bits.
+// Marching Tetrahedra, welded Marching Cubes and Naive Surface Nets emission from
+// the sign bits.
 //
 // MT shares vertices between cells: the reference keys every lattice edge in a
 // Dict and numbers a vertex when a cell first touches its edge in traversal
@@ -12,14 +13,16 @@
 //     first-use order after all vertices of earlier cells;
 //   * a cell that uses an edge owned by a neighbour needs the neighbour's case
 //     and first vertex.
+// Welded Marching Cubes (MESH_ALG_MC_WELDED) numbers the crossed lattice edges in the
+// same way, in the order of the first cell's Marching Cubes vertices.
 // NSN gives every active cell one vertex and connects the four cells around
 // every crossed base edge, so it needs the same neighbours' first vertices.
 //
 // Work items, words and lists of active cells are those of k_emit_bits.cu; a
 // batch is again 32 cells, one per lane.  Any cell's first vertex follows from
 // bits alone: its column's offset, the vertices of the words below (left by
-// k_count) and, in the word, population counts of the owned crossed edges (MT)
-// or active cells (NSN) below it.  So each lane reads the 3 x 3 columns around
+// k_count) and, in the word, population counts of the owned crossed edges or active
+// cells (NSN) below it.  So each lane reads the 3 x 3 columns around
 // its cell, at z - 1 .. z + 1, and leaves the cases and first vertices of the
 // cells one step back along each set of axes in shared memory; the batch's
 // vertices and faces are then dense task lists whatever the density.
@@ -87,16 +90,45 @@ constexpr int bits_of(uint32_t m) {
     return n;
 }
 
-struct alignas(16) MtTabs {
-    uint8_t ref[256][3 * MT_MAX_FACES];  // triangle corners: owner's axes back << 5 | the edge in the owner
-    uint8_t rank[256][20];               // interior cells: rank of an edge among the owned ones
-    uint8_t kth[256][8];                 // interior cells: the k-th owned crossed edge in first-use order
-    uint8_t nvf[256];                    // interior vertices | faces << 4
-    uint8_t unmoved[8][20];              // the edge of `ref` seen from the cells between it and the owner
-    uint8_t corner[32];                  // an edge's corners x | y << 1 | z << 2, start | end << 3
+// The same of the Marching Cubes edges (mesh_tables.h numbering, corner bits x | y << 1 | z << 2).
+constexpr int MC_A[12] = {0, 1, 3, 2, 4, 5, 7, 6, 0, 1, 3, 2}, MC_B[12] = {1, 3, 2, 0, 5, 7, 6, 4, 4, 5, 7, 6};
+constexpr int mc_low_axes(int e) { return 7 & ~(MC_A[e] | MC_B[e]); }
+constexpr int mc_moved_edge(int e, int s, int dir) {
+    const int a = dir > 0 ? MC_A[e] | s : MC_A[e] & ~s, b = dir > 0 ? MC_B[e] | s : MC_B[e] & ~s;
+    if (dir > 0 ? ((MC_A[e] | MC_B[e]) & s) != 0 : ((MC_A[e] & MC_B[e]) & s) != s) return 31;
+    for (int f = 0; f < 12; f++)
+        if ((MC_A[f] == a && MC_B[f] == b) || (MC_A[f] == b && MC_B[f] == a)) return f;
+    return 31;
+}
+constexpr uint32_t mc_own_mask(int bnd) {
+    uint32_t m = 0;
+    for (int e = 0; e < 12; e++)
+        if ((mc_low_axes(e) & ~bnd) == 0) m |= 1u << e;
+    return m;
+}
+
+// Per algorithm: most triangles, edges, own edges of an interior cell, most vertices.
+template <int ALG> struct EdgeDims { static constexpr int F = MT_MAX_FACES, E = 19, OWN = 8, V = MT_MAX_TOUCH; };
+template <> struct EdgeDims<MESH_ALG_MC_WELDED> { static constexpr int F = MC_MAX_FACES, E = 12, OWN = 4, V = MC_MAX_VERTS; };
+
+template <int ALG> struct alignas(16) EdgeTabs {
+    using D = EdgeDims<ALG>;
+    uint8_t ref[256][3 * D::F];        // triangle corners: owner's axes back << 5 | the edge in the owner
+    uint8_t rank[256][D::E];           // interior cells: rank of an edge among the owned ones
+    uint8_t kth[256][D::OWN];          // interior cells: the k-th owned crossed edge in first-use order
+    uint8_t nvf[256];                  // interior vertices | faces << 4
+    uint8_t unmoved[8][D::E];          // the edge of `ref` seen from the cells between it and the owner
+    uint8_t corner[32];                // an edge's corners x | y << 1 | z << 2, start | end << 3
 };
-constexpr MtTabs make_mt_tabs() {
-    MtTabs t{};
+// Cells on the grid's lower faces own more edges: the full tables.
+template <int ALG> struct EdgeFull {
+    using D = EdgeDims<ALG>;
+    uint32_t touched[256], before[256][D::E], own[8];
+    uint8_t order[256][D::V];
+};
+
+constexpr EdgeTabs<MESH_ALG_MT> make_mt_tabs() {
+    EdgeTabs<MESH_ALG_MT> t{};
     for (int i = 0; i < 256; i++) {
         const int c = (int)mt_case_of_bits((unsigned)i);
         for (int k = 0; k < 3 * MT_CASE_NFACES[c]; k++) {
@@ -119,26 +151,67 @@ constexpr MtTabs make_mt_tabs() {
     }
     return t;
 }
-__device__ const MtTabs d_mt = make_mt_tabs();
-static_assert(sizeof(MtTabs) % 16 == 0, "copied in 16-byte words");
-static_assert(MT_MAX_FACES <= 15 && bits_of(own_mask(0)) <= 8, "packed counts");
-
-// Cells on the grid's lower faces own more edges: the full tables.
-struct MtFull {
-    uint32_t touched[256], before[256][19];
-    uint8_t order[256][MT_MAX_TOUCH];
-};
-constexpr MtFull make_mt_full() {
-    MtFull t{};
+constexpr EdgeFull<MESH_ALG_MT> make_mt_full() {
+    EdgeFull<MESH_ALG_MT> t{};
     for (int i = 0; i < 256; i++) {
         const int c = (int)mt_case_of_bits((unsigned)i);
         t.touched[i] = MT_TOUCHED[c] & 0x7ffffu;
         for (int e = 0; e < 19; e++) t.before[i][e] = MT_BEFORE[c][e];
         for (int k = 0; k < MT_MAX_TOUCH; k++) t.order[i][k] = MT_TOUCH_ORDER[c][k];
     }
+    for (int b = 0; b < 8; b++) t.own[b] = own_mask(b);
     return t;
 }
-__device__ const MtFull d_mtf = make_mt_full();
+constexpr EdgeFull<MESH_ALG_MC_WELDED> make_mc_full() {
+    EdgeFull<MESH_ALG_MC_WELDED> t{};
+    for (int i = 0; i < 256; i++) {
+        const uint64_t v = MC_CASE_VERTS[mc_case_of_bits((unsigned)i)];
+        const int n = (int)((v >> 48) & 15u);
+        for (int k = 0; k < MC_MAX_VERTS; k++) t.order[i][k] = 255;
+        uint32_t m = 0;
+        for (int k = 0; k < n; k++) {
+            const int e = (int)((v >> (4 * k)) & 15u);
+            t.order[i][k] = (uint8_t)e;
+            t.before[i][e] = m;
+            m |= 1u << e;
+        }
+        t.touched[i] = m;
+    }
+    for (int b = 0; b < 8; b++) t.own[b] = mc_own_mask(b);
+    return t;
+}
+constexpr EdgeTabs<MESH_ALG_MC_WELDED> make_mc_tabs() {
+    EdgeTabs<MESH_ALG_MC_WELDED> t{};
+    constexpr EdgeFull<MESH_ALG_MC_WELDED> full = make_mc_full();
+    for (int i = 0; i < 256; i++) {
+        const unsigned c = mc_case_of_bits((unsigned)i);
+        const int nf = (int)((MC_CASE_VERTS[c] >> 52) & 7u);
+        for (int k = 0; k < 3 * nf; k++) {
+            const int e = full.order[i][(MC_CASE_FACES[c] >> (4 * k)) & 15u], s = mc_low_axes(e);
+            t.ref[i][k] = (uint8_t)((s << 5) | mc_moved_edge(e, s, 1));
+        }
+        for (int e = 0; e < 12; e++) t.rank[i][e] = (uint8_t)bits_of(full.before[i][e] & mc_own_mask(0));
+        int n = 0;
+        for (int k = 0; k < MC_MAX_VERTS; k++)
+            if (full.order[i][k] < 12 && ((mc_own_mask(0) >> full.order[i][k]) & 1u)) t.kth[i][n++] = full.order[i][k];
+        t.nvf[i] = (uint8_t)(n | (nf << 4));
+    }
+    for (int s = 0; s < 8; s++)
+        for (int e = 0; e < 12; e++) t.unmoved[s][e] = (uint8_t)mc_moved_edge(e, s, -1);
+    for (int e = 0; e < 12; e++) t.corner[e] = (uint8_t)(MC_A[e] | (MC_B[e] << 3));
+    return t;
+}
+__device__ const EdgeTabs<MESH_ALG_MT> d_mt = make_mt_tabs();
+__device__ const EdgeFull<MESH_ALG_MT> d_mt_full = make_mt_full();
+__device__ const EdgeTabs<MESH_ALG_MC_WELDED> d_mc = make_mc_tabs();
+__device__ const EdgeFull<MESH_ALG_MC_WELDED> d_mc_full = make_mc_full();
+template <int ALG> __device__ __forceinline__ const EdgeFull<ALG> &full_tabs() {
+    if constexpr (ALG == MESH_ALG_MT) return d_mt_full;
+    else return d_mc_full;
+}
+static_assert(sizeof(EdgeTabs<MESH_ALG_MT>) % 16 == 0 && sizeof(EdgeTabs<MESH_ALG_MC_WELDED>) % 16 == 0,
+              "copied in 16-byte words");
+static_assert(MT_MAX_FACES <= 15 && bits_of(own_mask(0)) <= 8 && bits_of(mc_own_mask(0)) <= 4, "packed counts");
 
 // NSN: a cell's crossed edges in MC edge order, start corner | axis << 3, and their number.
 struct alignas(16) NsnTabs {
@@ -164,7 +237,7 @@ constexpr NsnTabs make_nsn_tabs() {
 __device__ const NsnTabs d_nsn = make_nsn_tabs();
 static_assert(sizeof(NsnTabs) % 16 == 0, "copied in 16-byte words");
 
-template <int ALG> struct TabsOf { using type = MtTabs; };
+template <int ALG> struct TabsOf { using type = EdgeTabs<ALG>; };
 template <> struct TabsOf<MESH_ALG_NSN> { using type = NsnTabs; };
 
 // ---- shared memory of one warp ----
@@ -177,7 +250,7 @@ template <class P> struct Pairs<P, MESH_ALG_NSN> {
 template <class T, class P, int ALG> struct SharedWarp {
     unsigned long long win[3][NC];  // rows y-1 .. y+1: bit 0 the sample below the word, 1-32 the word, 33 above
     long long col[2][NC];           // rows y-1, y, columns x0-1 ..: first vertex of the column's word
-    long long nb[8][32];            // per cell: first vertex (MT: << 8 | cell index) of the cell back along the axes
+    long long nb[8][32];            // per cell: first vertex (NSN; else << 8 | cell index) of the cell back along the axes
     long long fb[32];               // per cell: first face
     P p[NT], d[NT];                 // nodes and spacings
     Pairs<P, ALG> pr;
@@ -262,9 +335,11 @@ __device__ __forceinline__ bool put_node(W &w, int i, const Tabs &tb, int64_t ax
     return bits_zero(w.p[i]) && signbit(w.p[i]);
 }
 
-// MT vertices of a column's word below bit z (m: the lower cells that exist), the
-// column's corner words in MT corner order.
-__device__ __forceinline__ uint32_t mt_below(const uint32_t (&w)[8], uint32_t m) {
+// Vertices of a column's word below bit z (m: the lower cells that exist) that its
+// cells own inside the grid, the column's corner words in MT corner order.
+template <int ALG> __device__ __forceinline__ uint32_t own_below(const uint32_t (&w)[8], uint32_t m) {
+    if constexpr (ALG == MESH_ALG_MC_WELDED)  // the three edges that end at the upper corner
+        return __popc((w[6] ^ w[5]) & m) + __popc((w[6] ^ w[7]) & m) + __popc((w[6] ^ w[2]) & m);
     uint32_t n = 0;
 #pragma unroll
     for (int k = 0; k < 8; k++) n += k == 6 ? 0u : __popc((w[k] ^ w[6]) & m);
@@ -275,21 +350,24 @@ __device__ __forceinline__ uint32_t mt_below(const uint32_t (&w)[8], uint32_t m)
 struct EdgeInfo {
     uint8_t a[19], b[19], low[19];
 };
-constexpr EdgeInfo make_edge_info() {
+constexpr EdgeInfo make_edge_info(bool mc) {
     EdgeInfo t{};
-    for (int e = 0; e < 19; e++) {
-        t.a[e] = MT_EDGE_CORNERS[e][0];
-        t.b[e] = MT_EDGE_CORNERS[e][1];
-        t.low[e] = (uint8_t)low_axes(e);
+    constexpr int WORD[8] = {0, 3, 1, 2, 4, 7, 5, 6};  // corner bits -> MT corner order
+    for (int e = 0; e < (mc ? 12 : 19); e++) {
+        t.a[e] = mc ? (uint8_t)WORD[MC_A[e]] : MT_EDGE_CORNERS[e][0];
+        t.b[e] = mc ? (uint8_t)WORD[MC_B[e]] : MT_EDGE_CORNERS[e][1];
+        t.low[e] = (uint8_t)(mc ? mc_low_axes(e) : low_axes(e));
     }
     return t;
 }
-constexpr EdgeInfo EDGE = make_edge_info();
-template <int E> __device__ __forceinline__ uint32_t mt_extra(const uint32_t (&w)[8], uint32_t m, uint32_t z0, int low) {
-    constexpr int la = EDGE.low[E], ea = EDGE.a[E], eb = EDGE.b[E];
+constexpr EdgeInfo MT_INFO = make_edge_info(false), MC_INFO = make_edge_info(true);
+template <int ALG, int E> __device__ __forceinline__ uint32_t own_extra(const uint32_t (&w)[8], uint32_t m, uint32_t z0, int low) {
+    constexpr bool mc = ALG == MESH_ALG_MC_WELDED;
+    constexpr int la = mc ? MC_INFO.low[E] : MT_INFO.low[E], ea = mc ? MC_INFO.a[E] : MT_INFO.a[E],
+                  eb = mc ? MC_INFO.b[E] : MT_INFO.b[E];
     uint32_t r = 0;
     if constexpr (la != 0) r = (la & ~low & 3) ? 0u : __popc((w[ea] ^ w[eb]) & ((la & 4) ? z0 : m));
-    if constexpr (E + 1 < 19) return r + mt_extra<E + 1>(w, m, z0, low);
+    if constexpr (E + 1 < EdgeDims<ALG>::E) return r + own_extra<ALG, E + 1>(w, m, z0, low);
     return r;
 }
 
@@ -297,6 +375,7 @@ template <class T, class Q, class A, class P, int ALG>
 __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const Tabs &tb, SharedWarp<T, P, ALG> &w,
                                           const typename TabsOf<ALG>::type &ct, const P *rcp, int lane, int xb, int y,
                                           int seg, uint32_t cols) {
+    constexpr bool EDGES = ALG != MESH_ALG_NSN;  // vertices on lattice edges
     const int mw = mask_words(min(v.zws, (v.cz + 31) / 32 - seg * v.zws));
     const uint32_t *mp = p.wmask + bmask(v, seg, y, xb);
     const int x0 = xb * BCOL, x = x0 + lane;
@@ -411,7 +490,7 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                 const int cx = x0 + ln, cz = z0 + zc;
                 const int gx = (int)min((int64_t)2, cx + p.xg0), gy = min(2, y), gz = min(2, cz);
                 // a cell on a lower face, or with a neighbour there
-                const bool edge = ALG == MESH_ALG_MT && __any_sync(FULL, on && (gx < 2 || gy < 2 || gz < 2));
+                const bool edge = EDGES && __any_sync(FULL, on && (gx < 2 || gy < 2 || gz < 2));
                 uint32_t idx = 0;
                 long long id = 0;
 #pragma unroll
@@ -420,13 +499,13 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                     for (int dx = 0; dx < 2; dx++) {
                         const int r = 1 - dy, c = 1 - dx;
                         uint32_t pre;
-                        if constexpr (ALG == MESH_ALG_MT) {
+                        if constexpr (EDGES) {
                             const uint32_t ws[8] = {cu[r][c], cu[r + 1][c], cu[r + 1][c + 1], cu[r][c + 1],
                                                     sh[r][c], sh[r + 1][c], sh[r + 1][c + 1], sh[r][c + 1]};
-                            pre = mt_below(ws, low);
+                            pre = own_below<ALG>(ws, low);
                             // (the first word holds cells of the first plane below this one)
                             if (edge || zw == 0)
-                                pre += mt_extra<0>(ws, low, zw == 0 ? low & 1u : 0u, (gx == dx) | ((gy == dy) << 1));
+                                pre += own_extra<ALG, 0>(ws, low, zw == 0 ? low & 1u : 0u, (gx == dx) | ((gy == dy) << 1));
                         } else {
                             const uint32_t o = cu[r][c] | cu[r][c + 1] | cu[r + 1][c] | cu[r + 1][c + 1] | sh[r][c] |
                                                sh[r][c + 1] | sh[r + 1][c] | sh[r + 1][c + 1];
@@ -439,9 +518,11 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                         const uint32_t k0 = t0[r][c] | (t0[r][c + 1] << 2) | (t0[r + 1][c] << 4) | (t0[r + 1][c + 1] << 6);
                         // and the one below it
                         uint32_t n0;
-                        if constexpr (ALG == MESH_ALG_MT) {
+                        if constexpr (EDGES) {
                             n0 = ct.nvf[k0] & 15u;
-                            if (edge) n0 = __popc(d_mtf.touched[k0] & p.own[(gx == dx) | ((gy == dy) << 1) | ((gz == 1) << 2)]);
+                            if (edge)
+                                n0 = __popc(full_tabs<ALG>().touched[k0] &
+                                            full_tabs<ALG>().own[(gx == dx) | ((gy == dy) << 1) | ((gz == 1) << 2)]);
                             w.nb[dx | (dy << 1)][lane] = (i1 << 8) | k1;
                             if (dx + dy < 2) w.nb[4 | dx | (dy << 1)][lane] = ((i1 - n0) << 8) | k0;
                         } else {
@@ -457,10 +538,10 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                 // own vertices (NSN: crossings) and faces
                 const int bnd = (gx == 0) | ((gy == 0) << 1) | ((gz == 0) << 2);
                 uint32_t nv, nf, nverts = 1;
-                if constexpr (ALG == MESH_ALG_MT) {
+                if constexpr (EDGES) {
                     nv = ct.nvf[idx] & 15u;
                     nf = ct.nvf[idx] >> 4;
-                    if (edge && bnd) nv = __popc(d_mtf.touched[idx] & p.own[bnd]);
+                    if (edge && bnd) nv = __popc(full_tabs<ALG>().touched[idx] & full_tabs<ALG>().own[bnd]);
                     nverts = nv;
                 } else {
                     nv = ct.n[idx];
@@ -525,16 +606,16 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                     if (t >= VW) continue;
                     const uint32_t ci = rc & 255u;
                     const int cl = (int)((rc >> 8) & 31u), zz = (int)((rc >> 13) & 31u), i = t - (int)(rc >> 18);
-                    if constexpr (ALG == MESH_ALG_MT) {
-                        int e = ct.kth[ci][i & 7];
+                    if constexpr (EDGES) {
+                        int e = ct.kth[ci][i & (EdgeDims<ALG>::OWN - 1)];
                         if (edge) {
                             const int b = (x0 + cl + p.xg0 == 0) | ((y == 0) << 1) | ((z0 + zz == 0) << 2);
                             if (b) {
-                                uint32_t om = p.own[b] & d_mtf.touched[ci];
+                                const uint32_t om = full_tabs<ALG>().own[b] & full_tabs<ALG>().touched[ci];
                                 int seen = i;
-                                for (int u = 0; u < MT_MAX_TOUCH; u++) {
-                                    const int ee = d_mtf.order[ci][u];
-                                    if (ee < 19 && ((om >> ee) & 1u) && seen-- == 0) {
+                                for (int u = 0; u < EdgeDims<ALG>::V; u++) {
+                                    const int ee = full_tabs<ALG>().order[ci][u];
+                                    if (ee < EdgeDims<ALG>::E && ((om >> ee) & 1u) && seen-- == 0) {
                                         e = ee;
                                         break;
                                     }
@@ -542,9 +623,25 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                             }
                         }
                         const int cc = ct.corner[e], c1 = cc & 7, c2 = cc >> 3;
-                        const P b3[3] = {w.p[NX + cl], w.p[NY], w.p[NZ + zz]}, d3[3] = {w.d[NX + cl], w.d[NY], w.d[NZ + zz]};
                         P pt[3];
-                        mt_point<T, Q, A, P>(p, c1, c2, w.val[j * VS + c1], w.val[j * VS + c2], b3, d3, pt);
+                        if constexpr (ALG == MESH_ALG_MT) {
+                            const P b3[3] = {w.p[NX + cl], w.p[NY], w.p[NZ + zz]}, d3[3] = {w.d[NX + cl], w.d[NY], w.d[NZ + zz]};
+                            mt_point<T, Q, A, P>(p, c1, c2, w.val[j * VS + c1], w.val[j * VS + c2], b3, d3, pt);
+                        } else {
+                            // vertex_interp (src/marching_cubes.jl:100-104) from the edge's start
+                            const Q mu = quotient<Q>(w.val[j * VS + c1], w.val[j * VS + c2], p);
+                            const int lo[3] = {NX + cl, NY, NZ + zz};
+                            const bool lit = zero || !bits_finite(mu);
+#pragma unroll
+                            for (int u = 0; u < 3; u++) {
+                                const int u1 = (c1 >> u) & 1;
+                                const P p1 = w.p[lo[u] + u1];
+                                if (u1 != ((c2 >> u) & 1))
+                                    pt[u] = Ar<P>::add(p1, Ar<P>::mul((P)mu, u1 ? -w.d[lo[u]] : w.d[lo[u]]));
+                                else
+                                    pt[u] = lit ? Ar<P>::add(p1, Ar<P>::mul((P)mu, P(0))) : p1;
+                            }
+                        }
                         store_point<P>(p, (w.nb[0][j] >> 8) + i, pt[0], pt[1], pt[2]);
                     } else {
                         const int g = ct.edge[ci][i], a = g & 7, ax = g >> 3, b = a ^ (1 << ax);
@@ -595,7 +692,7 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                     const uint32_t ci = rc & 255u;
                     const int i = t - (int)(rc >> 18);
                     long long *out = (long long *)p.faces + 3 * (w.fb[j] + i);
-                    if constexpr (ALG == MESH_ALG_MT) {
+                    if constexpr (EDGES) {
                         long long vid[3];
 #pragma unroll
                         for (int u = 0; u < 3; u++) {
@@ -611,7 +708,7 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                             }
                             const long long nb = w.nb[m][j];
                             const uint32_t ni = (uint32_t)nb & 255u;
-                            const int rank = b ? __popc(d_mtf.before[ni][e] & p.own[b]) : (int)ct.rank[ni][e];
+                            const int rank = b ? __popc(full_tabs<ALG>().before[ni][e] & full_tabs<ALG>().own[b]) : (int)ct.rank[ni][e];
                             vid[u] = (nb >> 8) + rank + 1;
                         }
                         put3((int64_t *)out, vid[0], vid[1], vid[2]);
@@ -644,7 +741,9 @@ __global__ void __launch_bounds__(32 * SW, 2) k_emit_shared(const Plan p, int se
     __shared__ P s_rcp[13];  // NSN: RN(1/n) for the crossing counts n
     Tab &ct = *reinterpret_cast<Tab *>(ssm);
     SharedWarp<T, P, ALG> *sw = reinterpret_cast<SharedWarp<T, P, ALG> *>(ssm + (sizeof(Tab) + 15) / 16 * 16);
-    const uint4 *src = ALG == MESH_ALG_MT ? reinterpret_cast<const uint4 *>(&d_mt) : reinterpret_cast<const uint4 *>(&d_nsn);
+    const uint4 *src = ALG == MESH_ALG_MT    ? reinterpret_cast<const uint4 *>(&d_mt)
+                       : ALG == MESH_ALG_NSN ? reinterpret_cast<const uint4 *>(&d_nsn)
+                                             : reinterpret_cast<const uint4 *>(&d_mc);
     for (int i = threadIdx.x; i < (int)(sizeof(Tab) / 16); i += blockDim.x) reinterpret_cast<uint4 *>(&ct)[i] = src[i];
     if (ALG == MESH_ALG_NSN && threadIdx.x <= 12)
         s_rcp[threadIdx.x] = threadIdx.x ? Ar<P>::div(P(1), (P)(int)threadIdx.x) : P(0);
@@ -709,6 +808,11 @@ template <class T> cudaError_t go_t(const Plan &p, int Q64, int A64, int P64, in
         if (P64) return go<T, float, float, double, MESH_ALG_MT>(p, seg0, nseg, s);
         return go<T, float, float, float, MESH_ALG_MT>(p, seg0, nseg, s);
     }
+    if (p.alg == MESH_ALG_MC_WELDED) {
+        if (Q64) return go<T, double, double, double, MESH_ALG_MC_WELDED>(p, seg0, nseg, s);
+        if (P64) return go<T, float, float, double, MESH_ALG_MC_WELDED>(p, seg0, nseg, s);
+        return go<T, float, float, float, MESH_ALG_MC_WELDED>(p, seg0, nseg, s);
+    }
     if (Q64) return go<T, double, double, double, MESH_ALG_NSN>(p, seg0, nseg, s);
     if (P64) return go<T, float, float, double, MESH_ALG_NSN>(p, seg0, nseg, s);
     return go<T, float, float, float, MESH_ALG_NSN>(p, seg0, nseg, s);
@@ -728,6 +832,7 @@ cudaError_t launch_emit_shared(const Plan &p, int Q64, int A64, int P64, int seg
     case MESH_DT_I64: return go_t<int64_t>(p, Q64, A64, P64, seg0, nseg, s);
     default:
         if (p.alg == MESH_ALG_MT) return go<double, double, double, double, MESH_ALG_MT>(p, seg0, nseg, s);
+        if (p.alg == MESH_ALG_MC_WELDED) return go<double, double, double, double, MESH_ALG_MC_WELDED>(p, seg0, nseg, s);
         return go<double, double, double, double, MESH_ALG_NSN>(p, seg0, nseg, s);
     }
 }

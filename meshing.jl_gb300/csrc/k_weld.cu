@@ -1,7 +1,8 @@
-// Welded Marching Cubes (MESH_ALG_MC_WELDED): one vertex per crossed lattice
-// edge, from the per-cell mesh and its per-vertex edge keys.
+// Welded Marching Cubes (MESH_ALG_MC_WELDED) in batches: one vertex per crossed
+// lattice edge, from the per-cell mesh and its per-vertex edge keys.  (A single
+// volume's welded mesh is emitted from the sign bits, k_emit_shared.cu.)
 //
-// The expansion writes, beside every vertex of the ordinary (per-cell) mesh,
+// The emission writes, beside every vertex of the ordinary (per-cell) mesh,
 // its lattice edge and whether the emitting cell is the first cell of the
 // emission order that meets that edge (Plan::vkey).  Because every crossed edge
 // of a cell carries a vertex of that cell (the case tables place one on each),
@@ -139,35 +140,6 @@ __global__ void __launch_bounds__(WT) k_weld_place(const long long *vkey, int64_
     }
 }
 
-__global__ void __launch_bounds__(WT) k_weld_faces(const long long *vkey, int64_t nv, int64_t *faces, int64_t n,
-                                                   const unsigned long long *hkey, const long long *hval,
-                                                   int64_t hcap, unsigned *err) {
-    const unsigned long long mask = (unsigned long long)hcap - 1;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t j = faces[i] - 1;
-        if (j < 0 || j >= nv) {
-            atomicOr(err, ERR_BOUNDS);
-            continue;
-        }
-        const unsigned long long key = (unsigned long long)(vkey[j] & ~OWN) + 1;
-        unsigned long long h = mix64(key) & mask;
-        long long id = -1;
-        for (int64_t probe = 0; probe < hcap; probe++, h = (h + 1) & mask) {
-            const unsigned long long k = hkey[h];
-            if (k == key) {
-                id = hval[h];
-                break;
-            }
-            if (k == 0ull) break;
-        }
-        if (id < 0) {
-            atomicOr(err, ERR_BOUNDS);
-            continue;
-        }
-        faces[i] = id + 1;
-    }
-}
-
 // Batches: the welded first vertex of every volume v (row n: the welded total)
 // is the number of owned vertices before its first ordinary vertex -- the
 // scanned count of its block plus the owned vertices of that block before it
@@ -246,28 +218,6 @@ int64_t weld_hash_slots(int64_t nv) {
 int64_t weld_blocks(int64_t nv) { return (nv + WB - 1) / WB; }
 
 // Scratch: bsum [nb + 1], hkey [hcap], hval [hcap]; wverts nv * 3 elements.
-cudaError_t launch_weld(const long long *vkey, int64_t nv, const void *verts, int out64, int64_t *faces, int64_t nf,
-                        long long *bsum, void *wverts, unsigned long long *hkey, long long *hval, int64_t hcap,
-                        unsigned *err, int sms, cudaStream_t s) {
-    const int64_t nb = weld_blocks(nv);
-    cudaError_t e = cudaMemsetAsync(hkey, 0, (size_t)hcap * sizeof(unsigned long long), s);
-    if (e != cudaSuccess) return e;
-    if (nb == 0) return cudaMemsetAsync(bsum, 0, sizeof(long long), s);
-    k_weld_count<<<(unsigned)nb, WT, 0, s>>>(vkey, nv, bsum);
-    k_weld_scan<<<1, 1024, 0, s>>>(bsum, nb);
-    if (out64)
-        k_weld_place<double><<<(unsigned)nb, WT, 0, s>>>(vkey, nv, bsum, (const double *)verts, (double *)wverts,
-                                                         hkey, hval, hcap, err);
-    else
-        k_weld_place<float><<<(unsigned)nb, WT, 0, s>>>(vkey, nv, bsum, (const float *)verts, (float *)wverts,
-                                                        hkey, hval, hcap, err);
-    const int64_t n = 3 * nf;
-    if (n > 0)
-        k_weld_faces<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((n + WT - 1) / WT, (int64_t)sms * 16)), WT,
-                       0, s>>>(vkey, nv, faces, n, hkey, hval, hcap, err);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_weld_batch(const long long *vkey, int64_t nvmax, int64_t nfmax, const int64_t *tot,
                               const void *verts, int out64, int64_t *faces, const int64_t *vol_off, int n,
                               int64_t *woff, long long *bsum, void *wverts, unsigned long long *hkey, long long *hval,

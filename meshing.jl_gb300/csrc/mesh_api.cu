@@ -334,13 +334,10 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
     P.cx = (int32_t)(nx - 1); P.cy = (int32_t)(ny - 1); P.cz = (int32_t)(nz - 1);
     set_types(P, T, p, &c->Q64, &c->A64, &c->P64);
     const int L32 = p->range_type == MESH_DT_F32;
-    // welded Marching Cubes runs the Marching Cubes kernels, then welds
-    c->weld = p->alg == MESH_ALG_MC_WELDED;
-    if (c->weld) P.alg = MESH_ALG_MC;
     // x window: MT / NSN take the grid-boundary rules at the whole volume's x = 0; with
     // a halo, the volume's first cell column is the previous slab's last (counted, not
     // emitted)
-    P.xg0 = c->win_nx ? c->win_x0 : 0;
+    P.xg0 = c->win_nx && P.alg != MESH_ALG_MC_WELDED ? c->win_x0 : 0;
     P.xhalo = c->win_nx && c->win_halo;
     if (P.xhalo && P.alg != MESH_ALG_MT && P.alg != MESH_ALG_NSN)
         return fail(c, MESH_EINVAL, "a halo column is for MarchingTetrahedra / NaiveSurfaceNets slabs");
@@ -471,9 +468,8 @@ void mark(mesh_ctx *c, int stage) {
 
 // Marching Cubes walked once, classification staging the active cells (opt-in;
 // also the form that reads a mapped host volume in place).
-// (welded meshes need the expansion in emission order, which writes the edge keys)
 bool one_walk(const mesh_ctx *c) {
-    return c->plan.alg == MESH_ALG_MC && !c->weld && (c->one_walk || c->host_mapped);
+    return c->plan.alg == MESH_ALG_MC && (c->one_walk || c->host_mapped);
 }
 
 // Classified into sign bits and emitted from them: all but the Marching Cubes forms
@@ -747,7 +743,7 @@ void mesh_ctx_destroy(mesh_ctx *c) {
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->copy) cudaStreamSynchronize(c->copy);
     DevBuf *bufs[] = {&c->vol,   &c->tabs,  &c->cnt, &c->base, &c->flags,    &c->scan,   &c->misc,
-                      &c->out_v, &c->out_f, &c->ent, &c->nrm,  &c->weld_buf, &c->weld_v, &c->gat,
+                      &c->out_v, &c->out_f, &c->ent, &c->nrm,  &c->gat,
                       &c->bits, &c->pc,   &c->tsum, &c->wmask,
                       &c->vpre};
     for (DevBuf *b : bufs) b->release();
@@ -790,47 +786,6 @@ int mesh_output_float_bits(int T, const mesh_params *p, int *bits) {
     if (rc) return rc;
     const int tys[4] = {p->range_type, T, p->iso_type, p->eps_type};
     *bits = out_is_f64(tys, p->alg == MESH_ALG_MT ? 4 : 3) ? 64 : 32;
-    return MESH_OK;
-}
-
-// Welded Marching Cubes: extract the per-cell mesh with its edge keys into the
-// context's buffers, weld it (k_weld.cu) and keep the welded counts.
-int run_weld(mesh_ctx *c) {
-    Plan &P = c->plan;
-    const int64_t nv = c->nverts, nf = c->nfaces;
-    const size_t es = P.out64 ? 8 : 4;
-    const int64_t nb = weld_blocks(nv), hcap = weld_hash_slots(nv);
-    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
-    const size_t o_bsum = up((size_t)nv * 8), o_hkey = o_bsum + up((size_t)(nb + 1) * 8),
-                 o_hval = o_hkey + up((size_t)hcap * 8), total = o_hval + up((size_t)hcap * 8);
-    cudaError_t e;
-    if ((e = c->out_v.ensure((size_t)nv * 3 * es + 16)) != cudaSuccess) return cuda_fail(c, e, "vertex buffer");
-    if ((e = c->out_f.ensure((size_t)nf * 24 + 16)) != cudaSuccess) return cuda_fail(c, e, "face buffer");
-    if ((e = c->weld_v.ensure((size_t)nv * 3 * es + 16)) != cudaSuccess) return cuda_fail(c, e, "welded vertices");
-    if ((e = c->weld_buf.ensure(total)) != cudaSuccess) return cuda_fail(c, e, "weld scratch");
-    char *wb = (char *)c->weld_buf.ptr;
-    P.verts = c->out_v.ptr;
-    P.faces = (int64_t *)c->out_f.ptr;
-    P.verts_cap = nv;
-    P.faces_cap = nf;
-    P.vkey = (long long *)wb;
-    int rc;
-    if (!c->bits_on) {
-        if ((rc = ensure_entries(c, c->nactive))) return rc;
-        if ((e = cudaMemsetAsync(P.err, 0, sizeof(unsigned), c->stream)) != cudaSuccess) return cuda_fail(c, e, "memset");
-    }
-    if ((rc = launch_emit(c))) return rc;
-    if ((e = launch_weld(P.vkey, nv, P.verts, P.out64, P.faces, nf, (long long *)(wb + o_bsum), c->weld_v.ptr,
-                         (unsigned long long *)(wb + o_hkey), (long long *)(wb + o_hval), hcap, P.err, c->sms,
-                         c->stream)) != cudaSuccess)
-        return cuda_fail(c, e, "weld launch");
-    long long nw = 0;
-    if ((e = cudaMemcpyAsync(&nw, wb + o_bsum + (size_t)nb * 8, 8, cudaMemcpyDeviceToHost, c->stream)) != cudaSuccess)
-        return cuda_fail(c, e, "welded count");
-    if ((rc = fetch_misc(c))) return rc;  // synchronizes
-    if ((rc = check_err(c))) return rc;
-    c->nverts = nw;
-    P.vkey = nullptr;
     return MESH_OK;
 }
 
@@ -904,7 +859,6 @@ int mesh_count(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int6
     c->nfaces = c->h_misc[1];
     c->nactive = c->h_misc[2];
     if (c->plan.xhalo && (rc = drop_halo_counts(c))) return rc;
-    if (c->weld && (rc = run_weld(c))) return rc;
     *nverts = c->nverts;
     *nfaces = c->nfaces;
     c->have_plan = 1;
@@ -920,16 +874,6 @@ int mesh_fill(mesh_ctx *c, void *verts, int64_t *faces, int out_on_device) {
     Plan &P = c->plan;
     const size_t vb = (size_t)c->nverts * 3 * (P.out64 ? 8 : 4), fbytes = (size_t)c->nfaces * 3 * 8;
     cudaError_t e;
-    if (c->weld) {  // the welded mesh was built by the count: copy it out
-        const cudaMemcpyKind k = out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-        if (vb && (e = cudaMemcpyAsync(verts, c->weld_v.ptr, vb, k, c->stream)) != cudaSuccess)
-            return cuda_fail(c, e, "welded vertex copy");
-        if (fbytes && (e = cudaMemcpyAsync(faces, c->out_f.ptr, fbytes, k, c->stream)) != cudaSuccess)
-            return cuda_fail(c, e, "welded face copy");
-        if ((e = cudaStreamSynchronize(c->stream)) != cudaSuccess) return cuda_fail(c, e, "synchronize");
-        c->have_plan = 0;
-        return MESH_OK;
-    }
     if (out_on_device) {
         P.verts = verts;
         P.faces = faces;

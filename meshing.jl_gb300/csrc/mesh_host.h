@@ -71,10 +71,6 @@ struct mesh_ctx {
     cudaEvent_t ev_cnt = nullptr;
     mesh::TabArgs targs{};
     mesh::DevBuf nrm;  // mesh_vertex_normals: double accumulators
-    // welded Marching Cubes (MESH_ALG_MC_WELDED): the count runs the whole
-    // extraction into out_v / out_f and welds it into weld_v; mesh_fill copies
-    int weld = 0;
-    mesh::DevBuf weld_buf, weld_v;
     int64_t *h_misc = nullptr;  // pinned: totals[NCNT], err
     // Pipelined host path (MESHING_GB300_PIPELINE_BYTES, default 256 MiB: host
     // volumes and meshes at least this large).  mesh_count uploads the volume in

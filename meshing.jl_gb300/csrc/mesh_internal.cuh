@@ -202,15 +202,12 @@ inline void bind_tables(Plan &P, const double *dp, int64_t nx, int64_t ny, int64
     set_tabs(P, tabs_at(dp, nx, ny, nz));
 }
 
-// Welded Marching Cubes (k_weld.cu): blocks of the ownership scan and hash slots
-// for nv per-cell vertices; launch_weld welds verts / faces (faces in place) into
+// Welded batches (k_weld.cu): blocks of the ownership scan and hash slots for nv
+// per-cell vertices; launch_weld_batch welds verts / faces (faces in place) into
 // wverts, bsum[nb] = the welded vertex count.
 int64_t weld_blocks(int64_t nv);
 int64_t weld_hash_slots(int64_t nv);
-cudaError_t launch_weld(const long long *vkey, int64_t nv, const void *verts, int out64, int64_t *faces, int64_t nf,
-                        long long *bsum, void *wverts, unsigned long long *hkey, long long *hval, int64_t hcap,
-                        unsigned *err, int sms, cudaStream_t s);
-// The same over a batch: the counts are read on the device (tot[0] vertices,
+// The counts are read on the device (tot[0] vertices,
 // tot[1] faces, at most nvmax / nfmax), faces are 1-based within their volume
 // (first vertex / face of volume v at vol_off[2v], vol_off[2v + 1]; row n the
 // totals) before and after, and woff receives the welded rows.

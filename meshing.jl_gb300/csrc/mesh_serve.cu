@@ -13,8 +13,7 @@
 //   * Marching Tetrahedra and Naive Surface Nets requests run the
 //     single-volume kernels on the slot's context, into their output blocks;
 //   * welded Marching Cubes requests run the slot context's welded extraction
-//     (the Marching Cubes kernels, then the weld, in the context's own scratch)
-//     and their welded mesh is copied into their output blocks.
+//     (mesh_count, which waits for its stream, and mesh_fill).
 // A host volume gets a block of the pool for itself at admission (counted
 // against the budget like the outputs), is uploaded on the slot's stream ahead
 // of its wave's kernels and gives the block back when the wave's results are
@@ -700,8 +699,8 @@ int launch_wave(mesh_server *s, Slot &sl) {
         for (size_t i = 0; i < sl.singles.size(); i++) {
             const Req &r = sl.wave.at(sl.singles[i]);
             if (r.p.alg == MESH_ALG_MC_WELDED) {
-                // the context's welded extraction (it waits for the slot's stream),
-                // then a device copy of the welded mesh into the output block
+                // the context's welded extraction (it waits for the slot's stream)
+                // into the output block
                 int64_t cnt[3] = {0, 0, 0};
                 int rc = mesh_count(sl.ctx, r.vol, r.T, r.dims[0], r.dims[1], r.dims[2], 1, &r.p, &cnt[0], &cnt[1]);
                 if (rc == MESH_OK && (cnt[0] > r.vcap || cnt[1] > r.fcap)) rc = MESH_ECAPACITY;

@@ -135,7 +135,8 @@ __global__ void __launch_bounds__(256) k_bits(const Plan p, int64_t nib, int w0,
 }
 
 // Batch: the CTAs of volume v pack its planes as above (Plan::bblk_vol names the
-// volume); the CTAs after all of them clear the counters.
+// volume); the CTAs after all of them clear the counters.  (Tables filled here as
+// well took 12 more registers and 15% of the rate.)
 template <class T> __global__ void __launch_bounds__(256) k_bits_batch(const Plan p) {
     if ((int64_t)blockIdx.x >= p.nbblk) {
         clear_counters(p, ((int64_t)blockIdx.x - p.nbblk) * 256 + threadIdx.x, ((int64_t)gridDim.x - p.nbblk) * 256);
@@ -606,23 +607,6 @@ __global__ void __launch_bounds__(OFF_T) k_offsets(const Plan p) {
     }
 }
 
-// Batch: first vertex / face of every volume, then the totals.
-__global__ void __launch_bounds__(256) k_batch_rows(const Plan p) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    after_previous();
-    if (i > p.nvols) return;
-    const int64_t e = i < p.nvols ? p.bvols[i].e0 : p.npc;
-    int64_t vo = p.totals[0], fo = p.totals[1];
-    if (e < p.npc) {
-        const ulonglong2 t = p.tsum[e / BITS_TILE];
-        const uint2 o = p.pc[e];
-        vo = (int64_t)(t.x + o.x);
-        fo = (int64_t)(t.y + o.y);
-    }
-    p.vol_off[2 * (int64_t)i] = vo;
-    p.vol_off[2 * (int64_t)i + 1] = fo;
-}
-
 __global__ void k_gather_pieces(const Plan p, const GatherIdx g, int64_t *dst) {
     const int i = threadIdx.x;
     if (i >= g.n) return;
@@ -718,10 +702,6 @@ cudaError_t launch_bits_batch(const Plan &p, cudaStream_t s) {
 
 cudaError_t launch_count_batch(const Plan &p, cudaStream_t s) {
     return go_count<MESH_ALG_MC, true>(p, 0, 0, false, s);
-}
-
-cudaError_t launch_batch_rows(const Plan &p, cudaStream_t s) {
-    return launch_after(k_batch_rows, (unsigned)(p.nvols / 256 + 1), 256, 0, s, p);
 }
 
 cudaError_t launch_offsets(const Plan &p, cudaStream_t s) {

@@ -404,6 +404,19 @@ __global__ void __launch_bounds__(32 * EW, 3) k_emit_bits_batch(const Plan p, in
     __syncthreads();
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
     after_previous();
+    // first vertex and face of every volume, then the totals
+    for (int i = blockIdx.x * (32 * EW) + threadIdx.x; i <= p.nvols; i += gridDim.x * (32 * EW)) {
+        const int64_t e = i < p.nvols ? p.bvols[i].e0 : p.npc;
+        int64_t vo = p.totals[0], fo = p.totals[1];
+        if (e < p.npc) {
+            const ulonglong2 t = p.tsum[e / BITS_TILE];
+            const uint2 o = p.pc[e];
+            vo = (int64_t)(t.x + o.x);
+            fo = (int64_t)(t.y + o.y);
+        }
+        p.vol_off[2 * (int64_t)i] = vo;
+        p.vol_off[2 * (int64_t)i + 1] = fo;
+    }
     for (;;) {
         unsigned item = 0;
         if (lane == 0) item = atomicAdd(p.work, 1u);
@@ -464,8 +477,7 @@ template <class T, class Q, class P, int PM> cudaError_t go_batch(const Plan &p,
     const int64_t nitems = p.ncblk * (BROW / rows);
     if (grid < 1) return cudaErrorInvalidDevice;
     if (nitems > 0x7fffffff) return cudaErrorInvalidConfiguration;
-    if (nitems < 1) return cudaSuccess;
-    return launch_after(k_emit_bits_batch<T, Q, P, PM>, (unsigned)std::min<int64_t>(grid, nitems), 32 * EW,
+    return launch_after(k_emit_bits_batch<T, Q, P, PM>, (unsigned)std::max<int64_t>(1, std::min<int64_t>(grid, nitems)), 32 * EW,
                         emit_smem<T, PM>(), s, p, nitems, rows);
 }
 

@@ -255,7 +255,7 @@ int prepare_bits(mesh_ctx *c) {
     P.vpre = (uint32_t *)c->vpre.ptr;
     int64_t *m = (int64_t *)c->misc.ptr;
     P.totals = m;
-    P.err = (unsigned int *)(c->h_misc + PIN_ERR);
+    P.err = c->err_out ? c->err_out : (unsigned int *)(c->h_misc + PIN_ERR);
     P.done = (unsigned int *)(m + MISC_DONE);
     P.work = (unsigned int *)(m + MISC_WORK);
     return MESH_OK;

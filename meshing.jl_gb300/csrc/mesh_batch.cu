@@ -141,7 +141,6 @@ cudaError_t launch_batch_counts(const Plan &P, cudaStream_t s) {
     cudaError_t e = launch_bits_batch(P, s);
     if (e == cudaSuccess) e = launch_count_batch(P, s);
     if (e == cudaSuccess) e = launch_offsets(P, s);
-    if (e == cudaSuccess) e = launch_batch_rows(P, s);
     return e;
 }
 

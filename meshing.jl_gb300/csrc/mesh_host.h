@@ -68,6 +68,7 @@ struct mesh_ctx {
     int64_t bits_max = 0;
     int win_segs = 0;
     int bits_on = 0;  // the current plan takes the sign-bit path
+    unsigned int *err_out = nullptr;  // where its kernels report errors (pinned; null: h_misc)
     cudaEvent_t ev_cnt = nullptr;
     mesh::TabArgs targs{};
     mesh::DevBuf nrm;  // mesh_vertex_normals: double accumulators
@@ -153,7 +154,7 @@ struct BatchBufs {
 };
 // The plan's sign-bit fields over those buffers (misc: MISC_WORDS words).
 void bind_batch(Plan &P, const BatchSizes &z, int n, const BatchBufs &b);
-// Sign words, piece counts and offsets, and every volume's first vertex / face.
+// Sign words, piece counts and offsets.
 cudaError_t launch_batch_counts(const Plan &P, cudaStream_t s);
 
 }  // namespace mesh

@@ -228,11 +228,10 @@ struct TabJob {
 };
 cudaError_t launch_tables_batch(const TabJob *jobs, int njobs, int64_t max_ntab, int L32, cudaStream_t s);
 // Batched Marching Cubes stages (k_bits.cu, k_emit_bits.cu); ctas: CTAs per SM of
-// the persistent emission (0 = as many as fit).  launch_batch_rows leaves the first
-// vertex and face of every volume in Plan::vol_off.
+// the persistent emission (0 = as many as fit), which also leaves the first vertex
+// and face of every volume in Plan::vol_off.
 cudaError_t launch_bits_batch(const Plan &p, cudaStream_t s);
 cudaError_t launch_count_batch(const Plan &p, cudaStream_t s);
-cudaError_t launch_batch_rows(const Plan &p, cudaStream_t s);
 cudaError_t launch_emit_batch(const Plan &p, int Q64, int P64, int ctas, cudaStream_t s);
 cudaError_t launch_classify(const Plan &p, cudaStream_t s);
 // Indices of a few pieces whose offsets the host wants.

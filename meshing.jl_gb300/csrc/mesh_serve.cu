@@ -182,8 +182,6 @@ struct Slot {
     size_t stage_cap = 0;
     int64_t *res = nullptr;        // pinned results: counts and error words
     size_t res_cap = 0;            // in int64 words
-    int64_t *d_counts = nullptr;   // device counts of the single-volume requests
-    size_t d_counts_cap = 0;
     std::vector<Group> groups;
     std::vector<int64_t> singles;  // single-volume requests of the wave
     size_t single_res_off = 0;
@@ -670,62 +668,42 @@ int launch_wave(mesh_server *s, Slot &sl) {
         if (!jobs.empty()) memcpy(hs + L.o_jobs, jobs.data(), sizeof(TabJob) * jobs.size());
         if ((e = cudaMemcpyAsync(blk, hs, L.head, cudaMemcpyHostToDevice, sl.stream)) != cudaSuccess)
             return MESH_ECUDA;
-        if (!jobs.empty() &&
-            (e = launch_tables_batch((const TabJob *)(blk + L.o_jobs), (int)jobs.size(), L.z.max_ntab, L32,
-                                     sl.stream)) != cudaSuccess)
-            return MESH_ECUDA;
         bind_batch(P, L.z, n,
                    BatchBufs{blk, blk + L.o_bvol, blk + L.o_cvol, blk + L.o_bits, blk + L.o_pc, blk + L.o_tsum,
                              blk + L.o_mask, blk + L.o_misc, blk + L.o_offs});
         P.vol_outputs = 1;  // each volume checks its own block
-        if ((e = launch_batch_counts(P, sl.stream)) != cudaSuccess ||
-            (e = launch_emit_batch(P, Q64, P64, 0, sl.stream)) != cudaSuccess ||
-            (e = cudaMemcpyAsync(sl.res + g.res_off, P.vol_off, 16 * (size_t)(n + 1), cudaMemcpyDeviceToHost,
-                                 sl.stream)) != cudaSuccess ||
-            (e = cudaMemcpyAsync(sl.res + g.res_off + 2 * (n + 1), P.err, 4, cudaMemcpyDeviceToHost, sl.stream)) !=
-                cudaSuccess)
+        // offsets and error word go straight to the slot's pinned results
+        P.vol_off = sl.res + g.res_off;
+        P.err = (unsigned int *)(sl.res + g.res_off + 2 * (n + 1));
+        if ((!jobs.empty() && (e = launch_tables_batch((const TabJob *)(blk + L.o_jobs), (int)jobs.size(), L.z.max_ntab,
+                                                       L32, sl.stream)) != cudaSuccess) ||
+            (e = launch_batch_counts(P, sl.stream)) != cudaSuccess ||
+            (e = launch_emit_batch(P, Q64, P64, 0, sl.stream)) != cudaSuccess)
             return MESH_ECUDA;
     }
-    if (!sl.singles.empty()) {
-        const size_t need = 3 * sl.singles.size() * 8;
-        if (need > sl.d_counts_cap) {
-            if (sl.d_counts) cudaFree(sl.d_counts);
-            sl.d_counts = nullptr;
-            sl.d_counts_cap = 0;
-            if ((e = cudaMalloc((void **)&sl.d_counts, 2 * need)) != cudaSuccess) return MESH_ENOMEM;
-            sl.d_counts_cap = 2 * need;
+    for (size_t i = 0; i < sl.singles.size(); i++) {
+        const Req &r = sl.wave.at(sl.singles[i]);
+        int64_t *res = sl.res + sl.single_res_off + 3 * i;  // vertices, faces, error word: zeroed above
+        int64_t *faces = (int64_t *)(s->arena + r.out.off + r.vbytes);
+        if (r.dims[0] < 2 || r.dims[1] < 2 || r.dims[2] < 2) continue;  // no cells
+        int rc;
+        if (r.p.alg == MESH_ALG_MC_WELDED) {
+            // the context's welded extraction (it waits for the slot's stream)
+            // into the output block
+            int64_t nv = 0, nf = 0;
+            rc = mesh_count(sl.ctx, r.vol, r.T, r.dims[0], r.dims[1], r.dims[2], 1, &r.p, &nv, &nf);
+            if (rc == MESH_OK && (nv > r.vcap || nf > r.fcap)) rc = MESH_ECAPACITY;
+            if (rc == MESH_OK) rc = mesh_fill(sl.ctx, s->arena + r.out.off, faces, 1);
+            res[0] = nv;
+            res[1] = nf;
+        } else {
+            // its kernels write the counts and the error word into the results
+            sl.ctx->err_out = (unsigned int *)(res + 2);
+            rc = mesh_extract_device(sl.ctx, r.vol, r.T, r.dims[0], r.dims[1], r.dims[2], &r.p, s->arena + r.out.off,
+                                     r.vcap, faces, r.fcap, res);
+            sl.ctx->err_out = nullptr;
         }
-        if ((e = cudaMemsetAsync(sl.d_counts, 0, need, sl.stream)) != cudaSuccess) return MESH_ECUDA;
-        for (size_t i = 0; i < sl.singles.size(); i++) {
-            const Req &r = sl.wave.at(sl.singles[i]);
-            if (r.p.alg == MESH_ALG_MC_WELDED) {
-                // the context's welded extraction (it waits for the slot's stream)
-                // into the output block
-                int64_t cnt[3] = {0, 0, 0};
-                int rc = mesh_count(sl.ctx, r.vol, r.T, r.dims[0], r.dims[1], r.dims[2], 1, &r.p, &cnt[0], &cnt[1]);
-                if (rc == MESH_OK && (cnt[0] > r.vcap || cnt[1] > r.fcap)) rc = MESH_ECAPACITY;
-                if (rc == MESH_OK)
-                    rc = mesh_fill(sl.ctx, s->arena + r.out.off, (int64_t *)(s->arena + r.out.off + r.vbytes), 1);
-                if (rc) return rc;
-                // (a pageable source: the copy takes the values before it returns)
-                if ((e = cudaMemcpyAsync(sl.d_counts + 3 * i, cnt, sizeof(cnt), cudaMemcpyHostToDevice, sl.stream)) !=
-                    cudaSuccess)
-                    return MESH_ECUDA;
-                continue;
-            }
-            int rc = mesh_extract_device(sl.ctx, r.vol, r.T, r.dims[0], r.dims[1], r.dims[2], &r.p,
-                                         s->arena + r.out.off, r.vcap, (int64_t *)(s->arena + r.out.off + r.vbytes),
-                                         r.fcap, sl.d_counts + 3 * i);
-            if (rc) return rc;
-            // the context's error word of this request
-            if (sl.ctx->plan.err &&
-                (e = cudaMemcpyAsync(sl.d_counts + 3 * i + 2, sl.ctx->plan.err, 4, cudaMemcpyDefault,
-                                     sl.stream)) != cudaSuccess)
-                return MESH_ECUDA;
-        }
-        if ((e = cudaMemcpyAsync(sl.res + sl.single_res_off, sl.d_counts, need, cudaMemcpyDeviceToHost, sl.stream)) !=
-            cudaSuccess)
-            return MESH_ECUDA;
+        if (rc) return rc;
     }
     WaveTag *tag = new (std::nothrow) WaveTag{&sl, sl.seq};
     if (!tag) return MESH_ENOMEM;
@@ -855,7 +833,6 @@ void mesh_server_destroy(mesh_server *s) {
         if (sl.stream) cudaStreamDestroy(sl.stream);
         if (sl.stage) cudaFreeHost(sl.stage);
         if (sl.res) cudaFreeHost(sl.res);
-        if (sl.d_counts) cudaFree(sl.d_counts);
     }
     if (s->arena) cudaFree(s->arena);
     delete s;

@@ -62,10 +62,11 @@ def load():
         'mesh_vertex_normals': (c_int, [vp, vp, c_int, ctypes.c_int64, vp, ctypes.c_int64, vp]),
         'mesh_status_string': (ctypes.c_char_p, [c_int]),
         'mesh_ctx_last_error': (ctypes.c_char_p, [vp]),
-        'mesh_output_float_bits': (c_int, [c_int, P(MeshParams), P(c_int)]),
-        'mesh_count': (c_int, [vp, vp, c_int, i64, i64, i64, c_int, P(MeshParams), P(i64), P(i64)]),
+        'mesh_output_float_bits': (c_int, [c_int, vp, vp]),
+        # (pointers to structures as plain addresses on the calls made per extraction)
+        'mesh_count': (c_int, [vp, vp, c_int, i64, i64, i64, c_int, vp, vp, vp]),
         'mesh_fill': (c_int, [vp, vp, vp, c_int]),
-        'mesh_extract_device': (c_int, [vp, vp, c_int, i64, i64, i64, P(MeshParams), vp, i64, vp, i64, vp]),
+        'mesh_extract_device': (c_int, [vp, vp, c_int, i64, i64, i64, vp, vp, i64, vp, i64, vp]),
         'mesh_ctx_sync': (c_int, [vp]),
         'mesh_ctx_enable_timing': (c_int, [vp, c_int]),
         'mesh_ctx_stage_times': (c_int, [vp, P(ctypes.c_double), P(i64)]),
@@ -83,9 +84,9 @@ def load():
         'mesh_server_create': (c_int, [c_int, i64, c_int, c_int, c_int, P(vp)]),
         'mesh_server_destroy': (None, [vp]),
         'mesh_server_last_error': (ctypes.c_char_p, [vp]),
-        'mesh_server_submit': (c_int, [vp, vp, c_int, i64, i64, i64, c_int, P(MeshParams), P(i64)]),
-        'mesh_server_poll': (c_int, [vp, i64, P(c_int), P(i64), P(i64), P(vp), P(vp)]),
-        'mesh_server_wait': (c_int, [vp, i64, i64, P(c_int), P(i64), P(i64), P(vp), P(vp)]),
+        'mesh_server_submit': (c_int, [vp, vp, c_int, i64, i64, i64, c_int, vp, vp]),
+        'mesh_server_poll': (c_int, [vp, i64, vp, vp, vp, vp, vp]),
+        'mesh_server_wait': (c_int, [vp, i64, i64, vp, vp, vp, vp, vp]),
         'mesh_server_release': (c_int, [vp, i64]),
         'mesh_server_stats': (c_int, [vp, P(ctypes.c_double)]),
         'mesh_server_reset_stats': (c_int, [vp]),
@@ -164,9 +165,14 @@ class Context:
         self.set_stream(h if h else CUDA_STREAM_LEGACY)
 
 
+_torch_codes = {}
+
+
 def torch_dtype_code(dtype):
     """Volume dtype code of a torch dtype (None if unsupported)."""
-    import torch
-    return {torch.uint16: MESH_DT_U16, torch.float32: MESH_DT_F32, torch.float64: MESH_DT_F64,
-            torch.int32: MESH_DT_I32, torch.int64: MESH_DT_I64, torch.float16: MESH_DT_F16, torch.int16: MESH_DT_I16,
-            torch.int8: MESH_DT_I8, torch.uint8: MESH_DT_U8}.get(dtype)
+    if not _torch_codes:
+        import torch
+        _torch_codes.update({torch.uint16: MESH_DT_U16, torch.float32: MESH_DT_F32, torch.float64: MESH_DT_F64,
+                             torch.int32: MESH_DT_I32, torch.int64: MESH_DT_I64, torch.float16: MESH_DT_F16,
+                             torch.int16: MESH_DT_I16, torch.int8: MESH_DT_I8, torch.uint8: MESH_DT_U8})
+    return _torch_codes.get(dtype)

@@ -69,6 +69,8 @@ _VOL_DT = {np.dtype(np.uint16): MESH_DT_U16, np.dtype(np.float32): MESH_DT_F32, 
 
 def _scalar(v, what):
     """(mesh dtype, value) of a scalar, following the Julia type of the Python value."""
+    if type(v) is float:
+        return MESH_DT_F64, v
     if isinstance(v, (bool, np.bool_)):
         raise TypeError('%s: Bool is not supported' % what)
     if isinstance(v, np.float32):
@@ -101,30 +103,27 @@ def _first_last(r, what):
 
 def make_params(method, X=(-1, 1), Y=(-1, 1), Z=(-1, 1)):
     """MeshParams for an algorithm instance and the X, Y, Z arguments."""
-    if type(method) not in _ALG:
+    alg = _ALG.get(type(method))
+    if alg is None:
         raise TypeError('method must be MarchingCubes, MarchingTetrahedra or NaiveSurfaceNets')
-    p = MeshParams()
-    _lib.load().mesh_params_default(ctypes.byref(p))
-    p.alg = _ALG[type(method)]
-    if getattr(method, 'weld', False):
-        p.alg = _lib.MESH_ALG_MC_WELDED
-    p.iso_type, p.iso = _scalar(method.iso, 'iso')
-    if isinstance(method, MarchingTetrahedra):
-        p.eps_type, p.eps = _scalar(method.eps, 'eps')
-        if p.eps_type == MESH_DT_I64:
+    if alg == MESH_ALG_MC and method.weld:
+        alg = _lib.MESH_ALG_MC_WELDED
+    iso_type, iso = _scalar(method.iso, 'iso')
+    eps_type, eps = MESH_DT_F64, 1e-3  # mesh_params_default's
+    if alg == MESH_ALG_MT:
+        eps_type, eps = _scalar(method.eps, 'eps')
+        if eps_type == MESH_DT_I64:
             raise TypeError('eps must be a Float32 or Float64')
-    ends = []
-    for r, n in ((X, 'X'), (Y, 'Y'), (Z, 'Z')):
-        ends.extend(_first_last(r, n))
-    tys = set()
-    for i, e in enumerate(ends):
-        t, v = _scalar(e, 'range endpoint')
-        tys.add(t)
-        p.range[i] = v
-    if len(tys) != 1:
+    ends = (*_first_last(X, 'X'), *_first_last(Y, 'Y'), *_first_last(Z, 'Z'))
+    kinds = {type(e) for e in ends}
+    if kinds == {float}:
+        return MeshParams(alg, iso_type, iso, eps_type, eps, MESH_DT_F64, ends)
+    if kinds == {int} and max(map(abs, ends)) <= 2 ** 53:
+        return MeshParams(alg, iso_type, iso, eps_type, eps, MESH_DT_I64, ends)
+    got = [_scalar(e, 'range endpoint') for e in ends]
+    if len({t for t, _ in got}) != 1:
         raise TypeError('X, Y and Z endpoints must share one type')
-    p.range_type = tys.pop()
-    return p
+    return MeshParams(alg, iso_type, iso, eps_type, eps, got[0][0], tuple(v for _, v in got))
 
 
 def output_float_bits(vol_dtype, method, X=(-1, 1), Y=(-1, 1), Z=(-1, 1)):
@@ -193,19 +192,22 @@ def isosurface(A, *args, ctx=None):
         if dt is None:
             raise TypeError('unsupported volume eltype %s' % A.dtype)
         t = _torch_julia_layout(A)
-        c = ctx or default_context(t.device.index or 0)
-        c.follow_torch(t.device)
-        nv, nf = ctypes.c_int64(), ctypes.c_int64()
+        device = t.device
+        c = ctx or default_context(device.index or 0)
+        c.follow_torch(device)
+        n = (ctypes.c_int64 * 2)()  # vertices, faces
+        pn, pp = ctypes.addressof(n), ctypes.addressof(p)
         nx, ny, nz = t.shape
-        check(lib.mesh_count(c.handle, ctypes.c_void_p(t.data_ptr()), dt, nx, ny, nz, 1, ctypes.byref(p),
-                             ctypes.byref(nv), ctypes.byref(nf)), c.handle)
+        rc = lib.mesh_count(c.handle, t.data_ptr(), dt, nx, ny, nz, 1, pp, pn, pn + 8)
+        if rc:
+            check(rc, c.handle)
         bits = ctypes.c_int()
-        check(lib.mesh_output_float_bits(dt, ctypes.byref(p), ctypes.byref(bits)))
-        ft = torch.float32 if bits.value == 32 else torch.float64
-        verts = torch.empty((nv.value, 3), dtype=ft, device=t.device)
-        faces = torch.empty((nf.value, 3), dtype=torch.int64, device=t.device)
-        check(lib.mesh_fill(c.handle, ctypes.c_void_p(verts.data_ptr()), ctypes.c_void_p(faces.data_ptr()), 1),
-              c.handle)
+        check(lib.mesh_output_float_bits(dt, pp, ctypes.addressof(bits)))
+        verts = torch.empty((n[0], 3), dtype=torch.float32 if bits.value == 32 else torch.float64, device=device)
+        faces = torch.empty((n[1], 3), dtype=torch.int64, device=device)
+        rc = lib.mesh_fill(c.handle, verts.data_ptr(), faces.data_ptr(), 1)
+        if rc:
+            check(rc, c.handle)
         return verts, faces
     A = np.asarray(A)
     if A.ndim != 3:
@@ -315,12 +317,13 @@ def isosurface_device(A, method=None, X=(-1, 1), Y=(-1, 1), Z=(-1, 1), verts=Non
     if counts is None:
         counts = torch.zeros(2, dtype=torch.int64, device=t.device)
     nx, ny, nz = t.shape
-    vp = ctypes.c_void_p(verts.data_ptr()) if verts is not None else None
-    fp = ctypes.c_void_p(faces.data_ptr()) if faces is not None else None
-    check(_lib.load().mesh_extract_device(c.handle, ctypes.c_void_p(t.data_ptr()), dt, nx, ny, nz, ctypes.byref(p),
-                                          vp, verts.shape[0] if verts is not None else 0, fp,
-                                          faces.shape[0] if faces is not None else 0,
-                                          ctypes.c_void_p(counts.data_ptr())), c.handle)
+    rc = _lib.load().mesh_extract_device(c.handle, t.data_ptr(), dt, nx, ny, nz, ctypes.addressof(p),
+                                         verts.data_ptr() if verts is not None else None,
+                                         verts.shape[0] if verts is not None else 0,
+                                         faces.data_ptr() if faces is not None else None,
+                                         faces.shape[0] if faces is not None else 0, counts.data_ptr())
+    if rc:
+        check(rc, c.handle)
     return counts
 
 

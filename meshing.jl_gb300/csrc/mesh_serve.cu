@@ -861,7 +861,7 @@ int mesh_server_submit(mesh_server *s, const void *vol, int vol_dtype, int64_t n
     mesh_output_float_bits(vol_dtype, p, &bits);
     r.out64 = bits == 64;
     bounds(&r);
-    std::lock_guard<std::mutex> lk(s->mu);
+    std::unique_lock<std::mutex> lk(s->mu);
     if (!s->have_t0) {
         s->have_t0 = true;
         s->t0 = clk::now();
@@ -882,6 +882,7 @@ int mesh_server_submit(mesh_server *s, const void *vol, int vol_dtype, int64_t n
     *id = r.id;
     s->reqs.emplace(r.id, r);
     s->queue.push_back(r.id);
+    lk.unlock();  // the loop thread wakes to a free lock
     s->cv.notify_all();
     return MESH_OK;
 }

@@ -77,7 +77,9 @@ class Server:
                 raise TypeError('volume must be a 3-D tensor of a supported eltype')
             t = _torch_julia_layout(A)
             # the server reads the volume on its own streams: finish writing it first
-            torch.cuda.current_stream(t.device).synchronize()
+            stream = torch.cuda.current_stream(t.device)
+            if not stream.query():
+                stream.synchronize()
             ptr, shape, on_device = t.data_ptr(), tuple(t.shape), 1
         else:
             t = np.asfortranarray(A.numpy() if hasattr(A, 'numpy') else np.asarray(A))
@@ -85,22 +87,19 @@ class Server:
             if dt is None or t.ndim != 3:
                 raise TypeError('volume must be a 3-D array of a supported eltype')
             ptr, shape, on_device = t.ctypes.data, t.shape, 0
-        bits = ctypes.c_int()
-        self._check(self._lib.mesh_output_float_bits(dt, ctypes.byref(p), ctypes.byref(bits)))
-        rid = ctypes.c_int64()
+        bits, rid = ctypes.c_int(), ctypes.c_int64()
+        pp = ctypes.addressof(p)
+        self._check(self._lib.mesh_output_float_bits(dt, pp, ctypes.addressof(bits)))
         nx, ny, nz = shape
-        self._check(self._lib.mesh_server_submit(self.handle, ctypes.c_void_p(ptr), dt, nx, ny, nz, on_device,
-                                                 ctypes.byref(p), ctypes.byref(rid)))
+        self._check(self._lib.mesh_server_submit(self.handle, ptr, dt, nx, ny, nz, on_device, pp, ctypes.addressof(rid)))
         self._live[rid.value] = (t, bits.value)
         return rid.value
 
     def _query(self, fn, rid, *extra):
-        st, nv, nf = ctypes.c_int(), ctypes.c_int64(), ctypes.c_int64()
-        v, f = ctypes.c_void_p(), ctypes.c_void_p()
-        rc = fn(self.handle, rid, *extra, ctypes.byref(st), ctypes.byref(nv), ctypes.byref(nf), ctypes.byref(v),
-                ctypes.byref(f))
-        self._check(rc)
-        return st.value, nv.value, nf.value, v.value, f.value
+        w = (ctypes.c_int64 * 5)()  # state (its low half), vertices, faces and their addresses
+        a = ctypes.addressof(w)
+        self._check(fn(self.handle, rid, *extra, a, a + 8, a + 16, a + 24, a + 32))
+        return w[0], w[1], w[2], w[3], w[4]
 
     def poll(self, rid):
         """'queued', 'running', 'done' (or MeshError if the request failed)."""
@@ -117,8 +116,8 @@ class Server:
         if st != 2:
             raise TimeoutError('request %d is %s' % (rid, STATE[st]))
         bits = self._live[rid][1]
-        dev = torch.device('cuda', self.device)
         ft = torch.float32 if bits == 32 else torch.float64
+        dev = torch.device('cuda', self.device)
         verts = torch.as_tensor(_DeviceArray(v, (nv, 3), '<f4' if bits == 32 else '<f8'), device=dev) if nv else \
             torch.empty((0, 3), dtype=ft, device=dev)
         faces = torch.as_tensor(_DeviceArray(f, (nf, 3), '<i8'), device=dev) if nf else \

@@ -329,6 +329,7 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
     Plan &P = c->plan;
     P = Plan{};
     c->have_plan = 0;
+    c->emitted = 0;
     c->ngroups = 1;
     P.nx = nx; P.ny = ny; P.nz = nz;
     P.cx = (int32_t)(nx - 1); P.cy = (int32_t)(ny - 1); P.cz = (int32_t)(nz - 1);
@@ -889,6 +890,11 @@ int mesh_fill(mesh_ctx *c, void *verts, int64_t *faces, int out_on_device) {
     if (!one_walk(c) && !c->bits_on && (rc = ensure_entries(c, c->nactive))) return rc;
     if (!c->bits_on && (e = cudaMemsetAsync(P.err, 0, sizeof(unsigned), c->stream)) != cudaSuccess)
         return cuda_fail(c, e, "memset");
+    // a fill whose download failed may be called again
+    if (c->bits_on && c->emitted &&
+        (e = cudaMemsetAsync(P.work, 0, WORK_SLOTS * 2 * sizeof(unsigned), c->stream)) != cudaSuccess)
+        return cuda_fail(c, e, "memset");
+    c->emitted = 1;
     int parts = 1;
     if (!out_on_device && P.alg == MESH_ALG_MC && c->bits_on && c->pipe_bytes > 0 &&
         (int64_t)(vb + fbytes) >= c->pipe_bytes && P.nxb >= 2) {

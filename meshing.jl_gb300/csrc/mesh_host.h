@@ -90,6 +90,7 @@ struct mesh_ctx {
     int64_t *h_gat = nullptr;
     mesh::Plan plan{};
     int have_plan = 0;
+    int emitted = 0;  // mesh_fill has launched this plan's emission: its work counters are spent
     int Q64 = 0, A64 = 0, P64 = 0;
     int64_t nverts = 0, nfaces = 0, nactive = 0;
     int64_t ent_cap_seen = 0;  // largest active-cell list prepared on this context

@@ -7,9 +7,9 @@ seeded a_k ~ N(0,1), |w_k| ~ U[1,8] with a random direction, phi_k ~ U[0,2pi)).
 The volume is 4 GiB, larger than L2, so no flush is needed between steps.
 
 Metric: Gvoxels/s counting input samples nx*ny*nz.
-  value  -- device-resident: mesh_extract_device (classify -> scan ->
-            compaction of the active cells -> expansion into vertices and
-            faces) with the volume and preallocated outputs in HBM;
+  value  -- device-resident: mesh_extract_device (sign bits and piece counts ->
+            offsets -> vertices and faces of the active cells) with the volume
+            and preallocated outputs in HBM;
   e2e    -- the two-phase drop-in call (mesh_count + mesh_fill) with pinned
             host buffers: upload, extraction and download of the mesh.
 The roofline object reports the dominant kernel's algorithmic bytes over its
@@ -143,15 +143,25 @@ def measured_peak():
 
 
 def pieces(nx, ny, nz, sms):
-    """Pieces (one z segment of one cell column) of a volume: the engine's tiling rule
-    (mesh_api.cu, prepare): 31 x 4-cell warp tiles, z segments of whole 8-cell chunks,
-    about 64 warp tiles per SM in all."""
+    """Pieces (one z segment of one cell column) of a volume in the list form: the engine's
+    tiling rule (mesh_api.cu, prepare): 31 x 4-cell warp tiles, z segments of whole 8-cell
+    chunks, about 64 warp tiles per SM in all."""
     cx, cy, cz = nx - 1, ny - 1, nz - 1
     per_seg = ((cx + 30) // 31) * ((cy + 3) // 4)
     nseg = min((cz + 7) // 8, max(1, (sms * 64 + per_seg - 1) // per_seg))
     zs = (cz + nseg - 1) // nseg
     zs = (zs + 7) // 8 * 8
     return ((cz + zs - 1) // zs) * cy * cx
+
+
+def bit_pieces(nx, ny, nz, sms):
+    """The same in the sign-bit form (mesh_api.cu, prepare_bits): items of 32 columns of one
+    cell row, z segments of whole 32-sample words, 512 items per SM."""
+    cx, cy, ncw = nx - 1, ny - 1, (nz - 1 + 31) // 32
+    rows = (cx + 31) // 32 * cy
+    nseg = min(ncw, max(1, (sms * 512 + rows - 1) // rows))
+    zws = (ncw + nseg - 1) // nseg
+    return ((ncw + zws - 1) // zws) * cy * cx
 
 
 def max_over_ranks(dist, values, device='cpu'):
@@ -402,27 +412,28 @@ def run_ours(args, rank, world, dist):
     out_b = nv * 12 + nf * 24
     stage = {k: v[0] / args.steps for k, v in st.items()}  # each timed step runs every stage once
     # algorithmic bytes per launch (input 4 B per sample, mesh 12 B per vertex and
-    # 24 B per face): classify reads every sample (k_classify_tma_mc, staged by
-    # TMA, for volumes with 16-byte aligned rows; the load walk k_classify with
-    # MESHING_GB300_TMA=0); the scan reads 3
-    # u32 counts and writes 3 int64 bases per piece; the direct emission
-    # (k_direct_mc) writes the mesh (its second read of the samples of active
-    # cells is not algorithmic and is not counted).  In the list form
-    # (MESHING_GB300_LIST_EMIT=1) the compaction (k_compact_mc) reads the
-    # samples of the active chunks and writes the list of active cells, and the
-    # expansion (k_expand_mc) writes the mesh: only the expansion gets bytes.
+    # 24 B per face): classify (k_bits and k_count) reads every sample; the scan
+    # (k_offsets) turns 8 B of counts per piece into offsets in place; the emission
+    # (k_emit_bits_mc) writes the mesh (its read of the samples of active cells is not
+    # algorithmic and is not counted).  In the list form (MESHING_GB300_LIST_EMIT=1)
+    # k_classify reads every sample, the scan reads 3 u32 counts and writes 3 int64
+    # bases per piece, the compaction (k_compact_mc) reads the samples of the active
+    # chunks and writes the list of active cells, and the expansion (k_expand_mc)
+    # writes the mesh: only the expansion gets bytes.
     sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    lists = bool(stage.get('expand'))
     kern = {
-        'classify': {'ms': stage['classify'], 'bytes': in_b,
-                     'kernel': 'k_classify' if os.environ.get('MESHING_GB300_TMA') == '0' else 'k_classify_tma_mc'},
-        'scan': {'ms': stage['scan'], 'bytes': float(pieces(n, n, n, sms) * 3 * (4 + 8)), 'kernel': 'k_scan'},
+        'classify': {'ms': stage['classify'], 'bytes': in_b, 'kernel': 'k_classify' if lists else 'k_bits, k_count'},
+        'scan': {'ms': stage['scan'], 'bytes': float(pieces(n, n, n, sms) * 3 * (4 + 8) if lists
+                                                     else bit_pieces(n, n, n, sms) * 16),
+                 'kernel': 'k_scan' if lists else 'k_offsets'},
     }
-    if stage.get('expand'):
+    if lists:
         kern['compact'] = {'ms': stage['emit'], 'bytes': None, 'kernel': 'k_compact_mc',
                            'note': 'reads the samples of active chunks, writes the active-cell list'}
         kern['expand'] = {'ms': stage['expand'], 'bytes': float(out_b), 'kernel': 'k_expand_mc'}
     else:
-        kern['emit'] = {'ms': stage['emit'], 'bytes': float(out_b), 'kernel': 'k_direct_mc',
+        kern['emit'] = {'ms': stage['emit'], 'bytes': float(out_b), 'kernel': 'k_emit_bits_mc',
                         'note': 'writes the mesh; its read of the samples of active cells is not counted'}
     for k in kern.values():
         k['gbs'] = k['bytes'] / (k['ms'] * 1e-3) / 1e9 if k['ms'] and k['bytes'] else None
@@ -763,7 +774,7 @@ def measure_ct(args, rank, world, dev):
     kern = {'classify': (st.get('classify', 0), in_b)}
     if st.get('expand'):  # list form: compaction, then expansion (writes the mesh)
         kern['expand'] = (st['expand'], out_b)
-    else:  # direct emission (writes the mesh)
+    else:  # emission from the sign bits (writes the mesh)
         kern['emit'] = (st.get('emit', 0), out_b)
     roof = {k: {'ms': t_, 'gbs': b / (t_ * 1e-3) / 1e9 if t_ else None,
                 'frac': b / (t_ * 1e-3) / 1e9 / peak if t_ else None} for k, (t_, b) in kern.items()}

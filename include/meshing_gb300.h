@@ -98,7 +98,7 @@ MESH_API void mesh_ctx_destroy(mesh_ctx *ctx);
 /* Makes the context issue its work on `stream` (a cudaStream_t; NULL = the context's own).
    Host-buffer calls on volumes or meshes of at least MESHING_GB300_PIPELINE_BYTES (default
    256 MiB; 0 = never) also use a second, internal copy stream, ordered against `stream` by
-   events: mesh_count uploads in groups of z segments, each classified on arrival, and
+   events: mesh_count uploads in groups of z planes, each classified on arrival, and
    mesh_fill downloads a Marching Cubes mesh in x ranges while the next range is emitted.
    Both calls still return only when their work is complete. */
 MESH_API int mesh_ctx_set_stream(mesh_ctx *ctx, void *stream);
@@ -166,11 +166,10 @@ MESH_API int mesh_vertex_normals(mesh_ctx *ctx, const void *verts, int float_bit
 /* Diagnostics (no counterpart in the reference, which has no instrumentation):
  * with timing enabled the context brackets every kernel launch with CUDA
  * events on its stream.  mesh_ctx_stage_times waits for them and returns, per
- * stage -- 0 classify, 1 scan, 2 emit (the Marching Cubes active-cell
- * compaction, or the whole MT / NSN emit), 3 Marching Cubes expansion -- the
+ * stage -- 0 classify (sign bits, piece counts, totals), 1 scan (piece offsets), 2
+ * emit (in the list form the active-cell compaction), 3 list-form expansion -- the
  * summed device milliseconds ms[0..3] and the number of kernel launches
- * launches[0..3] since the previous query (the coordinate-table kernel counts
- * with stage 0, the four scan kernels with stage 1), then resets. */
+ * launches[0..3] since the previous query, then resets. */
 MESH_API int mesh_ctx_enable_timing(mesh_ctx *ctx, int enable);
 MESH_API int mesh_ctx_stage_times(mesh_ctx *ctx, double *ms, int64_t *launches);
 

@@ -103,6 +103,9 @@ class Batch:
         return {'zs': k[0], 'classify_ctas': k[1], 'compact_ctas': k[2], 'scan_threads': k[3]}
 
     def set_knobs(self, zs=0, classify_ctas=0, compact_ctas=0, scan_threads=1024):
+        """zs: z cells per segment (0: chosen from the batch; rounded up to 32);
+        compact_ctas: CTAs per SM of the emission (0: as many as fit).  The other two
+        are kept and have no effect."""
         k = (ctypes.c_int * 4)(zs, classify_ctas, compact_ctas, scan_threads)
         check(self._lib.mesh_batch_set_knobs(self.handle, k), self.ctx.handle)
 

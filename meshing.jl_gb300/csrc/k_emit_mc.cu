@@ -1,4 +1,4 @@
-// K3 (Marching Cubes), two-pass form -- emit vertices and faces at the
+// K3 (Marching Cubes), list form -- emit vertices and faces at the
 // scanned offsets, after a second walk over the volume.
 //
 // Replaces process_mc_voxel! (src/marching_cubes.jl:67-92).  Two kernels:
@@ -13,9 +13,10 @@
 //
 // K3b expand (mesh_mc.cuh, k_expand_mc<..., EXP_ORDERED>).
 //
-// This is the default form: the one walk of k_walk_mc.cu reads the volume
-// once but costs more in total on GB300.  Its scratch is also known exactly
-// after the scan, which the allocation-free entry point needs.
+// The default is the emission from sign bits (k_emit_bits.cu: 1.78 ms a call at
+// 1024^3 Float32 against 2.37).  This form is the allocation-free entry's, whose
+// static scratch has no room for a word per 32 samples, and runs with
+// MESHING_GB300_LIST_EMIT=1 as an independent form to compare with.
 #define MESH_TBL static __device__ const
 #include "mesh_internal.cuh"
 #include "mesh_tables.h"

@@ -29,9 +29,14 @@
 //
 // Measured per call against the form it replaced, which classified every sample of
 // 4 + 1 rows step by step and worked on one plane's few cells at a time: 256^3
-// gyroid with Float64 vertices, MT 613 -> 319 us, NSN 718 -> 299 us; 509 x 387 x 301
-// Float32 sines, MT 1230 -> 567 us.  Bound by FP64 (2 lanes per SM and cycle) in the
-// Float64 forms.
+// gyroid with Float64 vertices, MT 613 -> 265 us, NSN 718 -> 249 us; 509 x 387 x 301
+// Float32 sines, MT 1230 -> 530 us (this kernel 386 of them: 254 M warp instructions
+// at 57% of issue, 146 MB read and 500 MB written); welded 301 x 187 x 250 Float32
+// gyroid 438 -> 176 us.  The quotients and clamps run on the integer pipes
+// (mesh_quot.h); what bounds it is issue and shared memory (52% of its wavefronts, a
+// third of those bank conflicts of the neighbour look-ups) at the 16 warps per SM that
+// 122 registers and 76-81 KB of tables and staging leave.  Three CTAs per SM (80
+// registers, triangle references read through L1) are slower: MT 281 and 552 us, NSN 257.
 #define MESH_TBL static constexpr
 #include "mesh_internal.cuh"
 #include "mesh_tables.h"

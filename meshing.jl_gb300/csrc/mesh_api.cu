@@ -603,9 +603,8 @@ int launch_emit(mesh_ctx *c) {
 
 // Marching Cubes emission into host buffers in K x ranges of whole x tiles.  The
 // emission order is x-major, so the cells of an x range own one contiguous run of
-// list entries, vertices and faces, starting at the scanned base of the range's
-// first piece (seg 0, y 0, x0).  Range g is compacted and expanded on the compute
-// stream; its vertices and faces go down on the copy stream while range g + 1 is
+// vertices and faces, starting at the offset of the range's first piece
+// (seg 0, y 0, x0).  Range g is emitted on the compute stream; its vertices and faces go down on the copy stream while range g + 1 is
 // emitted.  All launches are enqueued before the copies, so a pageable (blocking)
 // destination still overlaps the copies with the emission.
 int emit_pipelined(mesh_ctx *c, int K, void *verts, int64_t *faces) {

@@ -75,8 +75,8 @@ struct mesh_ctx {
     int64_t *h_misc = nullptr;  // pinned: totals[NCNT], err
     // Pipelined host path (MESHING_GB300_PIPELINE_BYTES, default 256 MiB: host
     // volumes and meshes at least this large).  mesh_count uploads the volume in
-    // groups of z segments on the copy stream and classifies each group as soon
-    // as its planes have arrived; mesh_fill emits the Marching Cubes mesh in x
+    // groups of 32-sample words of z on the copy stream and packs each group's sign
+    // words as soon as its planes have arrived; mesh_fill emits the Marching Cubes mesh in x
     // ranges (contiguous in the x-major emission order) and downloads each range
     // on the copy stream while the next one is emitted.  Events order the two
     // streams; the split points come from the scanned piece bases (gat / h_gat).

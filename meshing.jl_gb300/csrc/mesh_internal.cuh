@@ -77,7 +77,7 @@ struct Plan {
     uint32_t *cnt;        // [NCNT][nseg][cy][cx] per-piece vertex / face / active-cell counts
     int64_t *base;        // [NCNT][nseg][cy][cx] exclusive prefix in traversal order
     uint8_t *flags;       // [nchunks][tiles_x][cy] 1 if the tile row has an active cell
-    unsigned long long *scan_state;  // [NCNT][scan tiles] decoupled look-back words
+    unsigned long long *scan_state;  // list form: run and column sums of the scan
     unsigned int *scan_ticket;
     int64_t *totals;      // [NCNT] total vertices, faces, active cells
     unsigned int *err;    // device error word
@@ -243,7 +243,6 @@ struct GatherIdx {
 // First vertex and face of pieces e[0..n) (after the offset scan): dst[2 i], dst[2 i + 1].
 cudaError_t launch_gather_pieces(const Plan &p, const GatherIdx &g, int64_t *dst, cudaStream_t s);
 cudaError_t launch_scan(const Plan &p, cudaStream_t s);
-cudaError_t launch_emit(const Plan &p, int Q64, int A64, int P64, cudaStream_t s);
 // Sign bits of words w0 .. w0 + nw - 1 of z (k_bits.cu); with a job, the launch
 // also fills its coordinate tables and clears the counters (Plan::totals, tsum).
 struct TabArgs {

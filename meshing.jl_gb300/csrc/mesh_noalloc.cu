@@ -6,7 +6,7 @@
 // block in the allocator.  This entry point serves them.  The caller passes the volume, the output buffers
 // and a small counts buffer (device memory it already owns); every piece of
 // scratch the kernels need -- per-column counts and their scan, activity
-// bytes, look-back state, coordinate tables, the Marching Cubes active-cell
+// bytes, scan sums, coordinate tables, the Marching Cubes active-cell
 // list -- lives in one file-scope __device__ array of NOALLOC_SCRATCH_BYTES.
 // The coordinate tables are computed on the device with the same arithmetic
 // the host path uses, so no host buffer is needed either.

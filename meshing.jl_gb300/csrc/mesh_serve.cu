@@ -8,7 +8,7 @@
 // each one's worst-case vertex / face output (and the wave's scratch), and
 // launches them together as one wave on the slot's stream:
 //   * Marching Cubes requests with the same volume type and iso run as one
-//     batch (k_classify_batch .. k_expand_mc<EXP_BATCH>) that writes every
+//     batch (k_bits_batch .. k_emit_bits_batch) that writes every
 //     volume's mesh straight into that request's own output block;
 //   * Marching Tetrahedra and Naive Surface Nets requests run the
 //     single-volume kernels on the slot's context, into their output blocks;

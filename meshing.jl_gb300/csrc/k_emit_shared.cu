@@ -29,14 +29,16 @@
 //
 // Measured per call against the form it replaced, which classified every sample of
 // 4 + 1 rows step by step and worked on one plane's few cells at a time: 256^3
-// gyroid with Float64 vertices, MT 613 -> 265 us, NSN 718 -> 249 us; 509 x 387 x 301
-// Float32 sines, MT 1230 -> 530 us (this kernel 386 of them: 254 M warp instructions
-// at 57% of issue, 146 MB read and 500 MB written); welded 301 x 187 x 250 Float32
-// gyroid 438 -> 176 us.  The quotients and clamps run on the integer pipes
-// (mesh_quot.h); what bounds it is issue and shared memory (52% of its wavefronts, a
-// third of those bank conflicts of the neighbour look-ups) at the 16 warps per SM that
-// 122 registers and 76-81 KB of tables and staging leave.  Three CTAs per SM (80
-// registers, triangle references read through L1) are slower: MT 281 and 552 us, NSN 257.
+// gyroid with Float64 vertices, MT 613 -> 256 us, NSN 718 -> 243 us; 509 x 387 x 301
+// Float32 sines, MT 1230 -> 523 us (this kernel about 380 of them: 254 M warp
+// instructions at 57% of issue, 146 MB read and 500 MB written); welded 301 x 187 x 250
+// Float32 gyroid 438 -> 172 us.  The quotients and clamps run on the integer pipes
+// (mesh_quot.h); what bounds it is issue and shared memory (half of its wavefronts) at
+// the 16 warps per SM that 122 registers and 77-85 KB of tables and staging leave.  A
+// triangle's three corners come in one word, and the neighbours' rows are padded so that
+// the corners of one cell fall into different banks: MT 260 -> 256, NSN 248 -> 243,
+// welded 177 -> 172, sines 528 -> 523 us.  Three CTAs per SM (80 registers, triangle
+// references read through L1) are slower: MT 281 and 552 us, NSN 257.
 #define MESH_TBL static constexpr
 #include "mesh_internal.cuh"
 #include "mesh_tables.h"
@@ -118,7 +120,7 @@ template <> struct EdgeDims<MESH_ALG_MC_WELDED> { static constexpr int F = MC_MA
 
 template <int ALG> struct alignas(16) EdgeTabs {
     using D = EdgeDims<ALG>;
-    uint8_t ref[256][3 * D::F];        // triangle corners: owner's axes back << 5 | the edge in the owner
+    uint32_t ref[256][D::F];           // a triangle's corners, a byte each: owner's axes back << 5 | the edge in the owner
     uint8_t rank[256][D::E];           // interior cells: rank of an edge among the owned ones
     uint8_t kth[256][D::OWN];          // interior cells: the k-th owned crossed edge in first-use order
     uint8_t nvf[256];                  // interior vertices | faces << 4
@@ -138,7 +140,7 @@ constexpr EdgeTabs<MESH_ALG_MT> make_mt_tabs() {
         const int c = (int)mt_case_of_bits((unsigned)i);
         for (int k = 0; k < 3 * MT_CASE_NFACES[c]; k++) {
             const int e = MT_CASE_FACES[c][k], s = low_axes(e);
-            t.ref[i][k] = (uint8_t)((s << 5) | moved_edge(e, s, 1));
+            t.ref[i][k / 3] |= (uint32_t)((s << 5) | moved_edge(e, s, 1)) << (8 * (k % 3));
         }
         for (int e = 0; e < 19; e++) t.rank[i][e] = (uint8_t)bits_of(MT_BEFORE[c][e] & own_mask(0));
         int n = 0;
@@ -193,7 +195,7 @@ constexpr EdgeTabs<MESH_ALG_MC_WELDED> make_mc_tabs() {
         const int nf = (int)((MC_CASE_VERTS[c] >> 52) & 7u);
         for (int k = 0; k < 3 * nf; k++) {
             const int e = full.order[i][(MC_CASE_FACES[c] >> (4 * k)) & 15u], s = mc_low_axes(e);
-            t.ref[i][k] = (uint8_t)((s << 5) | mc_moved_edge(e, s, 1));
+            t.ref[i][k / 3] |= (uint32_t)((s << 5) | mc_moved_edge(e, s, 1)) << (8 * (k % 3));
         }
         for (int e = 0; e < 12; e++) t.rank[i][e] = (uint8_t)bits_of(full.before[i][e] & mc_own_mask(0));
         int n = 0;
@@ -255,7 +257,7 @@ template <class P> struct Pairs<P, MESH_ALG_NSN> {
 template <class T, class P, int ALG> struct SharedWarp {
     unsigned long long win[3][NC];  // rows y-1 .. y+1: bit 0 the sample below the word, 1-32 the word, 33 above
     long long col[2][NC];           // rows y-1, y, columns x0-1 ..: first vertex of the column's word
-    long long nb[8][32];            // per cell: first vertex (NSN; else << 8 | cell index) of the cell back along the axes
+    long long nb[8][33];            // per cell: first vertex (NSN; else << 8 | cell index) of the cell back along the axes
     long long fb[32];               // per cell: first face
     P p[NT], d[NT];                 // nodes and spacings
     Pairs<P, ALG> pr;
@@ -699,9 +701,10 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
                     long long *out = (long long *)p.faces + 3 * (w.fb[j] + i);
                     if constexpr (EDGES) {
                         long long vid[3];
+                        const uint32_t corners = ct.ref[ci][i];
 #pragma unroll
                         for (int u = 0; u < 3; u++) {
-                            int g = ct.ref[ci][3 * i + u], m = g >> 5, e = g & 31;
+                            int e = (int)(corners >> (8 * u)) & 31, m = (int)(corners >> (8 * u + 5)) & 7;
                             int b = 0;
                             if (edge) {
                                 const int cl = (int)((rc >> 8) & 31u), zz = (int)((rc >> 13) & 31u);

@@ -100,7 +100,10 @@ MESH_API void mesh_ctx_destroy(mesh_ctx *ctx);
    256 MiB; 0 = never) also use a second, internal copy stream, ordered against `stream` by
    events: mesh_count uploads in groups of z planes, each classified on arrival, and
    mesh_fill downloads a Marching Cubes mesh in x ranges while the next range is emitted.
-   Both calls still return only when their work is complete. */
+   mesh_count returns when the counts are known and the host volume has been read; what it
+   leaves behind on its stream (the offsets that mesh_fill starts from) has ended when a later
+   mesh_ctx_set_stream returns, so the fill, or the next call, may be on another stream.
+   mesh_fill returns only when the mesh is complete. */
 MESH_API int mesh_ctx_set_stream(mesh_ctx *ctx, void *stream);
 /* No counterpart in the reference.  Until reset with (0, 0, 0), the volumes of
  * the context's calls are x samples x_first .. x_first+nx-1 of a volume whose x

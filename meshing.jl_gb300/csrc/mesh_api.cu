@@ -486,8 +486,11 @@ int run_count(mesh_ctx *c) {
         mark(c, 0);
         const int parts = c->ngroups > 1 ? c->ngroups + 1 : 2 * ((P.bseg + c->win_segs - 1) / c->win_segs);
         count_kernels(c, 0, parts);
-        if (P.tot_out == c->h_misc + PIN_TOT) {  // the host reads the totals while the offsets are scanned
+        const bool two_phase = P.tot_out == c->h_misc + PIN_TOT;
+        if (two_phase) {  // the host reads the totals while the offsets are scanned
             if (!c->ev_cnt && (e = cudaEventCreateWithFlags(&c->ev_cnt, cudaEventDisableTiming)) != cudaSuccess)
+                return cuda_fail(c, e, "count event");
+            if (!c->ev_off && (e = cudaEventCreateWithFlags(&c->ev_off, cudaEventDisableTiming)) != cudaSuccess)
                 return cuda_fail(c, e, "count event");
             if ((e = cudaEventRecord(c->ev_cnt, c->stream)) != cudaSuccess) return cuda_fail(c, e, "count event");
         }
@@ -495,6 +498,10 @@ int run_count(mesh_ctx *c) {
         if ((e = launch_offsets(P, c->stream)) != cudaSuccess) return cuda_fail(c, e, "scan launch");
         mark(c, 1);
         count_kernels(c, 1, 1);
+        if (two_phase) {
+            if ((e = cudaEventRecord(c->ev_off, c->stream)) != cudaSuccess) return cuda_fail(c, e, "count event");
+            c->off_pending = 1;
+        }
         return MESH_OK;
     }
     if ((e = cudaMemsetAsync(c->misc.ptr, 0, MISC_SLOTS * sizeof(int64_t), c->stream)) != cudaSuccess)
@@ -523,6 +530,7 @@ int fetch_misc(mesh_ctx *c) {
                                     c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "synchronize");
+    c->off_pending = 0;
     if (c->bits_on) c->h_misc[NCNT] = c->h_misc[PIN_ERR];
     c->h_misc[NCNT] &= 0xffffffffll;
     return MESH_OK;
@@ -545,6 +553,7 @@ int finish(mesh_ctx *c) {
     if (!c->bits_on) return fetch_misc(c);
     cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "synchronize");
+    c->off_pending = 0;
     c->h_misc[NCNT] = c->h_misc[PIN_ERR] & 0xffffffffll;
     return MESH_OK;
 }
@@ -752,6 +761,7 @@ void mesh_ctx_destroy(mesh_ctx *c) {
     if (c->ev_ready) cudaEventDestroy(c->ev_ready);
     if (c->ev_done) cudaEventDestroy(c->ev_done);
     if (c->ev_cnt) cudaEventDestroy(c->ev_cnt);
+    if (c->ev_off) cudaEventDestroy(c->ev_off);
     if (c->copy) cudaStreamDestroy(c->copy);
     if (c->h_gat) cudaFreeHost(c->h_gat);
     for (auto &v : c->ev_pairs)
@@ -764,6 +774,18 @@ void mesh_ctx_destroy(mesh_ctx *c) {
 
 int mesh_ctx_set_stream(mesh_ctx *c, void *stream) {
     if (!c) return MESH_EINVAL;
+    // A count's offsets may still be scanned on the old stream (an empty mesh, a fill that
+    // follows or never came): they end before anything is issued on the new one.  The host
+    // waits: the new stream may be capturing, and the old one destroyed by now.
+    if (c->off_pending) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        // (fails only when the device has failed, or for a count that was refused because its
+        // stream was capturing, whose offsets were never launched)
+        if (cudaEventSynchronize(c->ev_off) != cudaSuccess) cudaGetLastError();
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        c->off_pending = 0;
+    }
     c->stream = stream ? (cudaStream_t)stream : c->own;
     return MESH_OK;
 }

@@ -69,7 +69,10 @@ struct mesh_ctx {
     int win_segs = 0;
     int bits_on = 0;  // the current plan takes the sign-bit path
     unsigned int *err_out = nullptr;  // where its kernels report errors (pinned; null: h_misc)
-    cudaEvent_t ev_cnt = nullptr;
+    // mesh_count returns when the totals are known (ev_cnt), while its offsets are still
+    // scanned: ev_off follows them, and off_pending holds until something has waited
+    cudaEvent_t ev_cnt = nullptr, ev_off = nullptr;
+    int off_pending = 0;
     mesh::TabArgs targs{};
     mesh::DevBuf nrm;  // mesh_vertex_normals: double accumulators
     int64_t *h_misc = nullptr;  // pinned: totals[NCNT], err

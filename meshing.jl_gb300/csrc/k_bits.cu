@@ -656,7 +656,7 @@ cudaError_t launch_bits(const Plan &p, int w0, int nw, const TabArgs &ta, int sm
 constexpr int ONE_WAVE = 456;
 
 template <int ALG, bool BATCH>
-static cudaError_t go_count(const Plan &p, int seg0, int nseg, bool vpre_only, cudaStream_t s) {
+static cudaError_t go_count(const Plan &p, int seg0, int nseg, bool vpre_only, cudaStream_t s, int *kernels) {
     const int64_t per = (int64_t)p.nxb * p.nyb;
     // segments to an item: as many as leave 2048 items
     const int gs = BATCH ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(nseg, per * nseg / 2048));
@@ -664,19 +664,23 @@ static cudaError_t go_count(const Plan &p, int seg0, int nseg, bool vpre_only, c
     const bool one = nitems <= ONE_WAVE && (BATCH || nseg == p.bseg);
     if (nitems > 0x7fffffff) return cudaErrorInvalidConfiguration;
     cudaError_t e = cudaSuccess;
-    if (nitems > 0)
+    if (nitems > 0) {
         e = launch_after(k_count<ALG, BATCH>, (unsigned)nitems, 32 * BROW, 0, s, p, seg0, seg0 + nseg, gs,
                          one ? (unsigned)nitems : 0u, vpre_only);
-    if (e == cudaSuccess && !one && !vpre_only && (BATCH || seg0 + nseg == p.bseg))
+        ++*kernels;
+    }
+    if (e == cudaSuccess && !one && !vpre_only && (BATCH || seg0 + nseg == p.bseg)) {
         e = launch_after(k_scan_tiles, 1, 1024, 0, s, p);
+        ++*kernels;
+    }
     return e;
 }
 
-cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s, bool vpre_only) {
-    if (p.alg == MESH_ALG_MC) return go_count<MESH_ALG_MC, false>(p, seg0, nseg, vpre_only, s);
-    if (p.alg == MESH_ALG_MT) return go_count<MESH_ALG_MT, false>(p, seg0, nseg, vpre_only, s);
-    if (p.alg == MESH_ALG_MC_WELDED) return go_count<MESH_ALG_MC_WELDED, false>(p, seg0, nseg, vpre_only, s);
-    return go_count<MESH_ALG_NSN, false>(p, seg0, nseg, vpre_only, s);
+cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s, bool vpre_only, int *kernels) {
+    if (p.alg == MESH_ALG_MC) return go_count<MESH_ALG_MC, false>(p, seg0, nseg, vpre_only, s, kernels);
+    if (p.alg == MESH_ALG_MT) return go_count<MESH_ALG_MT, false>(p, seg0, nseg, vpre_only, s, kernels);
+    if (p.alg == MESH_ALG_MC_WELDED) return go_count<MESH_ALG_MC_WELDED, false>(p, seg0, nseg, vpre_only, s, kernels);
+    return go_count<MESH_ALG_NSN, false>(p, seg0, nseg, vpre_only, s, kernels);
 }
 
 template <class T> static cudaError_t go_bits_batch(const Plan &p, cudaStream_t s) {
@@ -701,7 +705,8 @@ cudaError_t launch_bits_batch(const Plan &p, cudaStream_t s) {
 }
 
 cudaError_t launch_count_batch(const Plan &p, cudaStream_t s) {
-    return go_count<MESH_ALG_MC, true>(p, 0, 0, false, s);
+    int kernels = 0;
+    return go_count<MESH_ALG_MC, true>(p, 0, 0, false, s, &kernels);
 }
 
 cudaError_t launch_offsets(const Plan &p, cudaStream_t s) {

@@ -270,8 +270,8 @@ cudaError_t window_bits(mesh_ctx *c, Plan &P, int s0, int s1, bool first) {
     return launch_bits(P, P.bw0, P.bw1 - P.bw0, ta, c->sms, c->stream);
 }
 
-// Sign words, piece counts and offsets.
-cudaError_t count_bits(mesh_ctx *c) {
+// Sign words and piece counts; adds the kernels launched to *kernels.
+cudaError_t count_bits(mesh_ctx *c, int *kernels) {
     Plan &P = c->plan;
     cudaError_t e = cudaSuccess;
     if (c->ngroups > 1) {
@@ -290,22 +290,26 @@ cudaError_t count_bits(mesh_ctx *c) {
             TabArgs ta = c->targs;
             ta.on = g == 0;
             if (e == cudaSuccess) e = launch_bits(P, w0, w1 - w0, ta, c->sms, c->stream);
+            ++*kernels;
         }
-        if (e == cudaSuccess) e = launch_count(P, 0, P.bseg, c->stream);
+        if (e == cudaSuccess) e = launch_count(P, 0, P.bseg, c->stream, false, kernels);
     } else {
         for (int s0 = 0; s0 < P.bseg && e == cudaSuccess; s0 += c->win_segs) {
             const int s1 = std::min(P.bseg, s0 + c->win_segs);
             e = window_bits(c, P, s0, s1, s0 == 0);
-            if (e == cudaSuccess) e = launch_count(P, s0, s1 - s0, c->stream);
+            ++*kernels;
+            if (e == cudaSuccess) e = launch_count(P, s0, s1 - s0, c->stream, false, kernels);
         }
     }
     return e;
 }
 
-// Emission of the column blocks of `q` (slot: its cleared work counter).
-cudaError_t emit_bits(mesh_ctx *c, Plan q, int slot) {
+// Emission of the column blocks of `q` (slot: its cleared work counter); adds the
+// kernels launched to *kernels.
+cudaError_t emit_bits(mesh_ctx *c, Plan q, int slot, int *kernels) {
     const bool mc = q.alg == MESH_ALG_MC;
     auto emit = [&](int s0, int n) {
+        ++*kernels;
         return mc ? launch_emit_bits_mc(q, c->Q64, c->P64, s0, n, c->stream)
                   : launch_emit_shared(q, c->Q64, c->A64, c->P64, s0, n, c->stream);
     };
@@ -317,8 +321,9 @@ cudaError_t emit_bits(mesh_ctx *c, Plan q, int slot) {
     for (int s0 = 0; s0 < q.bseg && e == cudaSuccess; s0 += c->win_segs) {
         const int s1 = std::min(q.bseg, s0 + c->win_segs);
         e = window_bits(c, q, s0, s1, false);
+        ++*kernels;
         if (e == cudaSuccess) e = cudaMemsetAsync(q.work, 0, sizeof(unsigned), c->stream);
-        if (e == cudaSuccess && !mc) e = launch_count(q, s0, s1 - s0, c->stream, true);
+        if (e == cudaSuccess && !mc) e = launch_count(q, s0, s1 - s0, c->stream, true, kernels);
         if (e == cudaSuccess) e = emit(s0, s1 - s0);
     }
     return e;
@@ -481,11 +486,11 @@ int run_count(mesh_ctx *c) {
     Plan &P = c->plan;
     cudaError_t e;
     if (c->bits_on) {
+        int kernels = 0;
         mark(c, 0);
-        if ((e = count_bits(c)) != cudaSuccess) return cuda_fail(c, e, "classify launch");
+        if ((e = count_bits(c, &kernels)) != cudaSuccess) return cuda_fail(c, e, "classify launch");
         mark(c, 0);
-        const int parts = c->ngroups > 1 ? c->ngroups + 1 : 2 * ((P.bseg + c->win_segs - 1) / c->win_segs);
-        count_kernels(c, 0, parts);
+        count_kernels(c, 0, kernels);
         const bool two_phase = P.tot_out == c->h_misc + PIN_TOT;
         if (two_phase) {  // the host reads the totals while the offsets are scanned
             if (!c->ev_cnt && (e = cudaEventCreateWithFlags(&c->ev_cnt, cudaEventDisableTiming)) != cudaSuccess)
@@ -592,10 +597,11 @@ int launch_emit(mesh_ctx *c) {
         return e != cudaSuccess ? cuda_fail(c, e, "expand launch") : MESH_OK;
     }
     if (c->bits_on) {
+        int kernels = 0;
         mark(c, 2);
-        e = emit_bits(c, c->plan, 0);
+        e = emit_bits(c, c->plan, 0, &kernels);
         mark(c, 2);
-        count_kernels(c, 2, 1);
+        count_kernels(c, 2, kernels);
         return e != cudaSuccess ? cuda_fail(c, e, "emit launch") : MESH_OK;
     }
     mark(c, 2);
@@ -641,16 +647,17 @@ int emit_pipelined(mesh_ctx *c, int K, void *verts, int64_t *faces) {
     for (int g = 0; g < K; g++)
         if (V[g] > V[g + 1] || F[g] > F[g + 1] || V[g + 1] > c->nverts || F[g + 1] > c->nfaces)
             return fail(c, MESH_EDEVICE, "inconsistent split points");
+    int kernels = 0;
     mark(c, 2);
     for (int g = 0; g < K && e == cudaSuccess; g++) {
         Plan q = P;
         q.tx0 = tx[g];
         q.ntx = tx[g + 1] - tx[g];
-        e = emit_bits(c, q, g);
+        e = emit_bits(c, q, g, &kernels);
         if (e == cudaSuccess) e = cudaEventRecord(c->ev_part[g], c->stream);
     }
     mark(c, 2);
-    count_kernels(c, 2, K);
+    count_kernels(c, 2, kernels);
     if (e != cudaSuccess) return cuda_fail(c, e, "emit launch");
     for (int g = 0; g < K && e == cudaSuccess; g++) {
         e = cudaStreamWaitEvent(c->copy, c->ev_part[g], 0);

@@ -253,9 +253,10 @@ struct TabArgs {
 };
 cudaError_t launch_bits(const Plan &p, int w0, int nw, const TabArgs &ta, int sms, cudaStream_t s);
 // Piece counts of segments seg0 .. seg0 + nseg - 1 from the bits; the last CTA of
-// all segments' launches leaves the totals and the tiles' offsets.
-cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s, bool vpre_only = false);
-// (vpre_only: leave the words' vertex prefixes alone, for a later window's emission)
+// all segments' launches leaves the totals and the tiles' offsets, or a launch after
+// them.  vpre_only: leave the words' vertex prefixes alone, for a window's emission.
+// Adds the kernels launched to *kernels.
+cudaError_t launch_count(const Plan &p, int seg0, int nseg, cudaStream_t s, bool vpre_only, int *kernels);
 // Piece counts to offsets within their tile.
 cudaError_t launch_offsets(const Plan &p, cudaStream_t s);
 // Marching Cubes emitted from the bits (k_emit_bits.cu).

@@ -214,7 +214,7 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BatchVol *b, cons
     const uint32_t *r0 = v.bits + (int64_t)(zws0 - v.bw0) * v.sxy + v.nx * y + min(x, v.cx - 1);
     const T *s0 = (const T *)v.vol + v.nx * y + x0;
     for (int q = 0; q < mw; q++) {
-        uint32_t todo = __ldg(mp + q);
+        uint32_t todo = mp[q];
         if (todo && !ready) {
             ready = true;
             if constexpr (BATCH) {
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(32 * EW, 3) k_emit_bits_batch(const Plan p, in
         if (lane < rows && y0 + lane < v.cy) {
             const uint32_t *mp = p.wmask + bmask(v, seg, y0 + lane, xb);
             const int mw = mask_words(min(v.zws, (v.cz + 31) / 32 - seg * v.zws));
-            for (int q = 0; q < mw; q++) any |= __ldg(mp + q);
+            for (int q = 0; q < mw; q++) any |= mp[q];
         }
         const Tabs tb = tabs_at(b->tabs, v.nx, v.ny, v.nz);
         for (uint32_t todo = __ballot_sync(FULL, any != 0u); todo; todo &= todo - 1)

@@ -402,7 +402,7 @@ __device__ __forceinline__ void emit_item(const Plan &p, const BView &v, const T
     };
     long long base[2] = {0, 0}, basex = 0;  // first vertex of this lane's column in rows y-1, y; lanes 0, 1: of column x0-1
     for (int q = 0; q < mw; q++) {
-        uint32_t todo = __ldg(mp + q);
+        uint32_t todo = mp[q];
         if (todo && !ready) {
             ready = true;
             long long F0 = 0, f = 0;

@@ -62,6 +62,10 @@ inline cudaError_t launch_after(void (*k)(A...), unsigned grid, unsigned threads
     c.numAttrs = 1;
     return cudaLaunchKernelEx(&c, k, static_cast<A>(args)...);
 }
+// What the previous kernel writes is read with plain loads: the read-only path (__ldg)
+// is for memory that nothing writes while the CTAs may be resident, here the samples and
+// the coordinate tables (windows of MT, NSN and welded meshes follow k_count, which writes
+// the activity masks, without a kernel between).
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ BView view_of(const Plan &p) {

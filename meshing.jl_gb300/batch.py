@@ -21,9 +21,11 @@ from .api import MarchingCubes, _torch_julia_layout, default_context, make_param
 
 
 class _DeviceArray:
-    """A device buffer seen by torch.as_tensor (zero copy)."""
+    """A device buffer seen by torch.as_tensor (zero copy).  The tensor, and every view of
+    it, holds this object and with it `owner`, whose memory it is."""
 
-    def __init__(self, ptr, shape, typestr):
+    def __init__(self, owner, ptr, shape, typestr):
+        self.owner = owner
         self.__cuda_array_interface__ = {'data': (int(ptr), False), 'shape': tuple(shape), 'typestr': typestr,
                                          'version': 3, 'strides': None}
 
@@ -117,18 +119,20 @@ class Batch:
         return buf.value.decode()
 
     def outputs(self):
-        """(verts [V,3], faces [F,3] int64 1-based per volume, offsets [n+1,2]) as CUDA tensors."""
+        """(verts [V,3], faces [F,3] int64 1-based per volume, offsets [n+1,2]) as CUDA tensors:
+        views of the batch's memory, which they keep until the last of them is dropped
+        (or close())."""
         import torch
         v, f, o = ctypes.c_void_p(), ctypes.c_void_p(), ctypes.c_void_p()
         check(self._lib.mesh_batch_outputs(self.handle, ctypes.byref(v), ctypes.byref(f), ctypes.byref(o)),
               self.ctx.handle)
         ft = '<f4' if self.float_bits == 32 else '<f8'
         dev = self.device
-        verts = torch.as_tensor(_DeviceArray(v.value, (self.nverts, 3), ft), device=dev) if self.nverts else \
+        verts = torch.as_tensor(_DeviceArray(self, v.value, (self.nverts, 3), ft), device=dev) if self.nverts else \
             torch.empty((0, 3), dtype=torch.float32 if self.float_bits == 32 else torch.float64, device=dev)
-        faces = torch.as_tensor(_DeviceArray(f.value, (self.nfaces, 3), '<i8'), device=dev) if self.nfaces else \
+        faces = torch.as_tensor(_DeviceArray(self, f.value, (self.nfaces, 3), '<i8'), device=dev) if self.nfaces else \
             torch.empty((0, 3), dtype=torch.int64, device=dev)
-        offs = torch.as_tensor(_DeviceArray(o.value, (self.n + 1, 2), '<i8'), device=dev)
+        offs = torch.as_tensor(_DeviceArray(self, o.value, (self.n + 1, 2), '<i8'), device=dev)
         return verts, faces, offs
 
     def volume(self, i, outputs=None, offsets=None):

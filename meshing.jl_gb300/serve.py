@@ -110,7 +110,8 @@ class Server:
         return STATE[st]
 
     def result(self, rid, timeout=60.0):
-        """(verts, faces) as CUDA tensor views of the request's resident mesh."""
+        """(verts, faces) as CUDA tensor views of the request's resident mesh.  They hold the
+        server; release() gives the memory back to its pool while they live."""
         import torch
         st, nv, nf, v, f = self._query(self._lib.mesh_server_wait, rid, int(timeout * 1e6))
         if st != 2:
@@ -118,9 +119,9 @@ class Server:
         bits = self._live[rid][1]
         ft = torch.float32 if bits == 32 else torch.float64
         dev = torch.device('cuda', self.device)
-        verts = torch.as_tensor(_DeviceArray(v, (nv, 3), '<f4' if bits == 32 else '<f8'), device=dev) if nv else \
+        verts = torch.as_tensor(_DeviceArray(self, v, (nv, 3), '<f4' if bits == 32 else '<f8'), device=dev) if nv else \
             torch.empty((0, 3), dtype=ft, device=dev)
-        faces = torch.as_tensor(_DeviceArray(f, (nf, 3), '<i8'), device=dev) if nf else \
+        faces = torch.as_tensor(_DeviceArray(self, f, (nf, 3), '<i8'), device=dev) if nf else \
             torch.empty((0, 3), dtype=torch.int64, device=dev)
         return verts, faces
 

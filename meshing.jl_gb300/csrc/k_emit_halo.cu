@@ -1,6 +1,7 @@
 // K3 (Marching Tetrahedra, Naive Surface Nets) -- emit with neighbour lookups, for
-// the allocation-free form (mesh_noalloc.cu): it needs no scratch per sample, where
-// the sign-bit form (k_emit_shared.cu, twice as fast) keeps a quarter of a byte.
+// the allocation-free form (mesh_noalloc.cu), which has no room for the quarter of a byte
+// per sample that the sign-bit form (k_emit_shared.cu, mostly twice as fast) keeps, and for
+// flat volumes of many columns, where this is the faster one (mesh_api.cu, flat()).
 //
 // MT shares vertices between cells: the reference keys every lattice edge in
 // a Dict and numbers a vertex when a cell first touches its edge in

@@ -24,6 +24,7 @@
 
 namespace mesh {
 cudaError_t launch_emit_mc(const Plan &p, int Q64, int P64, int stage, cudaStream_t s);
+cudaError_t launch_emit_halo(const Plan &p, int Q64, int A64, int P64, cudaStream_t s);
 size_t scan_scratch_bytes(const Plan &p);
 }  // namespace mesh
 
@@ -397,6 +398,17 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
     c->bits_on = bits_path(c);
     if ((e = c->tabs.ensure(table_bytes(ntab))) != cudaSuccess) return cuda_fail(c, e, "table buffer");
     if (c->win_nx && c->win_x0 + nx > c->win_nx) return fail(c, MESH_EINVAL, "volume extends past its x window");
+    const int64_t np = npieces(P);
+    const size_t fb = (size_t)P.nchunks * P.tiles_x * P.cy;
+    const size_t sb = (scan_scratch_bytes(P) + 255) / 256 * 256;
+    if (!c->bits_on && P.alg != MESH_ALG_MC &&
+        (c->cnt.ensure((size_t)np * NCNT * sizeof(uint32_t)) != cudaSuccess ||
+         c->base.ensure((size_t)np * NCNT * sizeof(int64_t)) != cudaSuccess || c->flags.ensure(fb) != cudaSuccess ||
+         c->scan.ensure(sb + 64) != cudaSuccess)) {
+        cudaGetLastError();  // the walk's scratch is twice that of the bits
+        for (DevBuf *b : {&c->cnt, &c->base, &c->flags, &c->scan}) b->release();
+        c->bits_on = 1;
+    }
     if (c->bits_on) {
         c->targs = TabArgs{(double *)c->tabs.ptr, nx, ny, nz, c->win_x0, c->win_nx, {}, L32, 0};
         for (int k = 0; k < 6; k++) c->targs.range[k] = p->range[k];
@@ -422,13 +434,10 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
     }
 
     // scratch
-    const int64_t np = npieces(P);
     P.pstride = np;
     if ((e = c->cnt.ensure((size_t)np * NCNT * sizeof(uint32_t))) != cudaSuccess) return cuda_fail(c, e, "count buffer");
     if ((e = c->base.ensure((size_t)np * NCNT * sizeof(int64_t))) != cudaSuccess) return cuda_fail(c, e, "base buffer");
-    const size_t fb = (size_t)P.nchunks * P.tiles_x * P.cy;
     if ((e = c->flags.ensure(fb)) != cudaSuccess) return cuda_fail(c, e, "flag buffer");
-    const size_t sb = (scan_scratch_bytes(P) + 255) / 256 * 256;
     if ((e = c->scan.ensure(sb + 64)) != cudaSuccess) return cuda_fail(c, e, "scan buffer");
     P.cnt = (uint32_t *)c->cnt.ptr;
     P.base = (int64_t *)c->base.ptr;
@@ -478,9 +487,29 @@ bool one_walk(const mesh_ctx *c) {
     return c->plan.alg == MESH_ALG_MC && (c->one_walk || c->host_mapped);
 }
 
-// Classified into sign bits and emitted from them: all but the Marching Cubes forms
-// kept for comparison.
-bool bits_path(const mesh_ctx *c) { return c->plan.alg != MESH_ALG_MC || (!c->list_emit && !one_walk(c)); }
+// MT and NSN on a few layers of cells under many columns: a word of the sign bits holds
+// two or three cells of a column there, and each of the emission's batches little more
+// than a row's few active ones, behind a column-strided look at the piece offsets.  The walk
+// over 4 rows at a time (k_classify.cu, k_emit_halo.cu) is then the faster form.  Calls on
+// smooth Float32 fields, walk against bits: 4096 x 4096 x 2 MT 1264 against 2254 us, NSN
+// 973 against 1942; 2048 x 2048 x 2 MT 423 against 607, NSN 335 against 518;
+// 4096 x 2048 x 3 MT 993 against 1288, NSN 827 against 1021; x 4 MT 1240 against 1404, NSN
+// 1110 against 1079.  With five planes, or below two million columns (where the walk's
+// four-kernel scan weighs more: 1000 x 999 x 3 MT 260 against 224), the bits are no slower.
+// (The walk reports errors with an atomic, which a caller's pinned word need not take.)
+constexpr int FLAT_CELLS = 3;
+constexpr int64_t FLAT_COLUMNS = (int64_t)1 << 21;
+bool flat(const mesh_ctx *c) {
+    const Plan &P = c->plan;
+    return (P.alg == MESH_ALG_MT || P.alg == MESH_ALG_NSN) && P.cz <= FLAT_CELLS &&
+           (int64_t)P.cx * P.cy >= FLAT_COLUMNS && !c->err_out;
+}
+
+// Classified into sign bits and emitted from them: all but flat MT / NSN volumes and the
+// Marching Cubes forms kept for comparison.
+bool bits_path(const mesh_ctx *c) {
+    return c->plan.alg == MESH_ALG_MC ? !c->list_emit && !one_walk(c) : !flat(c);
+}
 
 int run_count(mesh_ctx *c) {
     Plan &P = c->plan;
@@ -604,11 +633,14 @@ int launch_emit(mesh_ctx *c) {
         count_kernels(c, 2, kernels);
         return e != cudaSuccess ? cuda_fail(c, e, "emit launch") : MESH_OK;
     }
+    const bool mc = c->plan.alg == MESH_ALG_MC;
     mark(c, 2);
-    e = launch_emit_mc(c->plan, c->Q64, c->P64, 0, c->stream);
+    e = mc ? launch_emit_mc(c->plan, c->Q64, c->P64, 0, c->stream)
+           : launch_emit_halo(c->plan, c->Q64, c->A64, c->P64, c->stream);
     mark(c, 2);
     count_kernels(c, 2, 1);
     if (e != cudaSuccess) return cuda_fail(c, e, "emit launch");
+    if (!mc) return MESH_OK;
     mark(c, 3);
     e = launch_emit_mc(c->plan, c->Q64, c->P64, 1, c->stream);
     mark(c, 3);
@@ -828,13 +860,20 @@ int drop_halo_counts(mesh_ctx *c) {
     const Plan &P = c->plan;
     int64_t v0 = c->nverts, f0 = c->nfaces;  // a window of the halo column alone emits nothing
     if (P.cx > 1) {
-        GatherIdx gi{};
-        gi.n = 1;
-        gi.idx[0] = (int64_t)P.cy * P.bseg;
-        cudaError_t e = c->gat.ensure(GATHER_MAX * sizeof(int64_t));
-        if (e == cudaSuccess) e = launch_gather_pieces(P, gi, (int64_t *)c->gat.ptr, c->stream);
         int64_t h[2] = {0, 0};
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h, c->gat.ptr, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
+        cudaError_t e;
+        if (c->bits_on) {
+            GatherIdx gi{};
+            gi.n = 1;
+            gi.idx[0] = (int64_t)P.cy * P.bseg;
+            e = c->gat.ensure(GATHER_MAX * sizeof(int64_t));
+            if (e == cudaSuccess) e = launch_gather_pieces(P, gi, (int64_t *)c->gat.ptr, c->stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(h, c->gat.ptr, sizeof(h), cudaMemcpyDeviceToHost, c->stream);
+        } else {
+            const int64_t *b = P.base + piece(P, 0, 0, 1);  // the walk's prefixes
+            e = cudaMemcpyAsync(h, b, 8, cudaMemcpyDeviceToHost, c->stream);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(h + 1, b + P.pstride, 8, cudaMemcpyDeviceToHost, c->stream);
+        }
         if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
         if (e != cudaSuccess) return cuda_fail(c, e, "halo counts");
         v0 = h[0];
@@ -915,7 +954,7 @@ int mesh_fill(mesh_ctx *c, void *verts, int64_t *faces, int out_on_device) {
     P.verts_cap = c->nverts;
     P.faces_cap = c->nfaces;
     int rc;
-    if (!one_walk(c) && !c->bits_on && (rc = ensure_entries(c, c->nactive))) return rc;
+    if (P.alg == MESH_ALG_MC && !one_walk(c) && !c->bits_on && (rc = ensure_entries(c, c->nactive))) return rc;
     if (!c->bits_on && (e = cudaMemsetAsync(P.err, 0, sizeof(unsigned), c->stream)) != cudaSuccess)
         return cuda_fail(c, e, "memset");
     // a fill whose download failed may be called again
@@ -972,7 +1011,7 @@ int mesh_extract_device(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t
     if (c->bits_on) P.tot_out = counts;
     // an active Marching Cubes cell emits at least 3 vertices; the one walk
     // also leaves up to a block of slots per warp unused
-    if (!c->bits_on &&
+    if (P.alg == MESH_ALG_MC && !c->bits_on &&
         (rc = ensure_entries(c, P.verts_cap / 3 + (one_walk(c) ? stage_slack(P) : 0))))
         return rc;
     if ((rc = run_count(c))) return rc;

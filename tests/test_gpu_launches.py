@@ -35,7 +35,7 @@ def kernel_nodes(torch, call):
 
 
 @pytest.mark.parametrize('alg', ['mc', 'mt', 'nsn'])
-@pytest.mark.parametrize('shape,words', [((40, 30, 20), 0), ((300, 301, 40), 0), ((37, 11, 300), 3)])
+@pytest.mark.parametrize('shape,words', [((40, 30, 20), 0), ((300, 301, 40), 0), ((37, 11, 300), 3), ((1449, 1450, 3), 0)])
 def test_reported_launches_are_the_kernels_launched(pkg, cuda, monkeypatch, alg, shape, words):
     torch = cuda
     if words:

@@ -6,8 +6,8 @@
 //
 //   k_bits     reads every sample once: a lane walks 32 z samples of its
 //              column(s) and packs the strict `v < iso` tests into words
-//              (mesh_bits.cuh).  Three instructions per 32 samples, so the
-//              volume streams at the memory's rate.
+//              (mesh_bits.cuh).  4.8 warp instructions per 32 Float32 samples in
+//              the 16-byte form, so the volume streams at the memory's rate.
 //   k_count    a lane owns a column of cells and walks its words of z: eight
 //              words (four corner columns, at z and z + 1) give the active
 //              cells of 32 planes with a few logic instructions, and
@@ -652,7 +652,8 @@ cudaError_t launch_bits(const Plan &p, int w0, int nw, const TabArgs &ta, int sm
     }
 }
 
-// CTAs of k_count that 152 SMs hold at once.
+// CTAs of k_count that 152 SMs hold at once: three an SM at its 70-80 registers (the
+// batches' 64 allow four).
 constexpr int ONE_WAVE = 456;
 
 template <int ALG, bool BATCH>

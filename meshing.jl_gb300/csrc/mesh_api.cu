@@ -404,7 +404,7 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
     if (!c->bits_on && P.alg != MESH_ALG_MC &&
         (c->cnt.ensure((size_t)np * NCNT * sizeof(uint32_t)) != cudaSuccess ||
          c->base.ensure((size_t)np * NCNT * sizeof(int64_t)) != cudaSuccess || c->flags.ensure(fb) != cudaSuccess ||
-         c->scan.ensure(sb + 64) != cudaSuccess)) {
+         c->scan.ensure(sb) != cudaSuccess)) {
         cudaGetLastError();  // the walk's scratch is twice that of the bits
         for (DevBuf *b : {&c->cnt, &c->base, &c->flags, &c->scan}) b->release();
         c->bits_on = 1;
@@ -438,19 +438,17 @@ int prepare(mesh_ctx *c, const void *vol, int T, int64_t nx, int64_t ny, int64_t
     if ((e = c->cnt.ensure((size_t)np * NCNT * sizeof(uint32_t))) != cudaSuccess) return cuda_fail(c, e, "count buffer");
     if ((e = c->base.ensure((size_t)np * NCNT * sizeof(int64_t))) != cudaSuccess) return cuda_fail(c, e, "base buffer");
     if ((e = c->flags.ensure(fb)) != cudaSuccess) return cuda_fail(c, e, "flag buffer");
-    if ((e = c->scan.ensure(sb + 64)) != cudaSuccess) return cuda_fail(c, e, "scan buffer");
+    if ((e = c->scan.ensure(sb)) != cudaSuccess) return cuda_fail(c, e, "scan buffer");
     P.cnt = (uint32_t *)c->cnt.ptr;
     P.base = (int64_t *)c->base.ptr;
     P.flags = (uint8_t *)c->flags.ptr;
     P.scan_state = (unsigned long long *)c->scan.ptr;
-    P.scan_ticket = (unsigned int *)((char *)c->scan.ptr + sb);
     // misc: totals[NCNT] int64, then the error word, the work counter and the
     // staging counter
     P.totals = (int64_t *)c->misc.ptr;
     P.err = (unsigned int *)((int64_t *)c->misc.ptr + NCNT);
     P.work = (unsigned int *)((int64_t *)c->misc.ptr + NCNT + 1);
     P.stage_next = (unsigned long long *)((int64_t *)c->misc.ptr + NCNT + 2);
-    P.scan_spin_limit = 1 << 24;
     return MESH_OK;
 }
 

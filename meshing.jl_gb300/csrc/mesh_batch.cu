@@ -472,20 +472,24 @@ int mesh_batch_tune(mesh_batch *b, int reps, char *report, int report_len) {
     if (cudaSetDevice(c->device) != cudaSuccess) return fail(c, MESH_ECUDA, "cudaSetDevice");
     std::string rep;
     int cur[4] = {b->zs, b->cls_ctas, b->cmp_ctas, b->scan_threads};
-    const std::vector<int> cand[4] = {{0, 64, 32}, {}, {0, 2, 1}, {}};
-    const char *names[4] = {"zs", "classify_ctas", "compact_ctas", "scan_threads"};
+    struct {
+        int knob;
+        const char *name;
+        std::vector<int> values;
+    } const cand[2] = {{0, "zs", {0, 64, 32}}, {2, "compact_ctas", {0, 2, 1}}};  // (1 and 3 have no effect)
     double best_ms = -1;
     int rc;
-    for (int k = 0; k < 4; k++) {
+    for (const auto &t : cand) {
+        const int k = t.knob;
         int best = cur[k];
-        for (int val : cand[k]) {
+        for (int val : t.values) {
             int kn[4] = {cur[0], cur[1], cur[2], cur[3]};
             kn[k] = val;
             if ((rc = mesh_batch_set_knobs(b, kn)) || (rc = count(b))) return rc;
             double ms = 0;
             if ((rc = time_runs(b, reps, &ms))) return rc;
             char line[128];
-            snprintf(line, sizeof(line), "%s=%d %.4f ms\n", names[k], val, ms);
+            snprintf(line, sizeof(line), "%s=%d %.4f ms\n", t.name, val, ms);
             rep += line;
             if (best_ms < 0 || ms < best_ms) {
                 best_ms = ms;

@@ -78,7 +78,6 @@ struct Plan {
     int64_t *base;        // [NCNT][nseg][cy][cx] exclusive prefix in traversal order
     uint8_t *flags;       // [nchunks][tiles_x][cy] 1 if the tile row has an active cell
     unsigned long long *scan_state;  // list form: run and column sums of the scan
-    unsigned int *scan_ticket;
     int64_t *totals;      // [NCNT] total vertices, faces, active cells
     unsigned int *err;    // device error word
     unsigned int *work;   // work-item counter of the persistent kernels
@@ -102,7 +101,6 @@ struct Plan {
     void *verts;
     int64_t *faces;
     int64_t verts_cap, faces_cap;
-    int32_t scan_spin_limit;
     // batches (Marching Cubes over many volumes in one pass): per-volume
     // descriptors, and the first vertex / face of every volume ([nvols + 1][2],
     // the last row the totals)

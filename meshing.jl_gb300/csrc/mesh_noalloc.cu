@@ -113,7 +113,7 @@ extern "C" int mesh_extract_noalloc(const void *vol, int T, int64_t nx, int64_t 
     const int64_t nside = cap / ENT_BLOCK + 1;
     size_t off = 0;
     const size_t o_misc = off;   off += up256((NCNT + 2) * sizeof(int64_t));
-    const size_t o_scan = off;   off += up256(sb + 64);
+    const size_t o_scan = off;   off += up256(sb);
     const size_t o_tab = off;    off += up256(table_bytes(ntab));
     const size_t o_cnt = off;    off += up256((size_t)np * NCNT * 4);
     const size_t o_base = off;   off += up256((size_t)np * NCNT * 8);
@@ -130,7 +130,6 @@ extern "C" int mesh_extract_noalloc(const void *vol, int T, int64_t nx, int64_t 
     P.err = (unsigned int *)((int64_t *)(base + o_misc) + NCNT);
     P.work = (unsigned int *)((int64_t *)(base + o_misc) + NCNT + 1);
     P.scan_state = (unsigned long long *)(base + o_scan);
-    P.scan_ticket = (unsigned int *)(base + o_scan + sb);
     double *dp = (double *)(base + o_tab);
     bind_tables(P, dp, nx, ny, nz);
     P.pstride = np;
@@ -146,7 +145,6 @@ extern "C" int mesh_extract_noalloc(const void *vol, int T, int64_t nx, int64_t 
     P.faces = faces;
     P.verts_cap = verts ? verts_cap : 0;
     P.faces_cap = faces ? faces_cap : 0;
-    P.scan_spin_limit = 1 << 24;
 
     // totals, error word and work counter start at zero; the rest is overwritten
     if ((e = cudaMemsetAsync(base + o_misc, 0, (NCNT + 2) * sizeof(int64_t), s)) != cudaSuccess) return MESH_ECUDA;

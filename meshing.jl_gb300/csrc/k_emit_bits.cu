@@ -21,14 +21,15 @@
 //      population count finds a task's cell and a shuffle fetches its record.
 // The cells of one column are consecutive in the emission order, so task t of
 // column l goes to G[l] + t, G[l] being the column's next vertex (face) minus
-// its first task.  Every stage works on full warps whatever the density.
+// its first task.  A batch holds 24 to 27 cells on the fields below (the list ends with
+// the word); the tasks of each round fill the warp.
 //
 // Measured (1024^3 Float32, 17 M cells, 1.65 GB of mesh): 0.89 ms, 0.96 for the
 // form before it, which walked 8 planes of 31 columns at a time and classified
 // them again; 512^3 UInt16 0.35 against 0.42, 256^3 gyroid with Float64 vertices
 // 0.126 against 0.163 ms.  Of the 0.89 ms, leaving out the face stores saves 0.20,
 // the vertices 0.27, the task look-ups 0.12 and the batch set-up 0.19; leaving out
-// the corner loads alone 0.06 (512^3: 950 instructions per batch, 63% of issue).
+// the corner loads alone 0.06 (512^3: 950 instructions per batch, 66% of issue).
 // Three CTAs per SM: with four (64 registers) it is 4% slower, with five 13%.  A
 // batch of 1024 volumes (1.5 GB of samples): 0.383 ms against 0.575 for listing the
 // active cells and expanding the list.

@@ -30,8 +30,8 @@
 // Measured per call against the form it replaced, which classified every sample of
 // 4 + 1 rows step by step and worked on one plane's few cells at a time: 256^3
 // gyroid with Float64 vertices, MT 613 -> 256 us, NSN 718 -> 243 us; 509 x 387 x 301
-// Float32 sines, MT 1230 -> 523 us (this kernel about 380 of them: 254 M warp
-// instructions at 57% of issue, 146 MB read and 500 MB written); welded 301 x 187 x 250
+// Float32 sines, MT 1230 -> 523 us (this kernel 386 of them: 256 M warp
+// instructions at 58% of issue, 146 MB read and 500 MB written); welded 301 x 187 x 250
 // Float32 gyroid 438 -> 172 us.  The quotients and clamps run on the integer pipes
 // (mesh_quot.h); what bounds it is issue and shared memory (half of its wavefronts) at
 // the 16 warps per SM that 122 registers and 77-85 KB of tables and staging leave.  A
